@@ -34,9 +34,10 @@ int qkrylov_b200_device_count(void);
  * block, x of the block staged in shared memory, per-row class tables)
  * wherever the compiled operator has their tables, with per-die work queues
  * on a two-die GPU; 1: the generic kernel everywhere; 2: as 0 with the
- * blocks handed out in one grid-stride order (no per-die queues); 3: as 0
- * with Hubbard-type operators on the two-part row kernel instead of their
- * spin-product path.  For comparisons; process-wide.  Other values:
+ * blocks handed out in one grid-stride order (no per-die queues); 3: the row
+ * kernels (Hubbard-type operators on the two-part one instead of their
+ * spin-product path, small sectors without their row lists).  For
+ * comparisons; process-wide.  Other values:
  * QKRYLOV_ERROR_INVALID_ARG. */
 int qkrylov_b200_set_kernel_policy(int policy);
 /* Dies of the current device as the row kernels' topology probe measured

@@ -999,8 +999,8 @@ def set_kernel_policy(policy: str):
     """'auto' (the specialised row kernels where the operator has their
     tables, per-die work queues on a two-die GPU), 'generic' (the term-walk
     kernel only), 'no-die-queues' (auto with one grid-stride order) or
-    'no-spin-product' (auto with Hubbard-type operators on the two-part row
-    kernel), for comparisons."""
+    'no-spin-product' (the row kernels: Hubbard-type operators on the
+    two-part one, small sectors without their row lists), for comparisons."""
     codes = {"auto": 0, "generic": 1, "no-die-queues": 2, "no-spin-product": 3}
     _check(lib().qkrylov_b200_set_kernel_policy(codes[policy]), "set_kernel_policy")
 

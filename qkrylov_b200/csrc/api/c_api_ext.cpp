@@ -332,7 +332,7 @@ int qkrylov_b200_apply_operator(qkrylov_basis_h basis, qkrylov_site_h site, qkry
   if (!basis || !basis->table || !site || !opsum || device < 0 || !valid_dtype(dtype) || !x || !y || x == y)
     return QKRYLOV_ERROR_INVALID_ARG;
   return guarded([&] {
-    qkb::Operator op(site->family, basis->table, opsum->terms, device);
+    qkb::Operator op(site->family, basis->table, opsum->terms, device, true);
     const qk_dtype t = qk_dtype(dtype);
     if (!qk_dtype_complex(t) && !op.all_real()) {
       qkapi::set_error("apply_operator: a complex operator needs complex vectors");

@@ -3,7 +3,7 @@
 namespace qkb {
 
 Operator::Operator(Family site_family, std::shared_ptr<const SectorTable> basis,
-                   const std::vector<TermIn>& terms, int device)
+                   const std::vector<TermIn>& terms, int device, bool transient)
     : basis_(std::move(basis)), device_(device) {
   op_ = compile_opsum(site_family, *basis_, terms);
   Context::get(device_);
@@ -24,6 +24,7 @@ Operator::Operator(Family site_family, std::shared_ptr<const SectorTable> basis,
   d.has_diag = op_.has_diag;
   d.all_real = op_.all_real;
   d.pair_sites = is_pair(basis_->family) ? 1 : 0;
+  d.transient = transient ? 1 : 0;
   qkd_check(qkd_plan_create(&d, device_, &plan_), "operator upload");
 }
 

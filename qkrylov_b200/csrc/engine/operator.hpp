@@ -16,7 +16,7 @@ namespace qkb {
 class Operator {
  public:
   Operator(Family site_family, std::shared_ptr<const SectorTable> basis,
-           const std::vector<TermIn>& terms, int device);
+           const std::vector<TermIn>& terms, int device, bool transient = false);
   ~Operator();
   Operator(const Operator&) = delete;
   Operator& operator=(const Operator&) = delete;

@@ -44,6 +44,7 @@ typedef struct {
   const qk_group_t* groups; uint32_t ngroups;
   int has_diag, all_real;
   int pair_sites;  /* 1: two bits per site, up-spin at the even bit (Hubbard, t-J) */
+  int transient;   /* 1: applied once or twice and destroyed; no row lists are built */
 } qk_plan_desc;
 
 typedef struct qk_plan qk_plan;
@@ -57,8 +58,9 @@ size_t qkd_plan_device_bytes(const qk_plan* p);
 
 /* 0: use specialised kernels where the operator qualifies (default);
  * 1: generic kernel only; 2: as 0 without the per-die work queues of the
- * row kernel; 3: as 0 without the spin-product path of Hubbard-type
- * operators (for comparisons). */
+ * row kernel; 3: the row kernels without the spin-product path of
+ * Hubbard-type operators and without the row lists of small sectors (for
+ * comparisons). */
 int qkd_set_kernel_policy(int policy);
 /* Dies of the current device as measured by the row kernels' topology probe
  * (2 or 1) and the SMs on each. */

@@ -13,6 +13,7 @@
 #include <vector>
 
 #include "reduce.cuh"
+#include "hx_terms.cuh"
 #include "../engine/sector.hpp"
 
 namespace qkd {
@@ -24,6 +25,11 @@ PairHandle* pair_plan_create(const qk_plan_desc* d, const uint64_t* A_dev, const
                              const double* diag_ref, size_t* dev_bytes);
 void pair_plan_destroy(PairHandle* h);
 int pair_apply(const PairHandle* h, qk_dtype t, const void* x, void* y, cudaStream_t s, qk_workspace* w,
+               double* dot_out);
+struct ListHandle;
+ListHandle* list_plan_create(const DevPlan& p, uint64_t dim, const double* diag, size_t* dev_bytes);
+void list_plan_destroy(ListHandle* h);
+int list_apply(const ListHandle* h, qk_dtype t, const void* x, void* y, cudaStream_t s, qk_workspace* w,
                double* dot_out);
 bool spin_plan_is_gen(const SpinHandle* h);
 int spin_plan_set_diag(SpinHandle* h, const double* diag);
@@ -39,10 +45,13 @@ int spin_apply(const SpinHandle* h, qk_dtype t, const void* x, void* y, cudaStre
 
 static int g_kernel_policy = 0;  // 0: specialised kernels where eligible, 1: generic only
 static bool g_pair_path = true;  // the spin-product path of Hubbard-type operators
+static bool g_list_path = true;  // the row lists of small sectors
 
 struct qk_plan {
   qkd::SpinHandle* spin = nullptr;
   qkd::PairHandle* pair = nullptr;  // spin-product path (Hubbard-type operators), or null
+  qkd::ListHandle* list = nullptr;  // row lists (small sectors of real operators), or null
+  double* list_diag = nullptr;      // their diagonal where diag_re is null
   int device;
   int nbits, L;
   uint64_t dim, lmask;
@@ -66,42 +75,9 @@ namespace {
 
 constexpr int kTile = 256;
 
-struct DevPlan {
-  int L;
-  uint64_t lmask;
-  const double* __restrict__ diag_re;
-  const uint64_t* __restrict__ A;
-  const uint32_t* __restrict__ B;
-  const uint32_t* __restrict__ llist;
-  const qk_term_t* __restrict__ terms;
-  const qk_group_t* __restrict__ groups;
-  const qk_tile_t* __restrict__ tiles;
-  uint32_t nterms, ngroups, ntiles;
-  int has_diag;
-  uint64_t row_lo, row_hi;  // rows computed by k_hx: [row_lo, row_hi) (tiles never straddle a block)
-};
-
 DevPlan dev(const qk_plan* p, uint64_t row_lo = 0, uint64_t row_hi = ~0ull) {
   return DevPlan{p->L, p->lmask, p->diag_re, p->A, p->B, p->llist, p->terms, p->groups, p->tiles,
                  p->nterms, p->ngroups, p->ntiles, p->has_diag, row_lo, row_hi};
-}
-
-// Sum of the valid terms of one group on state s: returns false when none is valid.
-template <bool CC, class R>
-__device__ __forceinline__ bool group_coef(const qk_term_t* t, uint32_t first, uint32_t count,
-                                           uint64_t s, R& cr, R& ci) {
-  bool any = false;
-  cr = R(0); ci = R(0);
-  for (uint32_t q = first; q < first + count; ++q) {
-    const qk_term_t term = t[q];
-    if ((s & term.cmask) != term.cval) continue;
-    any = true;
-    const bool neg = __popcll(s & term.smask) & 1;
-    const R wr = R(term.wre);
-    cr += neg ? -wr : wr;
-    if (CC) { const R wi = R(term.wim); ci += neg ? -wi : wi; }
-  }
-  return any;
 }
 
 __device__ __forceinline__ void stage_plan(const DevPlan& p, qk_term_t*& st, qk_group_t*& sg) {
@@ -406,6 +382,25 @@ int launch_block_shape(const qk_plan* p, qk_workspace* w, int R, int lpr, const 
   return QKD_EINVAL;
 }
 
+// Row lists of a small sector, with the real diagonal they need.
+void make_lists(qk_plan* p) {
+  const double* diag = p->diag_re;
+  if (p->has_diag && !diag) {
+    if (p->dim > (1ull << 24)) return;
+    if (cudaMalloc(&p->list_diag, p->dim * 8) != cudaSuccess) {
+      (void)cudaGetLastError();
+      return;
+    }
+    if (qkd_diagonal(p, QK_F64, p->list_diag, nullptr) == QKD_OK) diag = p->list_diag;
+  }
+  if (!p->has_diag || diag) p->list = list_plan_create(dev(p), p->dim, diag, &p->bytes);
+  if (p->list && p->list_diag) p->bytes += p->dim * 8;
+  if (!p->list) {
+    cudaFree(p->list_diag);
+    p->list_diag = nullptr;
+  }
+}
+
 int r_index(int R) { return R == 32 ? 0 : R == 64 ? 1 : R == 128 ? 2 : -1; }
 
 }  // namespace
@@ -485,6 +480,7 @@ int qkd_plan_create(const qk_plan_desc* d, int device, qk_plan** out) {
     p->spin = nullptr;
   }
   if (d->pair_sites && p->diag_re) p->pair = qkd::pair_plan_create(d, p->A, p->B, p->diag_re, &p->bytes);
+  if (d->all_real && !d->transient && d->dim > 0) make_lists(p);
   *out = p;
   return QKD_OK;
 }
@@ -492,6 +488,7 @@ int qkd_plan_create(const qk_plan_desc* d, int device, qk_plan** out) {
 int qkd_set_kernel_policy(int policy) {
   if (policy < 0 || policy > 3) return QKD_EINVAL;
   g_kernel_policy = policy == 1 ? 1 : 0;
+  g_list_path = policy != 3;
   qkd::spin_set_die_queues(policy != 2);
   g_pair_path = policy != 3;
   return QKD_OK;
@@ -506,9 +503,11 @@ int qkd_plan_kernel(const qk_plan* p) {
 
 int qkd_plan_destroy(qk_plan* p) {
   if (!p) return QKD_OK;
+  qkd::list_plan_destroy(p->list);
   qkd::pair_plan_destroy(p->pair);
   qkd::spin_plan_destroy(p->spin);
   cudaFree(p->diag_re);
+  cudaFree(p->list_diag);
   cudaFree(p->A); cudaFree(p->B); cudaFree(p->llist);
   cudaFree(p->terms); cudaFree(p->groups); cudaFree(p->tiles);
   delete p;
@@ -523,6 +522,7 @@ int qkd_apply(const qk_plan* p, qk_dtype t, const void* x, void* y, cudaStream_t
   if (!p || !x || !y || x == y) return QKD_EINVAL;
   if (p->dim == 0 || p->ntiles == 0) return QKD_OK;
   if (!qk_dtype_complex(t) && !p->all_real) return QKD_EINVAL;
+  if (p->list && g_kernel_policy == 0 && g_list_path) return qkd::list_apply(p->list, t, x, y, s, nullptr, nullptr);
   if (p->pair && g_kernel_policy == 0 && g_pair_path) {
     const int rc = qkd::pair_apply(p->pair, t, x, y, s, nullptr, nullptr);
     if (rc != QKD_EINVAL) return rc;
@@ -555,6 +555,7 @@ int qkd_apply_dot(const qk_plan* p, qk_workspace* w, qk_dtype t, const void* x, 
   if (!p || !w || !x || !y || x == y || !dot_out) return QKD_EINVAL;
   if (p->dim == 0 || p->ntiles == 0) return QKD_OK;
   if (!qk_dtype_complex(t) && !p->all_real) return QKD_EINVAL;
+  if (p->list && g_kernel_policy == 0 && g_list_path) return qkd::list_apply(p->list, t, x, y, s, w, dot_out);
   if (p->pair && g_kernel_policy == 0 && g_pair_path) {
     const int rc = qkd::pair_apply(p->pair, t, x, y, s, w, dot_out);
     if (rc != QKD_EINVAL) return rc;

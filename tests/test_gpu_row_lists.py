@@ -1,0 +1,57 @@
+"""Row lists of small sectors (kernels/hx_list.cu) against the row kernels,
+the generic kernel and the CPU oracle, for every vector type: sectors below
+one 32-row slice, exact multiples of it and ragged ones, operators without a
+diagonal, and one with more coefficient values than the class table holds."""
+import numpy as np
+import pytest
+
+import oracle as O
+import qkrylov_b200 as qk
+from test_gpu_hx import ham, rel
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+
+def all_pairs(n):
+    """Distinct couplings on every pair: n (n - 1) / 2 coefficient values."""
+    r = np.random.default_rng(n)
+    t = []
+    for i in range(n):
+        for j in range(i + 1, n):
+            w = float(r.uniform(0.2, 1.0))
+            t += [(w, [("Sz", i), ("Sz", j)]), (0.5 * w, [("Sp", i), ("Sm", j)]), (0.5 * w, [("Sm", i), ("Sp", j)])]
+    return t
+
+
+@pytest.mark.parametrize("kind,N,sec,terms", [
+    ("spin", 4, dict(use_sz=1, sz2=0), O.heisenberg_chain(4)),                      # 6 rows: part of one slice
+    ("spin", 6, {}, O.heisenberg_chain(6)),                                         # 64 rows: two whole slices
+    ("spin", 11, dict(use_sz=1, sz2=1), O.heisenberg_chain(11, periodic=False)),    # 462 rows: ragged last slice
+    ("spin", 10, {}, [(0.5, [("Sz", i), ("Sz", (i + 1) % 10)]) for i in range(10)] + [(0.7, [("Sx", i)]) for i in range(10)]),
+    ("spin", 9, {}, [(0.7, [("Sx", i)]) for i in range(9)]),                        # no diagonal
+    ("spin", 12, dict(use_sz=1, sz2=0), all_pairs(12)),                             # 66 values: no lists, row kernel
+    ("fermion", 9, dict(use_n=1, n=4), [(-1.0, [("C", (i + 1) % 9), ("Cdag", i)]) for i in range(9)] +
+     [(-1.0, [("C", i), ("Cdag", (i + 1) % 9)]) for i in range(9)]),
+    ("hubbard", 6, dict(use_nup=1, nup=3, use_ndn=1, ndn=2), O.hubbard_square(3, 2)),
+    ("tj", 9, dict(use_nup=1, nup=4, use_ndn=1, ndn=3), O.tj_chain(9)),
+])
+def test_row_lists_match_other_kernels(kind, N, sec, terms):
+    H = ham(kind, N, sec, terms)
+    ref = O.port().hamiltonian(kind, N, sec, terms)
+    rng = np.random.default_rng(N)
+    xc = rng.standard_normal(H.dimension) + 1j * rng.standard_normal(H.dimension)
+    for code, tdt, tol in [(qk.DTYPE_C128, torch.complex128, 1e-13), (qk.DTYPE_C64, torch.complex64, 2e-6),
+                           (qk.DTYPE_F64, torch.float64, 1e-13), (qk.DTYPE_F32, torch.float32, 2e-6)]:
+        x = torch.tensor(xc if tdt.is_complex else xc.real, dtype=tdt, device="cuda")
+        want = ref.apply(x.cpu().numpy().astype(np.complex128))
+        try:
+            for pol in ("auto", "no-spin-product", "generic"):
+                qk.set_kernel_policy(pol)
+                y = torch.full_like(x, float("nan"))
+                torch.cuda.synchronize()
+                H.apply_device(x.data_ptr(), y.data_ptr(), code)
+                torch.cuda.synchronize()
+                assert rel(y.cpu().numpy().astype(np.complex128), want) < tol, (pol, code)
+        finally:
+            qk.set_kernel_policy("auto")
