@@ -30,7 +30,7 @@ struct ListHandle;
 ListHandle* list_plan_create(const DevPlan& p, uint64_t dim, const double* diag, size_t* dev_bytes);
 void list_plan_destroy(ListHandle* h);
 int list_apply(const ListHandle* h, qk_dtype t, const void* x, void* y, cudaStream_t s, qk_workspace* w,
-               double* dot_out);
+               double* dot_out, uint64_t row_lo, uint64_t row_hi);
 bool spin_plan_is_gen(const SpinHandle* h);
 int spin_plan_set_diag(SpinHandle* h, const double* diag);
 int spin_apply_block(const SpinHandle* h, qk_dtype t, int R, int lpr, const void* X, void* Y, double* dots,
@@ -522,7 +522,7 @@ int qkd_apply(const qk_plan* p, qk_dtype t, const void* x, void* y, cudaStream_t
   if (!p || !x || !y || x == y) return QKD_EINVAL;
   if (p->dim == 0 || p->ntiles == 0) return QKD_OK;
   if (!qk_dtype_complex(t) && !p->all_real) return QKD_EINVAL;
-  if (p->list && g_kernel_policy == 0 && g_list_path) return qkd::list_apply(p->list, t, x, y, s, nullptr, nullptr);
+  if (p->list && g_kernel_policy == 0 && g_list_path) return qkd::list_apply(p->list, t, x, y, s, nullptr, nullptr, 0, p->dim);
   if (p->pair && g_kernel_policy == 0 && g_pair_path) {
     const int rc = qkd::pair_apply(p->pair, t, x, y, s, nullptr, nullptr);
     if (rc != QKD_EINVAL) return rc;
@@ -540,6 +540,8 @@ int qkd_apply_range(const qk_plan* p, qk_dtype t, const void* x, void* y, uint64
   if (!p || !x || !y || x == y || row_lo > row_hi || row_hi > p->dim) return QKD_EINVAL;
   if (p->dim == 0 || p->ntiles == 0 || row_lo == row_hi) return QKD_OK;
   if (!qk_dtype_complex(t) && !p->all_real) return QKD_EINVAL;
+  if (p->list && g_kernel_policy == 0 && g_list_path)
+    return qkd::list_apply(p->list, t, x, y, s, nullptr, nullptr, row_lo, row_hi);
   if (p->spin && g_kernel_policy == 0) {
     const int rc = qkd::spin_apply_range(p->spin, t, x, y, s, row_lo, row_hi);
     if (rc != QKD_EINVAL) return rc;
@@ -555,7 +557,7 @@ int qkd_apply_dot(const qk_plan* p, qk_workspace* w, qk_dtype t, const void* x, 
   if (!p || !w || !x || !y || x == y || !dot_out) return QKD_EINVAL;
   if (p->dim == 0 || p->ntiles == 0) return QKD_OK;
   if (!qk_dtype_complex(t) && !p->all_real) return QKD_EINVAL;
-  if (p->list && g_kernel_policy == 0 && g_list_path) return qkd::list_apply(p->list, t, x, y, s, w, dot_out);
+  if (p->list && g_kernel_policy == 0 && g_list_path) return qkd::list_apply(p->list, t, x, y, s, w, dot_out, 0, p->dim);
   if (p->pair && g_kernel_policy == 0 && g_pair_path) {
     const int rc = qkd::pair_apply(p->pair, t, x, y, s, w, dot_out);
     if (rc != QKD_EINVAL) return rc;

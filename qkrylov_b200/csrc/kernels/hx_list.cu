@@ -41,6 +41,7 @@ constexpr size_t kListMaxBytes = size_t(64) << 20;
 
 struct ListPlan {
   uint32_t dim, nslice;
+  uint32_t row_lo, row_hi, slice0;  // rows written; first slice that holds one of them
   const uint32_t* start;  // per slice: first 4-slot group (nslice + 1)
   const uint4* words;     // four slots of a row per 16 bytes: [slot / 4][lane]
   const double* diag;     // or null
@@ -123,7 +124,7 @@ __global__ void __launch_bounds__(kListThreads) k_hx_list(const __grid_constant_
   using R = typename T::R;
   __shared__ R s_coef[kListClasses];
   const uint32_t lane = threadIdx.x & 31, nw = gridDim.x * (kListThreads / 32);
-  uint32_t sl = blockIdx.x * (kListThreads / 32) + (threadIdx.x >> 5);
+  uint32_t sl = p.slice0 + blockIdx.x * (kListThreads / 32) + (threadIdx.x >> 5);
   uint32_t b0 = 0, b1 = 0;
   if (sl < p.nslice) { b0 = __ldg(p.start + sl); b1 = __ldg(p.start + sl + 1); }
   if (threadIdx.x < kListClasses) s_coef[threadIdx.x] = R(p.coef[threadIdx.x]);
@@ -131,7 +132,7 @@ __global__ void __launch_bounds__(kListThreads) k_hx_list(const __grid_constant_
   double dr = 0.0, di = 0.0;
   while (sl < p.nslice) {
     const uint32_t row = sl * 32 + lane;
-    const bool in = row < p.dim;
+    const bool in = row >= p.row_lo && row < p.row_hi;
     R xr = R(0), xi = R(0), d = R(0);
     if (in) {
       T::ld(x, row, xr, xi);
@@ -255,14 +256,21 @@ ListHandle* list_plan_create(const DevPlan& p, uint64_t dim, const double* diag,
   return h;
 }
 
+// Rows [row_lo, row_hi) of y = H x, row_lo < row_hi <= dim; with dot_out
+// (whole vectors only) also <x, y>.
 int list_apply(const ListHandle* h, qk_dtype t, const void* x, void* y, cudaStream_t s, qk_workspace* w,
-               double* dot_out) {
-  const unsigned g = (h->plan.nslice + kListThreads / 32 - 1) / (kListThreads / 32);
+               double* dot_out, uint64_t row_lo, uint64_t row_hi) {
+  ListPlan p = h->plan;
+  p.row_lo = uint32_t(row_lo);
+  p.row_hi = uint32_t(row_hi);
+  p.slice0 = p.row_lo / 32;
+  p.nslice = (p.row_hi + 31) / 32;
+  const unsigned g = (p.nslice - p.slice0 + kListThreads / 32 - 1) / (kListThreads / 32);
   if (dot_out) {
     QKD_DISPATCH(t, (k_hx_list<DT, true><<<std::min<unsigned>(g, kMaxG), kListThreads, 0, s>>>(
-                        h->plan, x, y, w->partials, w->ticket, dot_out)));
+                        p, x, y, w->partials, w->ticket, dot_out)));
   } else {
-    QKD_DISPATCH(t, (k_hx_list<DT, false><<<g, kListThreads, 0, s>>>(h->plan, x, y, nullptr, nullptr, nullptr)));
+    QKD_DISPATCH(t, (k_hx_list<DT, false><<<g, kListThreads, 0, s>>>(p, x, y, nullptr, nullptr, nullptr)));
   }
   QKD_LAUNCH_CHECK();
   return QKD_OK;
