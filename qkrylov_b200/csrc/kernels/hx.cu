@@ -26,6 +26,12 @@ PairHandle* pair_plan_create(const qk_plan_desc* d, const uint64_t* A_dev, const
 void pair_plan_destroy(PairHandle* h);
 int pair_apply(const PairHandle* h, qk_dtype t, const void* x, void* y, cudaStream_t s, qk_workspace* w,
                double* dot_out);
+struct FlipHandle;
+bool flip_eligible(const qk_plan_desc* d);
+FlipHandle* flip_plan_create(const qk_plan_desc* d, const double* diag, size_t* dev_bytes);
+void flip_plan_destroy(FlipHandle* h);
+int flip_apply(const FlipHandle* h, qk_dtype t, const void* x, void* y, cudaStream_t s, qk_workspace* w,
+               double* dot_out, uint64_t row_lo, uint64_t row_hi);
 struct ListHandle;
 ListHandle* list_plan_create(const DevPlan& p, uint64_t dim, const double* diag, size_t* dev_bytes);
 void list_plan_destroy(ListHandle* h);
@@ -45,13 +51,14 @@ int spin_apply(const SpinHandle* h, qk_dtype t, const void* x, void* y, cudaStre
 
 static int g_kernel_policy = 0;  // 0: specialised kernels where eligible, 1: generic only
 static bool g_pair_path = true;  // the spin-product path of Hubbard-type operators
-static bool g_list_path = true;  // the row lists of small sectors
+static bool g_list_path = true;  // the row lists of small sectors, the flips of complete bases
 
 struct qk_plan {
   qkd::SpinHandle* spin = nullptr;
   qkd::PairHandle* pair = nullptr;  // spin-product path (Hubbard-type operators), or null
   qkd::ListHandle* list = nullptr;  // row lists (small sectors of real operators), or null
-  double* list_diag = nullptr;      // their diagonal where diag_re is null
+  qkd::FlipHandle* flip = nullptr;  // unconditional flips on a complete basis, or null
+  double* list_diag = nullptr;      // the diagonal of either where diag_re is null
   int device;
   int nbits, L;
   uint64_t dim, lmask;
@@ -382,20 +389,25 @@ int launch_block_shape(const qk_plan* p, qk_workspace* w, int R, int lpr, const 
   return QKD_EINVAL;
 }
 
-// Row lists of a small sector, with the real diagonal they need.
-void make_lists(qk_plan* p) {
+// The table-free kernel of unconditional flips, else the row lists of a small
+// sector, with the real diagonal they need.
+void make_lists(qk_plan* p, const qk_plan_desc* d) {
+  const bool flips = flip_eligible(d);
+  if (!flips && p->dim > (1ull << 24)) return;
   const double* diag = p->diag_re;
   if (p->has_diag && !diag) {
-    if (p->dim > (1ull << 24)) return;
     if (cudaMalloc(&p->list_diag, p->dim * 8) != cudaSuccess) {
       (void)cudaGetLastError();
       return;
     }
     if (qkd_diagonal(p, QK_F64, p->list_diag, nullptr) == QKD_OK) diag = p->list_diag;
   }
-  if (!p->has_diag || diag) p->list = list_plan_create(dev(p), p->dim, diag, &p->bytes);
-  if (p->list && p->list_diag) p->bytes += p->dim * 8;
-  if (!p->list) {
+  if (!p->has_diag || diag) {
+    if (flips) p->flip = flip_plan_create(d, diag, &p->bytes);
+    if (!p->flip) p->list = list_plan_create(dev(p), p->dim, diag, &p->bytes);
+  }
+  if ((p->list || p->flip) && p->list_diag) p->bytes += p->dim * 8;
+  if (!p->list && !p->flip) {
     cudaFree(p->list_diag);
     p->list_diag = nullptr;
   }
@@ -480,7 +492,7 @@ int qkd_plan_create(const qk_plan_desc* d, int device, qk_plan** out) {
     p->spin = nullptr;
   }
   if (d->pair_sites && p->diag_re) p->pair = qkd::pair_plan_create(d, p->A, p->B, p->diag_re, &p->bytes);
-  if (d->all_real && !d->transient && d->dim > 0) make_lists(p);
+  if (d->all_real && !d->transient && d->dim > 0) make_lists(p, d);
   *out = p;
   return QKD_OK;
 }
@@ -504,6 +516,7 @@ int qkd_plan_kernel(const qk_plan* p) {
 int qkd_plan_destroy(qk_plan* p) {
   if (!p) return QKD_OK;
   qkd::list_plan_destroy(p->list);
+  qkd::flip_plan_destroy(p->flip);
   qkd::pair_plan_destroy(p->pair);
   qkd::spin_plan_destroy(p->spin);
   cudaFree(p->diag_re);
@@ -522,6 +535,7 @@ int qkd_apply(const qk_plan* p, qk_dtype t, const void* x, void* y, cudaStream_t
   if (!p || !x || !y || x == y) return QKD_EINVAL;
   if (p->dim == 0 || p->ntiles == 0) return QKD_OK;
   if (!qk_dtype_complex(t) && !p->all_real) return QKD_EINVAL;
+  if (p->flip && g_kernel_policy == 0 && g_list_path) return qkd::flip_apply(p->flip, t, x, y, s, nullptr, nullptr, 0, p->dim);
   if (p->list && g_kernel_policy == 0 && g_list_path) return qkd::list_apply(p->list, t, x, y, s, nullptr, nullptr, 0, p->dim);
   if (p->pair && g_kernel_policy == 0 && g_pair_path) {
     const int rc = qkd::pair_apply(p->pair, t, x, y, s, nullptr, nullptr);
@@ -540,6 +554,8 @@ int qkd_apply_range(const qk_plan* p, qk_dtype t, const void* x, void* y, uint64
   if (!p || !x || !y || x == y || row_lo > row_hi || row_hi > p->dim) return QKD_EINVAL;
   if (p->dim == 0 || p->ntiles == 0 || row_lo == row_hi) return QKD_OK;
   if (!qk_dtype_complex(t) && !p->all_real) return QKD_EINVAL;
+  if (p->flip && g_kernel_policy == 0 && g_list_path)
+    return qkd::flip_apply(p->flip, t, x, y, s, nullptr, nullptr, row_lo, row_hi);
   if (p->list && g_kernel_policy == 0 && g_list_path)
     return qkd::list_apply(p->list, t, x, y, s, nullptr, nullptr, row_lo, row_hi);
   if (p->spin && g_kernel_policy == 0) {
@@ -557,6 +573,7 @@ int qkd_apply_dot(const qk_plan* p, qk_workspace* w, qk_dtype t, const void* x, 
   if (!p || !w || !x || !y || x == y || !dot_out) return QKD_EINVAL;
   if (p->dim == 0 || p->ntiles == 0) return QKD_OK;
   if (!qk_dtype_complex(t) && !p->all_real) return QKD_EINVAL;
+  if (p->flip && g_kernel_policy == 0 && g_list_path) return qkd::flip_apply(p->flip, t, x, y, s, w, dot_out, 0, p->dim);
   if (p->list && g_kernel_policy == 0 && g_list_path) return qkd::list_apply(p->list, t, x, y, s, w, dot_out, 0, p->dim);
   if (p->pair && g_kernel_policy == 0 && g_pair_path) {
     const int rc = qkd::pair_apply(p->pair, t, x, y, s, w, dot_out);

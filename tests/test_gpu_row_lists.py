@@ -1,7 +1,9 @@
-"""Row lists of small sectors (kernels/hx_list.cu) against the row kernels,
-the generic kernel and the CPU oracle, for every vector type: sectors below
-one 32-row slice, exact multiples of it and ragged ones, operators without a
-diagonal, and one with more coefficient values than the class table holds."""
+"""Row lists of small sectors (kernels/hx_list.cu) and the flips of complete
+bases (kernels/hx_flip.cu) against the row kernels, the generic kernel and
+the CPU oracle, for every vector type: sectors below one 32-row slice, exact
+multiples of it and ragged ones, operators without a diagonal, one with more
+coefficient values than the class table holds; flips of one tile and of four,
+with state-dependent coefficients, some of them zero."""
 import numpy as np
 import pytest
 
@@ -31,12 +33,16 @@ def all_pairs(n):
     ("spin", 10, {}, [(0.5, [("Sz", i), ("Sz", (i + 1) % 10)]) for i in range(10)] + [(0.7, [("Sx", i)]) for i in range(10)]),
     ("spin", 9, {}, [(0.7, [("Sx", i)]) for i in range(9)]),                        # no diagonal
     ("spin", 12, dict(use_sz=1, sz2=0), all_pairs(12)),                             # 66 values: no lists, row kernel
+    ("spin", 11, {}, [(0.5, [("Sz", i), ("Sz", (i + 1) % 11)]) for i in range(11)] + [(0.7, [("Sx", i)]) for i in range(11)]),
+    ("spin", 13, {}, [(0.7 + 0.1 * i, [("Sx", i)]) for i in range(13)]),            # flips, no diagonal
+    ("spin", 13, {}, [(w, [(o, i), (o, (i + 1) % 13)]) for i in range(13) for o, w in (("Sx", 0.4), ("Sy", 0.4), ("Sz", 0.3))]
+     + [(0.2, [("Sx", 3)])]),                                                       # coefficients zero for parallel spins
     ("fermion", 9, dict(use_n=1, n=4), [(-1.0, [("C", (i + 1) % 9), ("Cdag", i)]) for i in range(9)] +
      [(-1.0, [("C", i), ("Cdag", (i + 1) % 9)]) for i in range(9)]),
     ("hubbard", 6, dict(use_nup=1, nup=3, use_ndn=1, ndn=2), O.hubbard_square(3, 2)),
     ("tj", 9, dict(use_nup=1, nup=4, use_ndn=1, ndn=3), O.tj_chain(9)),
 ])
-def test_row_lists_match_other_kernels(kind, N, sec, terms):
+def test_small_sector_kernels_match_the_others(kind, N, sec, terms):
     H = ham(kind, N, sec, terms)
     ref = O.port().hamiltonian(kind, N, sec, terms)
     rng = np.random.default_rng(N)
