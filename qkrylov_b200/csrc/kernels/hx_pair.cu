@@ -43,16 +43,22 @@ struct PairPlan {
   const uint32_t* up_col;
   const double* up_val;
   const uint32_t* dn_ptr;  // CSR of T_dn (Dd + 1)
-  const uint16_t* dn_ent;  // column | (sign << 15) when every |T_dn| equals dn_mag
-  const uint32_t* dn_col;  // otherwise columns and values
+  const uint32_t* dn_col;
   const double* dn_val;
-  double dn_mag;
+  // T_dn by hop, when its elements have at most kMags magnitudes: per tile of
+  // 32 rows the first group and the groups of each magnitude (8 bits each); a
+  // slot is one hop, four slots of a row per uint2 ([group][lane]), each the
+  // target index with the sign in bit 15 (indices Dd .. Dd + 7: no target, a
+  // zero pack)
+  const uint2 *dn_rec, *dn_slot;
+  double dn_mag[4];
   const double* diag;      // D in product order (Du * Dd)
   const uint32_t* perm;    // rank(u, d) in product order (Du * Dd), or null: computed from A, B
 };
 
 namespace {
 
+constexpr int kMags = 4;  // magnitudes of the by-hop tables
 constexpr int kPT = 256;  // threads per CTA; k_pair_up takes row slabs of 2 * kPT elements
 constexpr int kDT = 1024; // k_pair_dn: one staged row shared by 32 warps (two CTAs per SM)
 
@@ -155,102 +161,178 @@ __global__ void __launch_bounds__(kPT) k_pair_up(const PairPlan* __restrict__ pp
   }
 }
 
-// NR rows u of the product order staged in shared memory; per column d the
-// down hops' table words are read once and serve all NR rows; per element
-// the hops and the diagonal are added to y_p and the result goes to its
-// reference-order slot with the sign S.  DOT: <x, y> summed per CTA in a
-// fixed order, then over CTAs (deterministic for a given grid).
-template <class E, int NR>
-struct alignas(sizeof(E) * NR) RowPack { E v[NR]; };
+// A 16-byte pack of NE elements that a hop reads with one load.
+template <class E, int NE>
+struct alignas(sizeof(E) * NE) RowPack { E v[NE]; };
 
-template <int DT, bool DOT, int NR>
-__global__ void __launch_bounds__(kDT) k_pair_dn(const PairPlan* __restrict__ pp, const void* __restrict__ xp,
-                                                 const void* __restrict__ yp, void* __restrict__ y,
-                                                 double* partials, unsigned* ticket, double* dot_out) {
+__device__ __forceinline__ double flip_sign(double v, uint32_t e) {  // -v when bit 15 of e is set
+  return __hiloint2double(__double2hiint(v) ^ int((e & 0x8000u) << 16), __double2loint(v));
+}
+__device__ __forceinline__ float flip_sign(float v, uint32_t e) {
+  return __int_as_float(__float_as_int(v) ^ int((e & 0x8000u) << 16));
+}
+
+// The hops of row c (tile c / 32) on the staged packs: sum over magnitudes of
+// magnitude * (sum of +-pack).  kAhead slot groups are loaded together, the
+// next ones while these are summed (Hubbard 4x4 float64, the whole kernel:
+// one group ahead 2.90 ms, four 2.67 ms).
+constexpr int kAhead = 4;
+template <class T, class Pack, int NE>
+__device__ __forceinline__ void hop_sum(const uint2* __restrict__ rec, const uint2* __restrict__ slot,
+                                        const double* mag, uint32_t c, const Pack* xs, typename T::R (&sr)[NE],
+                                        typename T::R (&si)[NE]) {
+  using R = typename T::R;
+  #pragma unroll
+  for (int r = 0; r < NE; ++r) { sr[r] = R(0); si[r] = R(0); }
+  const uint2 t = __ldg(rec + c / 32);
+  const uint2* __restrict__ g = slot + size_t(t.x) * 32 + (c & 31u);
+  for (int m = 0; m < kMags; ++m) {
+    const uint32_t ng = (t.y >> (8 * m)) & 0xFFu;
+    if (ng == 0) break;
+    R ar[NE], ai[NE];
+    #pragma unroll
+    for (int r = 0; r < NE; ++r) { ar[r] = R(0); ai[r] = R(0); }
+    auto hop = [&](uint32_t e) {
+      const Pack pk = xs[e & 0x7FFFu];
+      #pragma unroll
+      for (int r = 0; r < NE; ++r) {
+        if constexpr (T::cplx) {
+          ar[r] += flip_sign(pk.v[r].x, e);
+          ai[r] += flip_sign(pk.v[r].y, e);
+        } else {
+          ar[r] += flip_sign(pk.v[r], e);
+        }
+      }
+    };
+    uint2 q[kAhead];
+    #pragma unroll
+    for (int u = 0; u < kAhead; ++u)
+      if (uint32_t(u) < ng) q[u] = __ldg(g + u * 32);
+    for (uint32_t j = 0; j < ng; j += kAhead) {
+      uint2 w[kAhead];
+      #pragma unroll
+      for (int u = 0; u < kAhead; ++u) {
+        w[u] = q[u];
+        if (j + kAhead + u < ng) q[u] = __ldg(g + (j + kAhead + u) * 32);
+      }
+      #pragma unroll
+      for (int u = 0; u < kAhead; ++u)
+        if (j + u < ng) {
+          hop(w[u].x & 0xFFFFu);
+          hop(w[u].x >> 16);
+          hop(w[u].y & 0xFFFFu);
+          hop(w[u].y >> 16);
+        }
+    }
+    g += ng * 32;
+    const R f = R(mag[m]);
+    #pragma unroll
+    for (int r = 0; r < NE; ++r) { sr[r] += f * ar[r]; si[r] += f * ai[r]; }
+  }
+}
+
+// NE * PL rows u of the product order staged in shared memory as PL planes
+// of NE interleaved rows (16 bytes per column), so that one load fetches a
+// column of NE rows; per column d the down hops are decoded once for all rows
+// (SLOTS: from the by-hop tables, one plane; otherwise a CSR walk); per element the hops and the diagonal are added to y_p and the result
+// goes to its reference-order slot with the sign S.  DOT: <x, y> summed per
+// CTA in a fixed order, then over CTAs (deterministic for a given grid).
+template <int DT, bool DOT, int NE, int PL, int NT, bool SLOTS>
+__global__ void __launch_bounds__(NT) k_pair_dn(const PairPlan* __restrict__ pp, const void* __restrict__ xp,
+                                                const void* __restrict__ yp, void* __restrict__ y,
+                                                double* partials, unsigned* ticket, double* dot_out) {
   using T = VT<DT>;
   using R = typename T::R;
   using E = typename T::E;
+  constexpr int NR = NE * PL;
+  using Pack = RowPack<E, NE>;
   extern __shared__ __align__(16) unsigned char smraw[];
-  // the NR rows interleaved: element (r, d) at d * NR + r, so one vector
-  // load fetches a column of all NR rows
-  using Pack = RowPack<E, NR>;
-  E* xs = reinterpret_cast<E*>(smraw);
-  const Pack* xsp = reinterpret_cast<const Pack*>(smraw);
-  __shared__ double s_red[2 * (kDT / 32)];
+  Pack* xs = reinterpret_cast<Pack*>(smraw);
+  __shared__ double s_red[2 * (NT / 32)];
   const PairPlan& p = *pp;
-  const uint32_t Dd = p.Dd;
+  const uint32_t Dd = p.Dd, stride = Dd + 8;
   double dr = 0.0, di = 0.0;
-  const bool packed = p.dn_ent != nullptr;
-  const R mag = R(p.dn_mag);
   auto split = [](const E& v, R& re, R& im) {
     if constexpr (T::cplx) { re = v.x; im = v.y; } else { re = v; im = R(0); }
   };
+  if (threadIdx.x < 8 * PL) {  // slots without a target
+    Pack z;
+    #pragma unroll
+    for (int r = 0; r < NE; ++r) z.v[r] = E{};
+    xs[(threadIdx.x / 8) * stride + Dd + threadIdx.x % 8] = z;
+  }
   for (uint32_t iu0 = blockIdx.x * NR; iu0 < p.Du; iu0 += gridDim.x * NR) {
     const uint32_t nr = min(uint32_t(NR), p.Du - iu0);
     __syncthreads();  // the previous rows are finished with the staging
-    for (uint32_t i = threadIdx.x; i < nr * Dd; i += kDT) {
-      const uint32_t r = i / Dd, c = i - r * Dd;
-      xs[c * NR + r] = reinterpret_cast<const E*>(xp)[uint64_t(iu0) * Dd + i];
+    for (uint32_t c = threadIdx.x; c < Dd; c += NT) {
+      #pragma unroll
+      for (int pl = 0; pl < PL; ++pl) {
+        Pack v;
+        #pragma unroll
+        for (int r = 0; r < NE; ++r) {
+          const uint32_t k = pl * NE + r;
+          v.v[r] = k < nr ? __ldg(reinterpret_cast<const E*>(xp) + uint64_t(iu0 + k) * Dd + c) : E{};
+        }
+        xs[pl * stride + c] = v;
+      }
     }
     __syncthreads();
-    for (uint32_t c = threadIdx.x; c < Dd; c += kDT) {
-      const uint32_t k0 = __ldg(p.dn_ptr + c), k1 = __ldg(p.dn_ptr + c + 1);
-      R sr[NR], si[NR];
+    for (uint32_t c = threadIdx.x; c < Dd; c += NT) {
+      const uint32_t d = __ldg(p.dlist + c);
+      // what the end of the row needs, in flight during the hops
+      R ar[NR], ai[NR];
+      double dg[NR];
+      uint32_t rk[NR];
       #pragma unroll
-      for (int r = 0; r < NR; ++r) { sr[r] = R(0); si[r] = R(0); }
-      if (packed) {
-        // four hops at a time: their table words, then their row values
-        auto hop = [&](uint32_t e) {
-          const Pack pk = xsp[e & 0x7FFFu];
-          #pragma unroll
-          for (int r = 0; r < NR; ++r) {
-            R vr, vi;
-            split(pk.v[r], vr, vi);
-            if (e & 0x8000u) { sr[r] -= vr; if (T::cplx) si[r] -= vi; }
-            else { sr[r] += vr; if (T::cplx) si[r] += vi; }
-          }
-        };
-        uint32_t k = k0;
-        for (; k + 4 <= k1; k += 4) {
-          uint32_t e[4];
-          #pragma unroll
-          for (int j = 0; j < 4; ++j) e[j] = __ldg(p.dn_ent + k + j);
-          #pragma unroll
-          for (int j = 0; j < 4; ++j) hop(e[j]);
-        }
-        for (; k < k1; ++k) hop(__ldg(p.dn_ent + k));
-        #pragma unroll
-        for (int r = 0; r < NR; ++r) { sr[r] *= mag; si[r] *= mag; }
+      for (int r = 0; r < NR; ++r) {
+        const uint32_t u = iu0 + (uint32_t(r) < nr ? r : 0);
+        const uint64_t i = uint64_t(u) * Dd + c;
+        T::ld(yp, i, ar[r], ai[r]);
+        dg[r] = __ldg(p.diag + i);
+        rk[r] = p.perm ? __ldg(p.perm + i) : pair_rank(p, __ldg(p.ulist + u), d);
+      }
+      R sr[NR], si[NR];
+      if constexpr (SLOTS) {
+        static_assert(PL == 1, "the by-hop tables serve one plane");
+        hop_sum<T, Pack, NE>(p.dn_rec, p.dn_slot, p.dn_mag, c, xs, sr, si);
       } else {
+        const uint32_t k0 = __ldg(p.dn_ptr + c), k1 = __ldg(p.dn_ptr + c + 1);
+        #pragma unroll
+        for (int r = 0; r < NR; ++r) { sr[r] = R(0); si[r] = R(0); }
         for (uint32_t k = k0; k < k1; ++k) {
-          const Pack pk = xsp[__ldg(p.dn_col + k)];
+          const uint32_t t = __ldg(p.dn_col + k);
           const R w = R(__ldg(p.dn_val + k));
           #pragma unroll
-          for (int r = 0; r < NR; ++r) {
-            R vr, vi;
-            split(pk.v[r], vr, vi);
-            sr[r] += w * vr;
-            if (T::cplx) si[r] += w * vi;
+          for (int pl = 0; pl < PL; ++pl) {
+            const Pack pk = xs[pl * stride + t];
+            #pragma unroll
+            for (int r = 0; r < NE; ++r) {
+              R vr, vi;
+              split(pk.v[r], vr, vi);
+              sr[pl * NE + r] += w * vr;
+              if (T::cplx) si[pl * NE + r] += w * vi;
+            }
           }
         }
       }
-      const uint32_t d = __ldg(p.dlist + c);
       #pragma unroll
-      for (int r = 0; r < NR; ++r) {
-        if (uint32_t(r) >= nr) break;
-        const uint64_t i = uint64_t(iu0 + r) * Dd + c;
-        R ar, ai, xr, xi;
-        T::ld(yp, i, ar, ai);
-        split(xs[c * NR + r], xr, xi);
-        const R dg = R(__ldg(p.diag + i));
-        ar += dg * xr + sr[r];
-        if (T::cplx) ai += dg * xi + si[r];
-        const uint32_t u = __ldg(p.ulist + iu0 + r);
-        const R sg = R(pair_sign(u, d));
-        T::st(y, p.perm ? __ldg(p.perm + i) : pair_rank(p, u, d), sg * ar, sg * ai);
-        if (DOT) {  // <x, y> = <x_p, y_p> (S^2 = 1)
-          dr += double(xr) * double(ar) + double(xi) * double(ai);
-          di += double(xr) * double(ai) - double(xi) * double(ar);
+      for (int pl = 0; pl < PL; ++pl) {
+        const Pack own = xs[pl * stride + c];
+        #pragma unroll
+        for (int q = 0; q < NE; ++q) {
+          const int r = pl * NE + q;
+          if (uint32_t(r) < nr) {
+            R xr, xi;
+            split(own.v[q], xr, xi);
+            ar[r] += R(dg[r]) * xr + sr[r];
+            if (T::cplx) ai[r] += R(dg[r]) * xi + si[r];
+            const R sg = R(pair_sign(__ldg(p.ulist + iu0 + r), d));
+            T::st(y, rk[r], sg * ar[r], sg * ai[r]);
+            if (DOT) {  // <x, y> = <x_p, y_p> (S^2 = 1)
+              dr += double(xr) * double(ar[r]) + double(xi) * double(ai[r]);
+              di += double(xr) * double(ai[r]) - double(xi) * double(ar[r]);
+            }
+          }
         }
       }
     }
@@ -299,6 +381,76 @@ int host_pair_sign(uint32_t u, uint32_t d, int nsites) {
   return (c & 1) ? -1 : 1;
 }
 }  // namespace
+
+// By-hop tables of a sparse matrix in CSR form (hop[k]: the hop of entry k,
+// at most one entry per row and hop): per tile of 32 rows and magnitude one
+// slot for every hop with an entry in at least one row.  Rows without the hop
+// point at one of eight zero packs behind the staged rows, the one whose
+// 16-byte bank group no target of their quarter warp uses, so they cost no
+// extra wavefront (4x4 torus, 8 particles: 120 wavefronts per warp; one shared
+// zero pack 157, lists packed per row 155).  False when the elements have more
+// than kMags magnitudes.
+static bool hop_slots(const std::vector<uint32_t>& ptr, const std::vector<uint32_t>& col,
+                      const std::vector<double>& val, const std::vector<uint16_t>& hop, size_t nhop, double* mag,
+                      std::vector<uint2>& rec, std::vector<uint2>& slot) {
+  const uint32_t n = uint32_t(ptr.size() - 1);
+  if (n + 8 > 0x8000u) return false;
+  int nmag = 0;
+  std::vector<uint8_t> cls(val.size());
+  for (size_t k = 0; k < val.size(); ++k) {
+    int m = 0;
+    while (m < nmag && mag[m] != std::abs(val[k])) ++m;
+    if (m == kMags) return false;
+    if (m == nmag) mag[nmag++] = std::abs(val[k]);
+    cls[k] = uint8_t(m);
+  }
+  constexpr uint16_t kNone = 0xFFFFu;
+  std::vector<uint16_t> s(std::max<size_t>(nhop, 1) * 32);  // [hop][lane] of one magnitude
+  std::vector<uint8_t> used(std::max<size_t>(nhop, 1));
+  for (uint32_t r0 = 0; r0 < n; r0 += 32) {
+    uint2 rc = make_uint2(uint32_t(slot.size() / 32), 0u);
+    int out = 0;
+    // magnitudes without an entry in this tile would end the kernel's walk
+    // early, so every tile lists all of them: an absent one gets a group of
+    // zero packs unless no later one is present
+    int last = -1;
+    for (uint32_t k = ptr[r0]; k < ptr[std::min(n, r0 + 32)]; ++k) last = std::max(last, int(cls[k]));
+    for (int m = 0; m <= last; ++m, ++out) {
+      std::fill(s.begin(), s.end(), kNone);
+      std::fill(used.begin(), used.end(), uint8_t(0));
+      for (uint32_t i = 0; i < 32 && r0 + i < n; ++i)
+        for (uint32_t k = ptr[r0 + i]; k < ptr[r0 + i + 1]; ++k)
+          if (cls[k] == m) {
+            s[size_t(hop[k]) * 32 + i] = uint16_t(col[k] | (val[k] < 0 ? 0x8000u : 0u));
+            used[hop[k]] = 1;
+          }
+      std::vector<uint32_t> on;
+      for (uint32_t q = 0; q < nhop; ++q) if (used[q]) on.push_back(q);
+      for (uint32_t q : on)
+        for (uint32_t ph = 0; ph < 32; ph += 8) {  // quarter warps
+          uint32_t banks = 0, z = 0;
+          for (uint32_t i = ph; i < ph + 8; ++i)
+            if (s[q * 32 + i] != kNone) banks |= 1u << (s[q * 32 + i] & 7u);
+          while (z < 7 && (banks >> ((n + z) & 7u) & 1u)) ++z;
+          for (uint32_t i = ph; i < ph + 8; ++i)
+            if (s[q * 32 + i] == kNone) s[q * 32 + i] = uint16_t(n + z);
+        }
+      const uint32_t ng = std::max<uint32_t>(1, uint32_t((on.size() + 3) / 4));
+      if (ng > 255) return false;
+      rc.y |= ng << (8 * out);
+      for (uint32_t g = 0; g < ng; ++g)
+        for (uint32_t i = 0; i < 32; ++i) {
+          uint32_t t[4];
+          for (uint32_t u = 0; u < 4; ++u)  // padding: one address, a broadcast
+            t[u] = 4 * g + u < on.size() ? s[size_t(on[4 * g + u]) * 32 + i] : n;
+          slot.push_back(make_uint2(t[0] | (t[1] << 16), t[2] | (t[3] << 16)));
+        }
+    }
+    rec.push_back(rc);
+  }
+  if (slot.empty()) slot.push_back(make_uint2(0, 0));
+  return true;
+}
 
 // Host side: eligibility, T_up / T_dn from the compiled terms (the matrix
 // element of row s is the term's coefficient with its parity sign, target
@@ -353,12 +505,15 @@ PairHandle* pair_plan_create(const qk_plan_desc* d, const uint64_t* A_dev, const
   for (uint32_t i = 0; i < dl.size(); ++i) didx[dl[i]] = i;
   // row `a` of T_species at a fixed configuration `o` of the other species:
   // (column index, value) pairs in term order
+  std::vector<uint16_t> hop;  // of each pair: its position among the species' groups
   auto row = [&](bool up, uint32_t a, uint32_t o, std::vector<std::pair<uint32_t, double>>& out) -> bool {
     out.clear();
+    hop.clear();
     const uint64_t s = up ? interleave(a, o, ns) : interleave(o, a, ns);
     const int ss = up ? host_pair_sign(a, o, ns) : host_pair_sign(o, a, ns);
-    for (uint32_t gi : (up ? gup : gdn)) {
-      const qk_group_t& g = d->groups[gi];
+    const std::vector<uint32_t>& groups = up ? gup : gdn;
+    for (size_t gq = 0; gq < groups.size(); ++gq) {
+      const qk_group_t& g = d->groups[groups[gq]];
       const uint64_t t = s ^ g.flip;
       double c = 0.0;
       for (uint32_t q = g.first; q < g.first + g.count; ++q) {
@@ -374,11 +529,13 @@ PairHandle* pair_plan_create(const qk_plan_desc* d, const uint64_t* A_dev, const
       if (idx == ~0u) return false;
       const int ts = up ? host_pair_sign(a2, o, ns) : host_pair_sign(o, a2, ns);
       out.push_back({idx, double(ss * ts) * c});
+      hop.push_back(uint16_t(gq));
     }
     return true;
   };
   std::vector<uint32_t> uptr(1, 0), ucol, dptr(1, 0), dcol;
   std::vector<double> uval, dval;
+  std::vector<uint16_t> dhop;
   std::vector<std::pair<uint32_t, double>> r, r2;
   const uint32_t o_chk[2][2] = {{dl[dl.size() / 2], dl.back()}, {ul[ul.size() / 2], ul.back()}};
   for (int sp = 0; sp < 2; ++sp) {
@@ -394,16 +551,15 @@ PairHandle* pair_plan_create(const qk_plan_desc* d, const uint64_t* A_dev, const
         (up ? ucol : dcol).push_back(e.first);
         (up ? uval : dval).push_back(e.second);
       }
+      // the last call above was for another configuration of the other
+      // species with the same result, so its hops are this row's
+      if (!up) dhop.insert(dhop.end(), hop.begin(), hop.end());
       (up ? uptr : dptr).push_back(uint32_t((up ? ucol : dcol).size()));
     }
   }
-  // down hops packed as column | sign when they share one magnitude
-  double mag = dval.empty() ? 1.0 : std::abs(dval[0]);
-  bool uniform = true;
-  for (double v : dval) uniform = uniform && std::abs(v) == mag;
-  std::vector<uint16_t> dent;
-  if (uniform)
-    for (size_t k = 0; k < dcol.size(); ++k) dent.push_back(uint16_t(dcol[k] | (dval[k] < 0 ? 0x8000u : 0u)));
+  std::vector<uint2> drec, dslot;
+  double dmag[kMags] = {0.0, 0.0, 0.0, 0.0};
+  const bool dslots = hop_slots(dptr, dcol, dval, dhop, gdn.size(), dmag, drec, dslot);
   auto* out = new PairHandle;
   bool ok = true;
   auto up_ = [&](const void* src, size_t bytes) -> void* {
@@ -426,13 +582,14 @@ PairHandle* pair_plan_create(const qk_plan_desc* d, const uint64_t* A_dev, const
   h.up_col = static_cast<const uint32_t*>(up_(ucol.data(), ucol.size() * 4));
   h.up_val = static_cast<const double*>(up_(uval.data(), uval.size() * 8));
   h.dn_ptr = static_cast<const uint32_t*>(up_(dptr.data(), dptr.size() * 4));
-  if (uniform) {
-    h.dn_ent = static_cast<const uint16_t*>(up_(dent.data(), dent.size() * 2));
+  if (dslots) {
+    h.dn_rec = static_cast<const uint2*>(up_(drec.data(), drec.size() * sizeof(uint2)));
+    h.dn_slot = static_cast<const uint2*>(up_(dslot.data(), dslot.size() * sizeof(uint2)));
   } else {
     h.dn_col = static_cast<const uint32_t*>(up_(dcol.data(), dcol.size() * 4));
     h.dn_val = static_cast<const double*>(up_(dval.data(), dval.size() * 8));
   }
-  h.dn_mag = mag;
+  for (int m = 0; m < kMags; ++m) h.dn_mag[m] = dmag[m];
   double* dp = static_cast<double*>(up_(nullptr, d->dim * 8));
   h.diag = dp;
   if (ok) {
@@ -477,50 +634,69 @@ int pair_apply(const PairHandle* h, qk_dtype t, const void* x, void* y, cudaStre
                double* dot_out) {
   if (!h || !x || !y || x == y) return QKD_EINVAL;
   const size_t es = qk_dtype_size(t), n = size_t(h->host.Du) * h->host.Dd;
+  const size_t half = (n * es + 255) & ~size_t(255);  // x_p and y_p both on 256-byte boundaries
   void* scr = nullptr;
   {
     std::lock_guard<std::mutex> lk(h->mu);
-    if (h->scr_bytes < 2 * n * es) {
+    if (h->scr_bytes < 2 * half) {
       cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
       if (cudaStreamIsCapturing(s, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone) return QKD_EINVAL;
       cudaFree(h->scr);
       h->scr = nullptr;
       h->scr_bytes = 0;
-      if (cudaMalloc(&h->scr, 2 * n * es) != cudaSuccess) {
+      if (cudaMalloc(&h->scr, 2 * half) != cudaSuccess) {
         (void)cudaGetLastError();
         return QKD_EINVAL;
       }
-      h->scr_bytes = 2 * n * es;
+      h->scr_bytes = 2 * half;
     }
     scr = h->scr;
   }
   void* xp = scr;
-  void* yp = static_cast<char*>(scr) + n * es;
-  // rows staged per pass of the down-hop kernel: as many as 220 KB hold (1, 2
-  // or 4; a CTA may use up to 227 KB of shared memory)
+  void* yp = static_cast<char*>(scr) + half;
+  // rows staged per pass of the down-hop kernel: as many as fill 16 bytes per
+  // column (fewer where the stage cannot hold them); the CSR walk, which the
+  // decoding bounds, takes up to four
   constexpr size_t kStage = 220 * 1024;
-  const size_t row_bytes = es * h->host.Dd;
-  if (row_bytes > kStage) return QKD_EINVAL;
-  const int nr = row_bytes * 4 <= kStage ? 4 : row_bytes * 2 <= kStage ? 2 : 1;
-  const size_t smem = row_bytes * nr;
-#define QKD_PAIR_DN(DT, DOT, NR)                                                                           \
+  const size_t cols = size_t(h->host.Dd) + 8;
+  if (es * size_t(h->host.Dd) > kStage) return QKD_EINVAL;
+  int ne = int(std::max<size_t>(1, std::min<size_t>(16 / es, kStage / (es * cols))));
+  ne = ne >= 4 ? 4 : ne >= 2 ? 2 : 1;
+  int pl = 1;
+  if (!h->host.dn_rec && size_t(ne) * es == 16)
+    while (ne * pl < 4 && es * cols * ne * pl * 2 <= kStage) pl *= 2;
+  const size_t smem = es * cols * ne * pl;
+#define QKD_PAIR_DN1(DT, DOT, NE, PL, NT, SL)                                                               \
   {                                                                                                        \
-    auto k = k_pair_dn<DT, DOT, NR>;                                                                       \
+    auto k = k_pair_dn<DT, DOT, NE, PL, NT, SL>;                                                           \
     if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess)     \
       return QKD_EINVAL;                                                                                   \
-    const unsigned rows = (h->host.Du + NR - 1) / NR;                                                      \
-    const unsigned g = resident_grid(k, kDT, smem, DOT ? std::min<unsigned>(rows, kMaxG) : rows);          \
-    k<<<g, kDT, smem, s>>>(h->dev, xp, yp, y, DOT ? w->partials : nullptr, DOT ? w->ticket : nullptr, dot_out); \
+    const unsigned rows = (h->host.Du + NE * PL - 1) / (NE * PL);                                          \
+    const unsigned g = resident_grid(k, NT, smem, DOT ? std::min<unsigned>(rows, kMaxG) : rows);           \
+    k<<<g, NT, smem, s>>>(h->dev, xp, yp, y, DOT ? w->partials : nullptr, DOT ? w->ticket : nullptr, dot_out); \
+  }
+#define QKD_PAIR_DN(DT, DOT, NE)                                                                           \
+  {                                                                                                        \
+    constexpr bool full = NE * sizeof(VT<DT>::E) == 16;                                                    \
+    if (h->host.dn_rec) {                                                                                  \
+      if (smem <= kStage / 2) QKD_PAIR_DN1(DT, DOT, NE, 1, 512, true)                                      \
+      else QKD_PAIR_DN1(DT, DOT, NE, 1, kDT, true)                                                         \
+    } else if (full && pl == 4) QKD_PAIR_DN1(DT, DOT, NE, (full && NE == 1 ? 4 : 1), kDT, false)           \
+    else if (full && pl == 2) QKD_PAIR_DN1(DT, DOT, NE, (full && NE <= 2 ? 2 : 1), kDT, false)             \
+    else QKD_PAIR_DN1(DT, DOT, NE, 1, kDT, false)                                                          \
+  }
+#define QKD_PAIR_DNS(DT, DOT)                                                                              \
+  {                                                                                                        \
+    constexpr int MAXR = 16 / int(sizeof(VT<DT>::E));                                                      \
+    if constexpr (MAXR >= 4) { if (ne == 4) QKD_PAIR_DN(DT, DOT, 4) }                                      \
+    if constexpr (MAXR >= 2) { if (ne == 2) QKD_PAIR_DN(DT, DOT, 2) }                                      \
+    if (ne == 1) QKD_PAIR_DN(DT, DOT, 1)                                                                   \
   }
 #define QKD_PAIR(DT)                                                                                       \
   {                                                                                                        \
     k_pair_in<DT, true><<<resident_grid(k_pair_in<DT, true>, kPT, 0, 1u << 20), kPT, 0, s>>>(h->dev, x, xp); \
-    k_pair_up<DT><<<resident_grid(k_pair_up<DT>, kPT, 0, 1u << 20), kPT, 0, s>>>(h->dev, xp, yp);       \
-    if (dot_out) {                                                                                         \
-      if (nr == 4) QKD_PAIR_DN(DT, true, 4) else if (nr == 2) QKD_PAIR_DN(DT, true, 2) else QKD_PAIR_DN(DT, true, 1) \
-    } else {                                                                                               \
-      if (nr == 4) QKD_PAIR_DN(DT, false, 4) else if (nr == 2) QKD_PAIR_DN(DT, false, 2) else QKD_PAIR_DN(DT, false, 1) \
-    }                                                                                                      \
+    k_pair_up<DT><<<resident_grid(k_pair_up<DT>, kPT, 0, 1u << 20), kPT, 0, s>>>(h->dev, xp, yp);          \
+    if (dot_out) QKD_PAIR_DNS(DT, true) else QKD_PAIR_DNS(DT, false)                                       \
   }
   switch (t) {
     case QK_C128: QKD_PAIR(QK_C128); break;
@@ -530,7 +706,9 @@ int pair_apply(const PairHandle* h, qk_dtype t, const void* x, void* y, cudaStre
     default: return QKD_EINVAL;
   }
 #undef QKD_PAIR
+#undef QKD_PAIR_DNS
 #undef QKD_PAIR_DN
+#undef QKD_PAIR_DN1
   QKD_LAUNCH_CHECK();
   return QKD_OK;
 }
