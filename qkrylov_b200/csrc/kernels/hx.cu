@@ -10,6 +10,7 @@
 // consecutive addresses (coalesced); terms that flip low bits stay inside
 // the block, which L1 holds.  Each thread writes only its own y[row].
 #include <algorithm>
+#include <mutex>
 #include <vector>
 
 #include "reduce.cuh"
@@ -26,6 +27,12 @@ PairHandle* pair_plan_create(const qk_plan_desc* d, const uint64_t* A_dev, const
 void pair_plan_destroy(PairHandle* h);
 int pair_apply(const PairHandle* h, qk_dtype t, const void* x, void* y, cudaStream_t s, qk_workspace* w,
                double* dot_out);
+struct BlockListHandle;
+BlockListHandle* block_list_create(const DevPlan& p, uint64_t dim, const double* diag, size_t max_bytes,
+                                   size_t* dev_bytes);
+void block_list_destroy(BlockListHandle* h);
+int block_list_apply(const BlockListHandle* h, qk_dtype t, int R, int lpr, bool queues, const void* X, void* Y,
+                     double* dots, cudaStream_t s, const double* gacc);
 struct FlipHandle;
 bool flip_eligible(const qk_plan_desc* d);
 FlipHandle* flip_plan_create(const qk_plan_desc* d, const double* diag, size_t* dev_bytes);
@@ -51,6 +58,7 @@ int spin_apply(const SpinHandle* h, qk_dtype t, const void* x, void* y, cudaStre
 
 static int g_kernel_policy = 0;  // 0: specialised kernels where eligible, 1: generic only
 static bool g_pair_path = true;  // the spin-product path of Hubbard-type operators
+static bool g_die_queues = true;  // per-die work queues
 static bool g_list_path = true;  // the row lists of small sectors, the flips of complete bases
 
 struct qk_plan {
@@ -73,6 +81,9 @@ struct qk_plan {
   size_t bytes, smem;
   int rows_lpr[4][3];   // autotuned lanes per row of the block apply, by dtype and R = 32, 64, 128
   int rows_tile[4][3];  // autotuned tile shape of the block apply (row kernels: 256 / 128 / 512 rows)
+  int rows_list[4][3];  // lanes per row of the packed-list block kernel where it was the fastest, else 0
+  size_t block_list_tried;  // largest size the packed lists were refused
+  qkd::BlockListHandle* block_list;  // packed lists of the block apply, built by the tuner
   float rows_ms[4][3][9];  // the tuner's fastest launch (ms) per lanes per row (32/16/8) x tile code; 0: untimed
   double* diag_re;     // real diagonal (generic-kernel operators with a real diagonal), else null
 };
@@ -389,27 +400,38 @@ int launch_block_shape(const qk_plan* p, qk_workspace* w, int R, int lpr, const 
   return QKD_EINVAL;
 }
 
+// The real diagonal of a real operator as a device vector, made on first use
+// where the plan has none; null without a diagonal or without memory.
+const double* real_diag(qk_plan* p) {
+  if (!p->has_diag || p->diag_re) return p->diag_re;
+  if (!p->list_diag) {
+    if (cudaMalloc(&p->list_diag, p->dim * 8) != cudaSuccess) {
+      (void)cudaGetLastError();
+      p->list_diag = nullptr;
+    } else if (qkd_diagonal(p, QK_F64, p->list_diag, nullptr) != QKD_OK || cudaStreamSynchronize(nullptr) != cudaSuccess) {
+      (void)cudaGetLastError();
+      cudaFree(p->list_diag);
+      p->list_diag = nullptr;
+    } else {
+      p->bytes += p->dim * 8;
+    }
+  }
+  return p->list_diag;
+}
+
 // The table-free kernel of unconditional flips, else the row lists of a small
 // sector, with the real diagonal they need.
 void make_lists(qk_plan* p, const qk_plan_desc* d) {
   const bool flips = flip_eligible(d);
-  if (!flips && p->dim > (1ull << 24)) return;
-  const double* diag = p->diag_re;
-  if (p->has_diag && !diag) {
-    if (cudaMalloc(&p->list_diag, p->dim * 8) != cudaSuccess) {
-      (void)cudaGetLastError();
-      return;
-    }
-    if (qkd_diagonal(p, QK_F64, p->list_diag, nullptr) == QKD_OK) diag = p->list_diag;
-  }
-  if (!p->has_diag || diag) {
-    if (flips) p->flip = flip_plan_create(d, diag, &p->bytes);
-    if (!p->flip) p->list = list_plan_create(dev(p), p->dim, diag, &p->bytes);
-  }
-  if ((p->list || p->flip) && p->list_diag) p->bytes += p->dim * 8;
-  if (!p->list && !p->flip) {
+  if (!flips && size_t(p->dim) * 16 > (size_t(64) << 20)) return;  // no list of that many rows fits
+  const double* diag = real_diag(p);
+  if (p->has_diag && !diag) return;
+  if (flips) p->flip = flip_plan_create(d, diag, &p->bytes);
+  if (!p->flip) p->list = list_plan_create(dev(p), p->dim, diag, &p->bytes);
+  if (!p->list && !p->flip && p->list_diag) {
     cudaFree(p->list_diag);
     p->list_diag = nullptr;
+    p->bytes -= p->dim * 8;
   }
 }
 
@@ -502,6 +524,7 @@ int qkd_set_kernel_policy(int policy) {
   g_kernel_policy = policy == 1 ? 1 : 0;
   g_list_path = policy != 3;
   qkd::spin_set_die_queues(policy != 2);
+  g_die_queues = policy != 2;
   g_pair_path = policy != 3;
   return QKD_OK;
 }
@@ -516,6 +539,7 @@ int qkd_plan_kernel(const qk_plan* p) {
 int qkd_plan_destroy(qk_plan* p) {
   if (!p) return QKD_OK;
   qkd::list_plan_destroy(p->list);
+  qkd::block_list_destroy(p->block_list);
   qkd::flip_plan_destroy(p->flip);
   qkd::pair_plan_destroy(p->pair);
   qkd::spin_plan_destroy(p->spin);
@@ -620,6 +644,11 @@ int qkd_apply_rows(const qk_plan* p, qk_workspace* w, qk_dtype t, int R, int lan
   if (!p || r_index(R) < 0 || t < QK_C128 || t > QK_F32) return QKD_EINVAL;
   const int lpr = lanes_per_row ? lanes_per_row : (p->rows_lpr[t][r_index(R)] ? p->rows_lpr[t][r_index(R)] : 32);
   const int tilec = lanes_per_row ? 0 : p->rows_tile[t][r_index(R)];
+  const int list = lanes_per_row ? 0 : p->rows_list[t][r_index(R)];
+  if (list && w && X && Y && X != Y && g_kernel_policy == 0 && g_list_path) {
+    const int rc = block_list_apply(p->block_list, t, R, list, g_die_queues, X, Y, dots, s, nullptr);
+    if (rc != QKD_EINVAL) return rc;
+  }
   return apply_rows_shape(p, w, t, R, lpr, tilec, X, Y, diag, nullptr, dots, s);
 }
 
@@ -628,6 +657,11 @@ int qkd_apply_rows_acc(const qk_plan* p, qk_workspace* w, qk_dtype t, int R, int
   if (!p || !g || r_index(R) < 0 || t < QK_C128 || t > QK_F32) return QKD_EINVAL;
   const int lpr = lanes_per_row ? lanes_per_row : (p->rows_lpr[t][r_index(R)] ? p->rows_lpr[t][r_index(R)] : 32);
   const int tilec = lanes_per_row ? 0 : p->rows_tile[t][r_index(R)];
+  const int list = lanes_per_row ? 0 : p->rows_list[t][r_index(R)];
+  if (list && w && X && Y && X != Y && p->spin && g_kernel_policy == 0 && g_list_path) {
+    const int rc = block_list_apply(p->block_list, t, R, list, g_die_queues, X, Y, dots, s, g);
+    if (rc != QKD_EINVAL) return rc;
+  }
   return apply_rows_shape(p, w, t, R, lpr, tilec, X, Y, nullptr, g, dots, s);
 }
 
@@ -685,6 +719,38 @@ static int tune_rows(qk_plan* p, qk_workspace* w, qk_dtype t, int R, const void*
   for (int q = 0; q < 3; ++q)
     for (int tc = 0; tc < 3; ++tc)
       p->rows_ms[t][r_index(R)][q * 3 + tc] = (tc < ntile && fastest[q][tc] < 1e29f) ? fastest[q][tc] : 0.f;
+  // the packed lists (4 bytes per target against R elements of its row; at
+  // most half a block vector) against the best of those shapes
+  int pick_list = 0;
+  static std::mutex build_mu;  // two threads may tune the same plan
+  std::unique_lock<std::mutex> build(build_mu);
+  const size_t list_max = size_t(p->dim) * R * qk_dtype_size(t) / 2;
+  if (p->all_real && !p->block_list && g_kernel_policy == 0 && g_list_path && list_max > p->block_list_tried) {
+    p->block_list_tried = list_max;
+    if (const double* dv = real_diag(p); dv || !p->has_diag)
+      p->block_list = block_list_create(dev(p), p->dim, dv, list_max, &p->bytes);
+  }
+  build.unlock();
+  if (p->block_list && g_kernel_policy == 0 && g_list_path) {
+    cudaEvent_t s0, s1;
+    if (cudaEventCreate(&s0) != cudaSuccess || cudaEventCreate(&s1) != cudaSuccess) return QKD_ECUDA;
+    for (int q = 0; q < 3; ++q) {
+      if (R / lprs[q] > 8) continue;
+      for (int i = 0; i < 5; ++i) {  // the first is a warm-up, and sizes the dots' partials before a capture
+        cudaEventRecord(s0, s);
+        if (block_list_apply(p->block_list, t, R, lprs[q], g_die_queues, X, Y, i ? nullptr : qkd_workspace_results(w), s, g) != QKD_OK)
+          break;
+        cudaEventRecord(s1, s);
+        float ms = 0.f;
+        if (cudaEventSynchronize(s1) != cudaSuccess || cudaEventElapsedTime(&ms, s0, s1) != cudaSuccess) break;
+        if (i && ms < best) { best = ms; pick_list = lprs[q]; }
+      }
+    }
+    cudaEventDestroy(s0);
+    cudaEventDestroy(s1);
+    (void)cudaGetLastError();
+  }
+  p->rows_list[t][r_index(R)] = pick_list;
   p->rows_lpr[t][r_index(R)] = pick;
   p->rows_tile[t][r_index(R)] = pick_tc;
   if (chosen) *chosen = pick;

@@ -21,6 +21,7 @@
 // c128 18.5 -> 6.2, transverse Ising N=18 f64 16.4 -> 10.3.
 #include <algorithm>
 #include <cstring>
+#include <mutex>
 #include <vector>
 
 #include "hx_terms.cuh"
@@ -53,6 +54,28 @@ struct ListHandle {
   ListPlan plan{};
   void* bufs[3] = {};
 };
+
+struct BlockListPlan {
+  uint32_t dim;
+  const uint32_t* start;  // per row: first 4-word group (dim + 1)
+  const uint4* words;
+  const double* diag;     // or null
+  uint32_t* wq;           // per-die tile queues (null: grid-stride)
+  const uint8_t* sm_die;
+  uint32_t nsmid;
+  int n0, n1;             // SMs per die
+  double coef[kListClasses];
+};
+
+struct BlockListHandle {
+  BlockListPlan plan{};
+  void* bufs[3] = {};
+  mutable std::mutex mu;
+  mutable double* part = nullptr;  // per-tile column dots, sized on first use
+  mutable size_t part_cap = 0;
+};
+
+bool die_map(const uint8_t** dev_map, int* nsmid, int* n0, int* n1);
 
 namespace {
 
@@ -114,6 +137,220 @@ __global__ void __launch_bounds__(256) k_list_build(DevPlan p, uint32_t dim, con
     if (FILL)
       for (; n % 4; ++n) words[(size_t(start[sl]) + n / 4) * 128 + lane * 4 + n % 4] = 0u;
   }
+}
+
+// Packed lists for blocks of vectors: FILL false: targets of every row (and
+// the coefficient table); FILL true: the words, at 4 * start[row], padded to
+// whole groups of four with words of class 0.  One thread per row.
+template <bool FILL>
+__global__ void __launch_bounds__(256) k_packed_build(DevPlan p, uint32_t dim, const uint64_t* __restrict__ st,
+                                                      uint32_t* __restrict__ start, uint32_t* __restrict__ words,
+                                                      unsigned long long* table, int* overflow) {
+  for (uint32_t row = blockIdx.x * 256 + threadIdx.x; row < dim; row += gridDim.x * 256) {
+    const uint64_t s = st[row];
+    uint32_t n = 0;
+    uint32_t* out = FILL ? words + size_t(start[row]) * 4 : nullptr;
+    for (uint32_t g = p.has_diag ? 1u : 0u; g < p.ngroups; ++g) {
+      const qk_group_t grp = p.groups[g];
+      double c, ci;
+      if (!group_coef<false, double>(p.terms, grp.first, grp.count, s, c, ci)) continue;
+      const uint64_t t = s ^ grp.flip;
+      const uint64_t a = __ldg(p.A + (t >> p.L));
+      const uint32_t b = __ldg(p.B + (t & p.lmask));
+      if (uint32_t(a >> 56) != (b >> 24)) continue;
+      const uint32_t cls = coef_class(c, table);
+      if (cls == uint32_t(kListClasses)) { *overflow = 1; continue; }
+      if (cls == 0) continue;
+      if (FILL) out[n] = uint32_t((a & qkb::kOffsetMask) + (b & qkb::kRankMask)) | (cls << 24);
+      ++n;
+    }
+    if (FILL) for (; n % 4; ++n) out[n] = 0u;
+    else start[row] = (n + 3) / 4;
+  }
+}
+
+// Y = H X (gacc: Y += diag(gacc) H X) for R = LPR * VPL row-interleaved
+// vectors from the packed lists: LPR lanes share a row, the words of a row are
+// one broadcast load per four targets, and the four target rows are in flight
+// together with nothing to decode between them.  The block kernels on the
+// sector tables chain about eleven dependent loads per row (record, groups,
+// masks, crossing words, then targets a few at a time) at 16 to 32 warps per
+// SM and are bound by that latency; the words are 4 bytes per target against
+// 128 to 1024 bytes of its row.  Registers for five CTAs per SM at up to 16
+// bytes per lane, three at 32: eight targets in flight at fewer CTAs were
+// 10-20% slower (t-J N=18, 64 float32 vectors: 757 us with 3 CTAs, 721 with 4,
+// four targets and 5 CTAs 624; J1-J2 N=24, 32 float64 vectors: 1774 us with 2
+// CTAs, four targets and 3 CTAs 1514).  Against k_hx_rows_block: those two
+// 1117 -> 624 and 2173 -> 1514 us; t-J N=20, 64 vectors float32 4.97 -> 3.41,
+// float64 9.24 -> 6.60 ms; t-J N=13, 64 float32 56 -> 18 us.  Tiles of
+// kBlockTile rows from a queue per die; column dots per tile (sum_items).
+constexpr uint32_t kBlockTile = 128;
+template <class E, int VPL> struct alignas(sizeof(E) * VPL >= 16 ? 16 : sizeof(E) * VPL) ListPack { E v[VPL]; };
+template <int DT> __device__ __forceinline__ void unpk(const typename VT<DT>::E& e, typename VT<DT>::R& re, typename VT<DT>::R& im) {
+  if constexpr (VT<DT>::cplx) { re = e.x; im = e.y; } else { re = e; im = typename VT<DT>::R(0); }
+}
+
+template <int DT, int LPR, int VPL, int MINC>
+__global__ void __launch_bounds__(256, MINC)
+k_hx_block_list(const __grid_constant__ BlockListPlan p, const void* __restrict__ X, void* __restrict__ Y,
+                const double* __restrict__ gacc, uint32_t ntiles, uint32_t qsplit, double* part) {
+  using T = VT<DT>;
+  using R = typename T::R;
+  using E = typename T::E;
+  using Pack = ListPack<E, VPL>;
+  constexpr int RV = LPR * VPL, RPW = 32 / LPR;
+  __shared__ R s_coef[kListClasses];
+  __shared__ double red[(256 / 32) * RV * 2];
+  __shared__ uint32_t s_tile[2];
+  if (threadIdx.x < kListClasses) s_coef[threadIdx.x] = R(p.coef[threadIdx.x]);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sub = lane / LPR, l = lane % LPR;
+  const E* __restrict__ Xe = reinterpret_cast<const E*>(X) + l * VPL;
+  E* __restrict__ Ye = reinterpret_cast<E*>(Y) + l * VPL;
+  int die = 0;
+  if (p.wq) {
+    uint32_t sid;
+    asm volatile("mov.u32 %0, %%smid;" : "=r"(sid));
+    die = (p.sm_die && sid < p.nsmid) ? int(__ldg(p.sm_die + sid)) : 0;
+  }
+  auto fetch = [&](uint32_t prev) -> uint32_t {
+    if (!p.wq) return prev + gridDim.x;
+    for (int k = 0; k < 2; ++k) {
+      const int q = die ^ k;
+      const uint32_t beg = q ? qsplit : 0u, n = q ? ntiles - qsplit : qsplit;
+      const uint32_t i = atomicAdd(p.wq + q, 1u);
+      if (i < n) return beg + i;
+    }
+    return ntiles;
+  };
+  if (threadIdx.x == 0) s_tile[0] = p.wq ? fetch(0) : blockIdx.x;
+  __syncthreads();
+  uint32_t tile = s_tile[0];
+  R gcol[VPL];
+  #pragma unroll
+  for (int v = 0; v < VPL; ++v) gcol[v] = gacc ? R(gacc[l * VPL + v]) : R(1);
+  for (uint32_t it = 1; tile < ntiles; ++it) {
+    if (threadIdx.x == 0) s_tile[it & 1] = fetch(tile);
+    const uint32_t r1 = min(p.dim, (tile + 1) * kBlockTile);
+    double dr[VPL], di[VPL];
+    #pragma unroll
+    for (int v = 0; v < VPL; ++v) { dr[v] = 0.0; di[v] = 0.0; }
+    uint32_t r = tile * kBlockTile + warp * RPW + sub;
+    uint32_t b0 = 0, b1 = 0;
+    if (r < r1) { b0 = __ldg(p.start + r); b1 = __ldg(p.start + r + 1); }
+    for (; r < r1; r += (256 / 32) * RPW) {
+      const uint4* __restrict__ w = p.words + b0;
+      const uint32_t n = b1 - b0;
+      uint4 q = n ? __ldg(w) : make_uint4(0u, 0u, 0u, 0u);
+      const Pack own = *reinterpret_cast<const Pack*>(Xe + size_t(r) * RV);
+      const R d = p.diag ? R(__ldg(p.diag + r)) : R(0);
+      const uint32_t rn = r + (256 / 32) * RPW;
+      if (rn < r1) { b0 = __ldg(p.start + rn); b1 = __ldg(p.start + rn + 1); }
+      R ar[VPL], ai[VPL];
+      #pragma unroll
+      for (int v = 0; v < VPL; ++v) {
+        unpk<DT>(own.v[v], ar[v], ai[v]);
+        ar[v] *= d;
+        if (T::cplx) ai[v] *= d;
+      }
+      for (uint32_t j = 0; j < n; ++j) {
+        const uint32_t e[4] = {q.x, q.y, q.z, q.w};
+        Pack t[4];
+        #pragma unroll
+        for (int u = 0; u < 4; ++u)  // padding (class 0) reads row 0, always there, and is not added
+          t[u] = *reinterpret_cast<const Pack*>(Xe + size_t(e[u] & 0xFFFFFFu) * RV);
+        if (j + 1 < n) q = __ldg(w + j + 1);
+        #pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (e[u] >> 24) {
+            const R c = s_coef[e[u] >> 24];
+            #pragma unroll
+            for (int v = 0; v < VPL; ++v) {
+              R vr, vi;
+              unpk<DT>(t[u].v[v], vr, vi);
+              ar[v] += c * vr;
+              if (T::cplx) ai[v] += c * vi;
+            }
+          }
+      }
+      Pack* yp = reinterpret_cast<Pack*>(Ye + size_t(r) * RV);
+      if (gacc) {
+        const Pack y0 = *yp;
+        #pragma unroll
+        for (int v = 0; v < VPL; ++v) {
+          R y0r, y0i;
+          unpk<DT>(y0.v[v], y0r, y0i);
+          ar[v] = y0r + gcol[v] * ar[v];
+          if (T::cplx) ai[v] = y0i + gcol[v] * ai[v];
+        }
+      }
+      Pack yv;
+      #pragma unroll
+      for (int v = 0; v < VPL; ++v) {
+        if constexpr (T::cplx) { yv.v[v].x = ar[v]; yv.v[v].y = ai[v]; } else yv.v[v] = ar[v];
+        R xr, xi;
+        unpk<DT>(own.v[v], xr, xi);
+        if (T::cplx) {
+          dr[v] += double(xr) * double(ar[v]) + double(xi) * double(ai[v]);
+          di[v] += double(xr) * double(ai[v]) - double(xi) * double(ar[v]);
+        } else {
+          dr[v] += double(xr) * double(ar[v]);
+        }
+      }
+      *yp = yv;
+    }
+    if (part) {
+      #pragma unroll
+      for (int v = 0; v < VPL; ++v)
+        #pragma unroll
+        for (int o = LPR; o < 32; o <<= 1) {
+          dr[v] += __shfl_xor_sync(0xffffffffu, dr[v], o);
+          if (T::cplx) di[v] += __shfl_xor_sync(0xffffffffu, di[v], o);
+        }
+      if (lane < LPR) {
+        #pragma unroll
+        for (int v = 0; v < VPL; ++v) {
+          red[(warp * RV + l * VPL + v) * 2] = dr[v];
+          red[(warp * RV + l * VPL + v) * 2 + 1] = T::cplx ? di[v] : 0.0;
+        }
+      }
+    }
+    __syncthreads();
+    if (part) {
+      for (int c = threadIdx.x; c < RV; c += 256) {
+        double sr = 0.0, si = 0.0;
+        for (int k = 0; k < 256 / 32; ++k) { sr += red[(k * RV + c) * 2]; si += red[(k * RV + c) * 2 + 1]; }
+        double* o = part + (size_t(c) * ntiles + tile) * 2;
+        o[0] = sr;
+        o[1] = si;
+      }
+      __syncthreads();
+    }
+    tile = s_tile[it & 1];
+  }
+  if (p.wq && threadIdx.x == 0) {  // the last CTA resets the queues for the next launch
+    __threadfence();
+    if (atomicAdd(p.wq + 2, 1u) == gridDim.x - 1) {
+      atomicExch(p.wq, 0u);
+      atomicExch(p.wq + 1, 0u);
+      atomicExch(p.wq + 2, 0u);
+    }
+  }
+}
+
+// out[2c..2c+1] = sum over the n items of column c, in a fixed order, one CTA
+// per column (the last CTA of the block kernels summed all columns by itself:
+// about 100 us of the 2175 us of J1-J2 N=24, 32 columns).
+__global__ void __launch_bounds__(256) k_sum_items(const double* __restrict__ part, uint32_t n, double* __restrict__ out) {
+  const double2* __restrict__ p = reinterpret_cast<const double2*>(part) + size_t(blockIdx.x) * n;
+  double re = 0.0, im = 0.0;
+  for (uint32_t i = threadIdx.x; i < n; i += 256) {
+    const double2 v = __ldg(p + i);
+    re += v.x;
+    im += v.y;
+  }
+  __shared__ double sbuf[2 * (256 / 32)];
+  block_sum2(re, im, sbuf);
+  if (threadIdx.x == 0) { out[2 * blockIdx.x] = re; out[2 * blockIdx.x + 1] = im; }
 }
 
 template <int DT, bool DOT>
@@ -274,6 +511,142 @@ int list_apply(const ListHandle* h, qk_dtype t, const void* x, void* y, cudaStre
   }
   QKD_LAUNCH_CHECK();
   return QKD_OK;
+}
+
+
+int sum_items(const double* part, uint32_t n, int columns, double* out, cudaStream_t s) {
+  k_sum_items<<<columns, 256, 0, s>>>(part, n, out);
+  QKD_LAUNCH_CHECK();
+  return QKD_OK;
+}
+
+void block_list_destroy(BlockListHandle* h) {
+  if (!h) return;
+  for (void* b : h->bufs) cudaFree(b);
+  cudaFree(h->part);
+  delete h;
+}
+
+// Packed lists of a real operator (diag as in list_plan_create); null when
+// they exceed max_bytes, the ranks 24 bits, the coefficients the class table,
+// or the memory is not there.
+BlockListHandle* block_list_create(const DevPlan& p, uint64_t dim, const double* diag, size_t max_bytes,
+                                   size_t* dev_bytes) {
+  if (dim == 0 || dim > kListMaxDim || p.ngroups == 0) return nullptr;
+  uint64_t* st = nullptr;
+  unsigned long long* table = nullptr;
+  uint32_t *start = nullptr, *words = nullptr, *wq = nullptr;
+  std::vector<uint32_t> hs(dim + 1);
+  std::vector<unsigned long long> ht(kListClasses + 1, kNoCoef);
+  ht[kListClasses] = 0;
+  const unsigned g = unsigned(std::max<uint64_t>(1, std::min<uint64_t>((dim + 255) / 256, 148u * 8u)));
+  bool ok = cudaMalloc(&st, dim * 8) == cudaSuccess && cudaMalloc(&table, ht.size() * 8) == cudaSuccess &&
+            cudaMalloc(&start, hs.size() * 4) == cudaSuccess &&
+            cudaMemcpy(table, ht.data(), ht.size() * 8, cudaMemcpyHostToDevice) == cudaSuccess;
+  if (ok) {
+    k_list_states<<<std::max(1u, std::min(p.ntiles, 148u * 8u)), 256>>>(p, st);
+    k_packed_build<false><<<g, 256>>>(p, uint32_t(dim), st, start, nullptr, table,
+                                      reinterpret_cast<int*>(table + kListClasses));
+    ok = cudaGetLastError() == cudaSuccess &&
+         cudaMemcpy(hs.data(), start, dim * 4, cudaMemcpyDeviceToHost) == cudaSuccess &&
+         cudaMemcpy(ht.data(), table, ht.size() * 8, cudaMemcpyDeviceToHost) == cudaSuccess && ht[kListClasses] == 0;
+  }
+  uint64_t total = 0;
+  for (uint64_t i = 0; ok && i < dim; ++i) {
+    const uint32_t n = hs[i];
+    hs[i] = uint32_t(total);
+    total += n;
+  }
+  hs[dim] = uint32_t(total);
+  ok = ok && total < (1ull << 32) && total * 16 <= max_bytes &&
+       cudaMalloc(&words, std::max<uint64_t>(total, 1) * 16) == cudaSuccess &&
+       cudaMemcpy(start, hs.data(), hs.size() * 4, cudaMemcpyHostToDevice) == cudaSuccess;
+  if (ok) {
+    k_packed_build<true><<<g, 256>>>(p, uint32_t(dim), st, start, words, table,
+                                     reinterpret_cast<int*>(table + kListClasses));
+    ok = cudaGetLastError() == cudaSuccess && cudaDeviceSynchronize() == cudaSuccess;
+  }
+  cudaFree(st);
+  cudaFree(table);
+  auto* h = ok ? new BlockListHandle : nullptr;
+  if (!h) {
+    (void)cudaGetLastError();
+    cudaFree(start);
+    cudaFree(words);
+    return nullptr;
+  }
+  const uint8_t* map = nullptr;
+  int nsmid = 0, n0 = 0, n1 = 0;
+  if (die_map(&map, &nsmid, &n0, &n1) && cudaMalloc(&wq, 16) == cudaSuccess && cudaMemset(wq, 0, 16) == cudaSuccess) {
+    h->plan.wq = wq;
+    h->plan.sm_die = map;
+    h->plan.nsmid = uint32_t(nsmid);
+    h->plan.n0 = n0;
+    h->plan.n1 = n1;
+  } else {
+    (void)cudaGetLastError();
+  }
+  h->bufs[0] = start;
+  h->bufs[1] = words;
+  h->bufs[2] = wq;
+  *dev_bytes += hs.size() * 4 + std::max<uint64_t>(total, 1) * 16;
+  h->plan.dim = uint32_t(dim);
+  h->plan.start = start;
+  h->plan.words = reinterpret_cast<const uint4*>(words);
+  h->plan.diag = diag;
+  for (int k = 0; k < kListClasses; ++k) {
+    h->plan.coef[k] = 0.0;
+    if (k && ht[k] != kNoCoef) std::memcpy(&h->plan.coef[k], &ht[k], 8);
+  }
+  return h;
+}
+
+// lanes per row 32, 16 or 8 (R / lanes <= 8, 4 to 64 bytes per lane);
+// QKD_EINVAL for other shapes, or when the dots' partials have no memory
+// (during a capture, before a first use outside it).
+int block_list_apply(const BlockListHandle* h, qk_dtype t, int R, int lpr, bool queues, const void* X, void* Y,
+                     double* dots, cudaStream_t s, const double* gacc) {
+  BlockListPlan p = h->plan;
+  if (!queues) p.wq = nullptr;
+  const uint32_t ntiles = (p.dim + kBlockTile - 1) / kBlockTile;
+  const uint32_t qsplit = uint32_t(uint64_t(ntiles) * p.n0 / std::max(1, p.n0 + p.n1));
+  double* part = nullptr;
+  if (dots) {
+    std::lock_guard<std::mutex> lk(h->mu);
+    const size_t need = size_t(ntiles) * R * 2;
+    if (h->part_cap < need) {
+      cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+      if (cudaStreamIsCapturing(s, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone) return QKD_EINVAL;
+      cudaFree(h->part);
+      h->part = nullptr;
+      h->part_cap = 0;
+      if (cudaMalloc(&h->part, need * 8) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return QKD_EINVAL;
+      }
+      h->part_cap = need;
+    }
+    part = h->part;
+  }
+#define QKD_BL(RR, L, V)                                                                                     \
+  if (R == RR && lpr == L) {                                                                                 \
+    QKD_DISPATCH(t, {                                                                                        \
+      constexpr int B = V * int(sizeof(VT<DT>::E));                                                          \
+      if constexpr (B <= 32) {                                                                               \
+        auto k = k_hx_block_list<DT, L, V, B <= 16 ? 5 : 3>;                                                 \
+        k<<<resident_grid(k, 256, 0, ntiles), 256, 0, s>>>(p, X, Y, gacc, ntiles, qsplit, part);             \
+      } else {                                                                                               \
+        return QKD_EINVAL;                                                                                   \
+      }                                                                                                      \
+    });                                                                                                      \
+    QKD_LAUNCH_CHECK();                                                                                      \
+    return dots ? sum_items(part, ntiles, R, dots, s) : QKD_OK;                                              \
+  }
+  QKD_BL(32, 32, 1) QKD_BL(32, 16, 2) QKD_BL(32, 8, 4)
+  QKD_BL(64, 32, 2) QKD_BL(64, 16, 4) QKD_BL(64, 8, 8)
+  QKD_BL(128, 32, 4) QKD_BL(128, 16, 8)
+#undef QKD_BL
+  return QKD_EINVAL;
 }
 
 }  // namespace qkd

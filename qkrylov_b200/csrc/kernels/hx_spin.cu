@@ -857,10 +857,7 @@ k_hx_rows_block(const SpinPlan* __restrict__ pp, const void* __restrict__ X, voi
     chunk = cn;
   }
   if (wq) wq_done(wq);
-  if (tile_part) {
-    grid_finish_n(tile_part, ticket, RV, dots, nchunks);
-    return;
-  }
+  if (tile_part) return;  // summed by sum_items
   for (int v = 0; v < VPL; ++v) {
     __syncthreads();
     red[2 * threadIdx.x] = dr[v];
@@ -906,6 +903,7 @@ void spin_plan_destroy(SpinHandle* h) {
 }
 
 bool die_map(const uint8_t** dev_map, int* nsmid, int* n0, int* n1);
+int sum_items(const double* part, uint32_t n, int columns, double* out, cudaStream_t s);
 
 // Per-die work queues (process-wide switch, for comparisons).
 static bool g_die_queues = true;
@@ -1579,6 +1577,21 @@ int spin_apply_rows(const SpinHandle* h, qk_dtype t, const void* x, void* y, cud
   return QKD_OK;
 }
 
+// Memory for `need` doubles of per-item column-dot partials, kept in the
+// handle; null when it does not exist and cannot be had now (capture).
+static double* item_partials(const SpinHandle* h, size_t need, cudaStream_t s) {
+  std::lock_guard<std::mutex> lk(h->tp_mu);
+  if (h->tp_cap >= need) return h->tile_part;
+  cudaStreamCaptureStatus cap_st = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s, &cap_st) != cudaSuccess || cap_st != cudaStreamCaptureStatusNone) return nullptr;
+  cudaFree(h->tile_part);
+  h->tile_part = nullptr;
+  h->tp_cap = 0;
+  if (cudaMalloc(&h->tile_part, need * sizeof(double)) == cudaSuccess) h->tp_cap = need;
+  else (void)cudaGetLastError();
+  return h->tile_part;
+}
+
 template <int DT, bool GEN, int LPR, int VPL>
 int launch_rows_block(const SpinHandle* h, qk_workspace* w, const void* X, void* Y, double* dots, cudaStream_t s,
                       const double* gacc, int tilec) {
@@ -1592,20 +1605,8 @@ int launch_rows_block(const SpinHandle* h, qk_workspace* w, const void* X, void*
   uint32_t qsplit = nt;
   double* tp = nullptr;
   if (g_die_queues && h->wq && h->host.sm_die) {
-    // per-tile dot partials for the queued form (RV columns, 2 doubles each)
-    std::lock_guard<std::mutex> lk(h->tp_mu);
-    const size_t need = size_t(nt) * RV * 2;
-    cudaStreamCaptureStatus cap_st = cudaStreamCaptureStatusNone;
-    const bool capturing = cudaStreamIsCapturing(s, &cap_st) != cudaSuccess || cap_st != cudaStreamCaptureStatusNone;
-    if (h->tp_cap < need && !capturing) {  // (a graph keeps the grid-stride form unless sized before capture)
-      cudaFree(h->tile_part);
-      h->tile_part = nullptr;
-      h->tp_cap = 0;
-      if (cudaMalloc(&h->tile_part, need * sizeof(double)) == cudaSuccess) h->tp_cap = need;
-      else (void)cudaGetLastError();
-    }
-    if (h->tile_part && h->tp_cap >= need) {
-      tp = h->tile_part;
+    tp = item_partials(h, size_t(nt) * RV * 2, s);  // (a graph keeps the grid-stride form unless sized before capture)
+    if (tp) {
       wq = h->wq + 4;
       qsplit = uint32_t(uint64_t(nt) * h->n0 / std::max(1, h->n0 + h->n1));
     }
@@ -1613,7 +1614,7 @@ int launch_rows_block(const SpinHandle* h, qk_workspace* w, const void* X, void*
   k<<<g, 256, 0, s>>>(h->dev, X, Y, w->partials, w->ticket, dots ? dots : qkd_workspace_results(w), gacc, wq, nt,
                       qsplit, tp, tiles);
   QKD_LAUNCH_CHECK();
-  return QKD_OK;
+  return tp && dots ? sum_items(tp, nt, RV, dots, s) : QKD_OK;
 }
 
 template <int DT, bool GEN>

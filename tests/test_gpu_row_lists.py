@@ -61,3 +61,34 @@ def test_small_sector_kernels_match_the_others(kind, N, sec, terms):
                 assert rel(y.cpu().numpy().astype(np.complex128), want) < tol, (pol, code)
         finally:
             qk.set_kernel_policy("auto")
+
+
+@pytest.mark.parametrize("kind,N,sec,terms", [
+    ("spin", 7, {}, O.heisenberg_chain(7)),                                         # 128 rows: one whole tile
+    ("spin", 9, dict(use_sz=1, sz2=1), O.j1j2_chain(9, 1.0, 0.5)),                  # 126 rows: one ragged tile
+    ("spin", 9, {}, [(0.7, [("Sx", i)]) for i in range(9)]),                        # no diagonal; 9 targets a row
+    ("tj", 8, dict(use_nup=1, nup=3, use_ndn=1, ndn=3), O.tj_chain(8)),             # 560 rows, 0 to 12 targets
+])
+@pytest.mark.parametrize("R", [32, 64, 128])
+def test_tuned_block_apply_on_small_tiles(kind, N, sec, terms, R):
+    """The shape the tuner picks (the packed lists among its candidates) for
+    every vector type, with column dots that repeat bit for bit."""
+    H = ham(kind, N, sec, terms)
+    ref = O.port().hamiltonian(kind, N, sec, terms)
+    rng = np.random.default_rng(R + N)
+    Xc = rng.standard_normal((H.dimension, R)) + 1j * rng.standard_normal((H.dimension, R))
+    for code, tdt, tol in [(qk.DTYPE_C128, torch.complex128, 1e-12), (qk.DTYPE_C64, torch.complex64, 2e-5),
+                           (qk.DTYPE_F64, torch.float64, 1e-12), (qk.DTYPE_F32, torch.float32, 2e-5)]:
+        X = torch.tensor(Xc if tdt.is_complex else Xc.real, dtype=tdt, device="cuda").contiguous()
+        Xh = X.cpu().numpy().astype(np.complex128)
+        want = np.stack([ref.apply(np.ascontiguousarray(Xh[:, r])) for r in range(R)], axis=1)
+        Y = torch.full_like(X, float("nan"))
+        torch.cuda.synchronize()
+        H.apply_block_device(X.data_ptr(), Y.data_ptr(), code, R)
+        dots = [H.apply_block_device(X.data_ptr(), Y.data_ptr(), code, R, dots=True) for _ in range(2)]
+        torch.cuda.synchronize()
+        assert rel(Y.cpu().numpy().astype(np.complex128), want) < tol, code
+        d = np.einsum("ir,ir->r", Xh.conj(), want)
+        got = dots[0][0::2] + 1j * dots[0][1::2]
+        assert np.abs(got - d).max() <= 10 * tol * np.abs(d).max() + 1e-300, code
+        assert np.array_equal(dots[0], dots[1]), code
