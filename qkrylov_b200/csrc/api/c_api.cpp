@@ -269,12 +269,11 @@ int qkrylov_lanczos_ground_state_complex(qkrylov_hamiltonian_h h, int maxiter, f
                                          qkrylov_lanczos_result_c_t* result, float* eigenvector_complex) {
   if (!h || !h->op || !result) return QKRYLOV_ERROR_INVALID_ARG;
   return guarded([&] {
-    std::vector<std::complex<float>> ritz;
-    auto r = qkb::lanczos<float>(*h->op, maxiter, tol, nullptr, eigenvector_complex ? &ritz : nullptr);
+    auto r = qkb::lanczos<float>(*h->op, maxiter, tol, nullptr,
+                                 reinterpret_cast<std::complex<float>*>(eigenvector_complex));
     result->energy = r.energy;
     result->iterations = r.iterations;
     result->converged = r.converged ? 1 : 0;
-    if (eigenvector_complex && !ritz.empty()) std::memcpy(eigenvector_complex, ritz.data(), ritz.size() * 8);
     return QKRYLOV_SUCCESS;
   });
 }

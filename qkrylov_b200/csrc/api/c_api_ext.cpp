@@ -380,15 +380,13 @@ int qkrylov_lanczos_ground_state_f64(qkrylov_hamiltonian_h h, int maxiter, doubl
                                      double* betas) {
   if (!h || !h->op || !result) return QKRYLOV_ERROR_INVALID_ARG;
   return guarded([&] {
-    std::vector<std::complex<double>> ritz;
     auto r = qkb::lanczos<double>(*h->op, maxiter, tol, reinterpret_cast<const std::complex<double>*>(start),
-                                  evec ? &ritz : nullptr);
+                                  reinterpret_cast<std::complex<double>*>(evec));
     result->energy = r.energy;
     result->iterations = r.iterations;
     result->converged = r.converged;
     result->n_alpha = int(r.alphas.size());
     result->n_beta = int(r.betas.size());
-    if (evec && !ritz.empty()) std::memcpy(evec, ritz.data(), ritz.size() * 16);
     if (alphas) std::copy(r.alphas.begin(), r.alphas.end(), alphas);
     if (betas) std::copy(r.betas.begin(), r.betas.end(), betas);
     return QKRYLOV_SUCCESS;

@@ -16,8 +16,8 @@ template <typename ExecSpace>
 LanczosResult lanczos_ground_state(const MatrixFreeHamiltonian<ExecSpace>& H, int maxiter, Real tol) {
   LanczosResult res;
   if (H.dimension() == 0) return res;
-  std::vector<Complex> ritz;
-  auto r = qkb::lanczos<Real>(H.op(), maxiter, tol, nullptr, &ritz);
+  std::vector<Complex> ritz(H.dimension());
+  auto r = qkb::lanczos<Real>(H.op(), maxiter, tol, nullptr, reinterpret_cast<std::complex<Real>*>(ritz.data()));
   res.energy = r.energy;
   res.iterations = r.iterations;
   res.converged = r.converged;

@@ -77,6 +77,14 @@ const double* Context::fetch(const double* dev, int n) {
   return host;
 }
 
+const double* Context::fetch2(const double* a, int na, const double* b, int nb) {
+  if (na + nb > kHost) throw std::invalid_argument("qkrylov_b200: fetch too large");
+  cuda_check(cudaMemcpyAsync(host, a, sizeof(double) * na, cudaMemcpyDeviceToHost, stream), "fetch");
+  cuda_check(cudaMemcpyAsync(host + na, b, sizeof(double) * nb, cudaMemcpyDeviceToHost, stream), "fetch");
+  cuda_check(cudaStreamSynchronize(stream), "fetch sync");
+  return host;
+}
+
 void Context::sync() { cuda_check(cudaStreamSynchronize(stream), "stream sync"); }
 
 DevVec::DevVec(size_t n, qk_dtype t, int device, bool zero) : n_(n), t_(t), dev_(device) {
@@ -111,6 +119,13 @@ void PtrArray::set(size_t i, const void* p, cudaStream_t s) {
   h_[i] = p;
   // h_ outlives the copy: the element stays valid until overwritten.
   cuda_check(cudaMemcpyAsync(d_ + i, &h_[i], sizeof(void*), cudaMemcpyHostToDevice, s), "pointer upload");
+}
+
+void PtrArray::set2(size_t i, const void* p, const void* q, cudaStream_t s) {
+  if (i + 1 >= cap_) throw std::out_of_range("qkrylov_b200: pointer array");
+  h_[i] = p;
+  h_[i + 1] = q;
+  cuda_check(cudaMemcpyAsync(d_ + i, &h_[i], 2 * sizeof(void*), cudaMemcpyHostToDevice, s), "pointer upload");
 }
 
 }  // namespace qkb

@@ -35,6 +35,8 @@ class Context {
   double* dres(int i = 0) const { return qkd_workspace_results(ws) + i; }
   // Copy n doubles from device memory to the pinned buffer and wait.
   const double* fetch(const double* dev, int n);
+  // As fetch for two ranges, one after the other in the buffer, one wait.
+  const double* fetch2(const double* a, int na, const double* b, int nb);
   void sync();
   void activate() const;
   // Stream-ordered device memory on this context's stream (the device's
@@ -78,6 +80,7 @@ class PtrArray {
   PtrArray(size_t cap, int device);
   ~PtrArray();
   void set(size_t i, const void* p, cudaStream_t s);
+  void set2(size_t i, const void* p, const void* q, cudaStream_t s);  // elements i and i + 1, one copy
   const void* const* data() const { return reinterpret_cast<const void* const*>(d_); }
   const void* const* at(size_t i) const { return data() + i; }
   size_t capacity() const { return cap_; }

@@ -7,6 +7,7 @@
 #include <cmath>
 #include <numeric>
 #include <random>
+#include <type_traits>
 
 #include "dense.hpp"
 
@@ -46,17 +47,19 @@ struct Dev {
     qkd_check(qkd_axpy(t, n, a.real(), a.imag(), x, y, c.stream), "axpy");
   }
   // out[j] = <P_j, x> for j < k, after x -= sum a_m U_m (M <= 2); P chunked by 511.
+  // a0: the coefficient of U_0 on the device (rounded to float for
+  // single-precision recurrences), or null for a[0].
   void update_mdot(int M, const void* const* U, const double* a, const PtrArray& P, int k, void* x,
-                   double* out) const {
+                   double* out, const double* a0 = nullptr, bool round32 = false) const {
     constexpr int kChunk = 511;
     if (k == 0) {
-      if (M > 0) qkd_check(qkd_update_mdot(c.ws, t, n, M, U, a, 0, nullptr, x, out, c.stream), "update");
+      if (M > 0) qkd_check(qkd_update_mdot_dev(c.ws, t, n, M, U, a, a0, round32, 0, nullptr, x, out, c.stream), "update");
       return;
     }
     for (int j0 = 0; j0 < k; j0 += kChunk) {
       const int kk = std::min(kChunk, k - j0);
-      qkd_check(qkd_update_mdot(c.ws, t, n, j0 == 0 ? M : 0, U, a, kk, P.at(j0), x, out + 2 * j0, c.stream),
-                "multi-dot");
+      qkd_check(qkd_update_mdot_dev(c.ws, t, n, j0 == 0 ? M : 0, U, a, a0, round32, kk, P.at(j0), x, out + 2 * j0,
+                                    c.stream), "multi-dot");
     }
   }
   // x -= sum_j coef_j P_j (coef device, 2k doubles); nrm2 (device) if given.
@@ -97,7 +100,7 @@ void reference_uniform_start(uint64_t dim, std::vector<std::complex<Real>>& v) {
 
 template <class Real>
 LanczosOut<Real> lanczos(const Operator& H, int maxiter, Real tol, const std::complex<Real>* start,
-                         std::vector<std::complex<Real>>* ritz) {
+                         std::complex<Real>* ritz) {
   LanczosOut<Real> res;
   const uint64_t dim = H.dim();
   if (dim == 0) return res;
@@ -113,13 +116,12 @@ LanczosOut<Real> lanczos(const Operator& H, int maxiter, Real tol, const std::co
 
   {
     std::vector<C<Real>> hv;
-    if (start) hv.assign(start, start + dim);
-    else reference_uniform_start<Real>(dim, hv);
+    if (!start) reference_uniform_start<Real>(dim, hv);
     V.push_back(d.vec(false));
-    d.upload<Real>(hv.data(), V[0]);
+    d.upload<Real>(start ? start : hv.data(), V[0]);
+    normalize<Real>(d, V[0].data());  // waits, so hv may go
   }
-  normalize<Real>(d, V[0].data());
-  P.set(0, V[0].data(), d.c.stream);
+  if (lim > 0) H.apply_dot(T, V[0].data(), w.data(), d.c.dres(0));
 
   std::vector<Real>& alphas = res.alphas;
   std::vector<Real>& betas = res.betas;
@@ -129,19 +131,19 @@ LanczosOut<Real> lanczos(const Operator& H, int maxiter, Real tol, const std::co
   for (int iter = 0; iter < lim; ++iter) {
     actual = iter + 1;
     const int k = int(V.size()) - 1;  // current vector index (== iter)
-    H.apply_dot(T, V[k].data(), w.data(), d.c.dres(0));
-    const Real alpha = Real(d.c.fetch(d.c.dres(0), 1)[0]);
-    alphas.push_back(alpha);
-
-    // w -= alpha v_k + beta v_{k-1}, then c_j = <v_j, w> (j <= k) and <w, w>.
+    // w = H v_k and alpha = <v_k, w> are on their way (launched before the
+    // host's convergence check of the previous step): w -= alpha v_k + beta
+    // v_{k-1}, then c_j = <v_j, w> (j <= k) and <w, w>; one wait per step.
     const void* U[2] = {V[k].data(), k > 0 ? V[k - 1].data() : nullptr};
-    const double a[4] = {double(alpha), 0.0, k > 0 ? double(betas.back()) : 0.0, 0.0};
-    P.set(k + 1, w.data(), d.c.stream);
-    d.update_mdot(k > 0 ? 2 : 1, U, a, P, k + 2, w.data(), cd);
+    const double a[4] = {0.0, 0.0, k > 0 ? double(betas.back()) : 0.0, 0.0};
+    P.set2(k, V[k].data(), w.data(), d.c.stream);
+    d.update_mdot(k > 0 ? 2 : 1, U, a, P, k + 2, w.data(), cd, d.c.dres(0), std::is_same<Real, float>::value);
     d.mupdate(P, k + 1, cd, w.data(), cd + 2 * (k + 2));
-    const double* h = d.c.fetch(cd + 2 * (k + 1), 4);
-    const double before = h[0];
-    double after = h[2];
+    const double* h = d.c.fetch2(d.c.dres(0), 1, cd + 2 * (k + 1), 4);
+    const Real alpha = Real(h[0]);
+    alphas.push_back(alpha);
+    const double before = h[1];
+    double after = h[3];
     if (after < 0.25 * before) {  // CGS lost accuracy: project once more
       ++res.reorth_second_rounds;
       d.update_mdot(0, nullptr, nullptr, P, k + 1, w.data(), cd);
@@ -154,7 +156,7 @@ LanczosOut<Real> lanczos(const Operator& H, int maxiter, Real tol, const std::co
     betas.push_back(beta);
     V.push_back(d.vec(false));
     d.scale_into(double(Real(1) / beta), w.data(), V.back().data());
-    P.set(k + 1, V.back().data(), d.c.stream);
+    H.apply_dot(T, V.back().data(), w.data(), d.c.dres(0));  // runs while the host checks; unused if it stops here
     if (iter > 0) {
       const Real e = tridiag_ground<Real>(alphas, betas, int(alphas.size()), nullptr);
       if (std::abs(e - e_old) < tol) { e_old = e; converged = true; break; }
@@ -173,7 +175,8 @@ LanczosOut<Real> lanczos(const Operator& H, int maxiter, Real tol, const std::co
     cuda_check(cudaMemcpyAsync(cd, nz.data(), sizeof(double) * 2 * m, cudaMemcpyHostToDevice, d.c.stream), "H2D");
     d.mupdate(P, m, cd, r.data(), nullptr);
     normalize<Real>(d, r.data());
-    d.download<Real>(r, *ritz);
+    cuda_check(cudaMemcpyAsync(ritz, r.data(), dim * sizeof(C<Real>), cudaMemcpyDeviceToHost, d.c.stream), "D2H");
+    d.c.sync();
   }
   return res;
 }
@@ -205,29 +208,34 @@ CoreOut lanczos_core(const Operator& H, qk_dtype T, const void* start, int maxit
     if (n0 == 0.0) throw std::invalid_argument("qkrylov_b200: zero start vector");
     d.scal(1.0 / n0, V[0].data());
   }
-  P.set(0, V[0].data(), d.c.stream);
+  if (lim > 0) H.apply_dot(T, V[0].data(), w.data(), d.c.dres(0));
   std::vector<double>& a = res.alphas;
   std::vector<double>& b = res.betas;
   double e_old = 1e300;
   for (int iter = 0; iter < lim; ++iter) {
     res.iterations = iter + 1;
     const int k = int(V.size()) - 1;
-    H.apply_dot(T, V[k].data(), w.data(), d.c.dres(0));
-    const double alpha = d.c.fetch(d.c.dres(0), 1)[0];
-    a.push_back(alpha);
+    // as in lanczos(): the product of this step was launched by the previous one
     const void* U[2] = {V[k].data(), k > 0 ? V[k - 1].data() : nullptr};
-    const double co[4] = {alpha, 0.0, k > 0 ? b.back() : 0.0, 0.0};
-    P.set(k + 1, w.data(), d.c.stream);
-    d.update_mdot(k > 0 ? 2 : 1, U, co, P, k + 2, w.data(), cd);
+    const double co[4] = {0.0, 0.0, k > 0 ? b.back() : 0.0, 0.0};
+    P.set2(k, V[k].data(), w.data(), d.c.stream);
+    d.update_mdot(k > 0 ? 2 : 1, U, co, P, k + 2, w.data(), cd, d.c.dres(0));
     d.mupdate(P, k + 1, cd, w.data(), cd + 2 * (k + 2));
-    const double* hh = d.c.fetch(cd + 2 * (k + 1), 4);
-    double after = hh[2];
-    if (after < 0.25 * hh[0]) {
+    const double* hh = d.c.fetch2(d.c.dres(0), 1, cd + 2 * (k + 1), 4);
+    a.push_back(hh[0]);
+    double after = hh[3];
+    if (after < 0.25 * hh[1]) {
       d.update_mdot(0, nullptr, nullptr, P, k + 1, w.data(), cd);
       d.mupdate(P, k + 1, cd, w.data(), cd + 2 * (k + 2));
       after = d.c.fetch(cd + 2 * (k + 2), 1)[0];
     }
     const double beta = std::sqrt(after);
+    const bool more = beta >= 1e-15 && iter + 1 < lim;
+    if (more) {  // the next step's vector and product, while the host checks this one
+      V.push_back(d.vec(false));
+      d.scale_into(1.0 / beta, w.data(), V.back().data());
+      H.apply_dot(T, V.back().data(), w.data(), d.c.dres(0));
+    }
     std::vector<double> z;
     const double e = tridiag_ground<double>(a, b, int(a.size()), &z);
     const double rest = beta * std::abs(z.back());
@@ -239,11 +247,8 @@ CoreOut lanczos_core(const Operator& H, qk_dtype T, const void* start, int maxit
       break;
     }
     e_old = e;
-    if (iter + 1 == lim) break;
+    if (!more) break;
     b.push_back(beta);
-    V.push_back(d.vec(false));
-    d.scale_into(1.0 / beta, w.data(), V.back().data());
-    P.set(k + 1, V.back().data(), d.c.stream);
   }
   if (ritz) {
     std::vector<double> z;
@@ -1140,7 +1145,7 @@ Real spectral_function(const Real* alphas, const Real* betas, size_t n, Real nor
 #define QKB_INST(R)                                                                                 \
   template void reference_uniform_start<R>(uint64_t, std::vector<std::complex<R>>&);               \
   template LanczosOut<R> lanczos<R>(const Operator&, int, R, const std::complex<R>*,                \
-                                    std::vector<std::complex<R>>*);                                 \
+                                    std::complex<R>*);                                              \
   template CFOut<R> continued_fraction<R>(const Operator&, const std::complex<R>*, int);            \
   template std::vector<FTLMOut<R>> ftlm<R>(const Operator&, const std::vector<R>&, int, int);       \
   template DavidsonOut<R> davidson<R>(const Operator&, int, int, R);                                \

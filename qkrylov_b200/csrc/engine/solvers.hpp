@@ -58,7 +58,7 @@ template <class Real> void reference_uniform_start(uint64_t dim, std::vector<std
 // modified Gram-Schmidt; both project onto the same complement).
 template <class Real>
 LanczosOut<Real> lanczos(const Operator& H, int maxiter, Real tol,
-                         const std::complex<Real>* start, std::vector<std::complex<Real>>* ritz);
+                         const std::complex<Real>* start, std::complex<Real>* ritz);
 
 // Lanczos with full reorthogonalisation on device vectors of any dtype,
 // scalars (alpha, beta, reorthogonalisation coefficients, tridiagonal) in

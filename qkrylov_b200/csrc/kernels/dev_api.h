@@ -150,6 +150,11 @@ int qkd_dot(qk_workspace* w, qk_dtype t, size_t n, const void* x, const void* y,
 int qkd_update_mdot(qk_workspace* w, qk_dtype t, size_t n, int M, const void* const* U,
                     const double* a, int k, const void* const* V, void* x, double* out,
                     cudaStream_t s);
+/* The same with the coefficient of U_0 (real) read from device memory at
+ * *a0, rounded to float first when round32 (a[0], a[1] are not used). */
+int qkd_update_mdot_dev(qk_workspace* w, qk_dtype t, size_t n, int M, const void* const* U, const double* a,
+                        const double* a0, int round32, int k, const void* const* V, void* x, double* out,
+                        cudaStream_t s);
 /* x <- x - sum_{j<k} c_j V_j (c: 2k device doubles); if nrm2 != NULL also
  * writes ||x||^2 of the stored result to nrm2[0] (and 0 to nrm2[1]). */
 int qkd_mupdate(qk_workspace* w, qk_dtype t, size_t n, int k, const void* const* V,

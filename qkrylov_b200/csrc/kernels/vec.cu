@@ -99,7 +99,14 @@ __global__ void k_normalize_into(size_t n, const double* nrm2, const void* x, vo
   }
 }
 
-struct UPack { const void* u[4]; double ar[4], ai[4]; };
+// a0: when not null, the real coefficient of U_0 is *a0 (device), rounded to
+// float first when round32
+struct UPack { const void* u[4]; double ar[4], ai[4]; const double* a0; int round32; };
+__device__ __forceinline__ double upack_re(const UPack& U, int m) {
+  if (m != 0 || !U.a0) return U.ar[m];
+  const double v = __ldcg(U.a0);
+  return U.round32 ? double(float(v)) : v;
+}
 
 // 16-byte packs: W consecutive elements per lane and load (one complex128,
 // two complex64 or float64, four float32).
@@ -172,7 +179,7 @@ __device__ __forceinline__ void mdot_tiles(size_t nq, int M, const UPack& U, int
       #pragma unroll
       for (int m = 0; m < 4; ++m) {
         if (m >= M) break;
-        const double ar = U.ar[m], ai = U.ai[m];
+        const double ar = upack_re(U, m), ai = U.ai[m];
         #pragma unroll
         for (int e = 0; e < E; ++e) {
           double ur[W], ui[W];
@@ -270,8 +277,9 @@ k_update_mdot(size_t n, int M, UPack U, int k,
         R r, m; T::ld_plain(x, in ? i : 0, r, m); xr = r; xi = m;
         for (int mm = 0; mm < M; ++mm) {
           R ur, ui; T::ld(U.u[mm], i, ur, ui);
-          xr -= U.ar[mm] * double(ur) - U.ai[mm] * double(ui);
-          xi -= U.ar[mm] * double(ui) + U.ai[mm] * double(ur);
+          const double cr = upack_re(U, mm);
+          xr -= cr * double(ur) - U.ai[mm] * double(ui);
+          xi -= cr * double(ui) + U.ai[mm] * double(ur);
         }
         if (M > 0) { T::st(x, i, R(xr), R(xi)); xr = double(R(xr)); xi = double(R(xi)); }
       }
@@ -666,12 +674,19 @@ int qkd_axpby(qk_dtype t, size_t n, double are, double aim, const void* x, doubl
 int qkd_update_mdot(qk_workspace* w, qk_dtype t, size_t n, int M, const void* const* U,
                     const double* a, int k, const void* const* V, void* x, double* out,
                     cudaStream_t s) {
+  return qkd_update_mdot_dev(w, t, n, M, U, a, nullptr, 0, k, V, x, out, s);
+}
+int qkd_update_mdot_dev(qk_workspace* w, qk_dtype t, size_t n, int M, const void* const* U, const double* a,
+                        const double* a0, int round32, int k, const void* const* V, void* x, double* out,
+                        cudaStream_t s) {
   if (!w || !x || !out || M < 0 || M > 4 || k < 0 || k > kMaxK || (M > 0 && (!U || !a)) ||
       (k > 0 && !V))
     return QKD_EINVAL;
   if (k == 0 && M == 0) return QKD_OK;
   UPack up{};
   for (int m = 0; m < M; ++m) { up.u[m] = U[m]; up.ar[m] = a[2 * m]; up.ai[m] = a[2 * m + 1]; }
+  up.a0 = a0;
+  up.round32 = round32;
   const size_t smem = size_t(kThreads / 32) * std::max(k, 1) * 2 * sizeof(double) + size_t(k) * sizeof(void*);
   if (smem > 48 * 1024) {
     QKD_DISPATCH(t, cudaFuncSetAttribute(k_update_mdot<DT>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
