@@ -17,79 +17,10 @@
 #include <mutex>
 #include <vector>
 
-#include "reduce.cuh"
-#include "../engine/sector.hpp"
+#include "hx_group.hpp"
+#include "hx_rows.cuh"
 
 namespace qkd {
-
-constexpr int kSpinThreads = 512;
-constexpr int kMaxBonds = 64;
-constexpr int kMaxDiag = 128;
-
-struct SpinBond {
-  uint32_t lo_mask, hi_mask;  // flip split into the low / high part
-  double c[4];                // coefficient for (bit_i, bit_j) = 00, 10, 01, 11
-  uint8_t bi, bj;             // bit positions
-  uint8_t kind;               // 0 low, 1 high, 2 crossing
-  uint8_t valid_mask;         // which combos have a valid term
-};
-
-struct RowBlock {
-  uint32_t base, size, lst, ebeg;  // block offset, rows, llist position, first entry in bent
-  uint32_t nh, combo;              // high entries; sign pattern of the crossing Sz Sz terms
-  double dh;                       // diagonal terms inside the high part
-};
-
-struct SpinPlan {
-  int L, H;
-  uint64_t dim;
-  int nbonds, ndiag;
-  // bond classes (host-side, for building the row tables)
-  int nlow, nhigh, ncross, ndcross;
-  uint32_t low_mask[kMaxBonds], high_mask[kMaxBonds], cross_lo[kMaxBonds], cross_hi[kMaxBonds];
-  uint8_t low_i[kMaxBonds], high_i[kMaxBonds], cross_li[kMaxBonds];
-  double low_c01[kMaxBonds], low_c10[kMaxBonds], high_c01[kMaxBonds], high_c10[kMaxBonds];
-  double cross_c01[kMaxBonds], cross_c10[kMaxBonds];   // c01: low bit 0 / high bit 1
-  uint32_t max_block;      // largest block size
-  double coef[2 * kMaxBonds];
-  int ncoef;
-  uint32_t dcross_mask[kMaxDiag];
-  double dcross_w[kMaxDiag];
-  SpinBond bonds[kMaxBonds];
-  uint32_t diag_smask[kMaxDiag];
-  double diag_w[kMaxDiag];
-  const uint32_t* A32;   // 2^H block offsets (global copy, staged to smem)
-  const uint16_t* B16;   // 2^L in-class ranks (global copy, staged to smem)
-  const uint16_t* lrow;  // llist as u16
-  const qk_tile_t* tiles;
-  uint32_t ntiles;
-  size_t smem;
-  // class and block tables of the row kernel
-  const uint2* rrec;     // per llist position: first 4-entry group; groups per low class, 4 bits each
-  const uint2* lgrp;     // 4 in-class ranks (u16) per group; padding entries name the zero slot
-  const uint16_t* crk;   // [pos][cpad]: (low-side bit << 15) | partner in-class rank
-  const double* dtab;    // [combo][pos]: low-part diagonal plus the crossing Sz Sz terms
-  const RowBlock* brec;  // per sector block
-  const uint2* bent;     // per block: high entries (base, coef) then crossing (base, coef | bit_h << 16)
-  double lcls[4];        // coefficient of each low class
-  int ncls, cpad, ncombo;
-  uint32_t zero_slot, nllist;
-  bool rows_ok;
-  // two-part operators (any factorisable group, e.g. Hubbard and t-J hops)
-  bool gen;
-  uint32_t nblocks;       // block records (all 2^H, or only the non-empty ones)
-  const uint32_t* crk32;  // [ncross][pos] (coalesced over rows): rank | lv0 << 24 | ls0 << 25 | lv1 << 26 | ls1 << 27
-  const uint32_t* crm;    // [pos]: bit q set when a term of crossing group q has its low condition
-  const double* diag_full;  // two-part operators: the diagonal per row, summed in term order
-  const uint4* btiles;      // block apply: (block record, first row, rows) runs of <= 256 rows
-  uint32_t nbtiles;
-  const uint32_t* border;   // order in which the row kernel visits the block records (null: record order)
-  // per-die work queues of the row kernel: the SMs of die 0 take the visiting
-  // positions [0, qsplit), those of die 1 [qsplit, nblocks); a CTA whose
-  // queue is empty takes from the other one
-  const uint8_t* sm_die;    // die of each SM id (null: one die)
-  uint32_t nsmid, qsplit;
-};
 
 namespace {
 
@@ -208,7 +139,6 @@ constexpr int kRowHighC128 = 3;   // complex128: high bonds held in registers (4
 constexpr int kRowMinCtaC128 = 2; // complex128: CTAs per SM the registers are sized for
 constexpr int kRowThreadsC128 = 512;  // complex128: threads per CTA (one staged block shared by 16 warps)
 constexpr int kPrefetchAhead = 2; // row chunks of high-bond partner rows prefetched into L2
-constexpr int kRowCoef = 32, kRowEnt = 48, kRowCross = 16, kRowCls = 4;
 // Rows per thread and pass (K) and CTAs per SM the registers are sized for,
 // by vector type and table form.  The kernel is latency-bound, so resident
 // warps count for more than the words they spill; measured on Heisenberg
@@ -229,88 +159,6 @@ template <int DT> constexpr int kRowNT = DT == QK_C128 ? kRowThreadsC128 : kRowT
 // two-part crossing groups whose loads are issued together (fewer where a
 // thread holds several rows, to stay within its registers)
 template <int DT, bool GEN> constexpr int kCrossBatch = kRowBatchG<DT, GEN> == 1 ? 4 : 2;
-
-__device__ __forceinline__ void sld(const double2* s, uint32_t k, double& re, double& im) {
-  const double2 v = s[k]; re = v.x; im = v.y;
-}
-__device__ __forceinline__ void sld(const float2* s, uint32_t k, float& re, float& im) {
-  const float2 v = s[k]; re = v.x; im = v.y;
-}
-__device__ __forceinline__ void sld(const double* s, uint32_t k, double& re, double& im) { re = s[k]; im = 0; }
-__device__ __forceinline__ void sld(const float* s, uint32_t k, float& re, float& im) { re = s[k]; im = 0; }
-__device__ __forceinline__ void szero(double2& v) { v = make_double2(0.0, 0.0); }
-__device__ __forceinline__ void szero(float2& v) { v = make_float2(0.f, 0.f); }
-__device__ __forceinline__ void szero(double& v) { v = 0.0; }
-__device__ __forceinline__ void szero(float& v) { v = 0.f; }
-
-// L2 prefetch of elements [first, first + count) of a vector of `es`-byte
-// elements, rounded inward to 16-byte boundaries (bulk prefetch operands
-// must be 16-byte aligned and sized).
-__device__ __forceinline__ void l2_prefetch(const void* base, uint32_t es, uint32_t first, uint32_t count) {
-  const uintptr_t b = reinterpret_cast<uintptr_t>(base);
-  const uintptr_t lo = (b + uintptr_t(first) * es + 15) & ~uintptr_t(15);
-  const uintptr_t hi = (b + uintptr_t(first + count) * es) & ~uintptr_t(15);
-  if (hi > lo)
-    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(lo), "r"(uint32_t(hi - lo)) : "memory");
-}
-
-// Coefficient of a two-part crossing group in a row: up to two terms, each
-// valid when its low condition (row table word `ent`) and its high
-// condition (block entry flags `bf`) hold, signed by the parities of both
-// parts.  Terms are added in order (first, then second).
-template <class R>
-__device__ __forceinline__ R cross_coef(uint32_t ent, uint32_t bf, const R* s_coef) {
-  R c = R(0);
-  if ((ent >> 24) & (bf >> 16) & 1u) {
-    const R w = s_coef[bf & 0xFFu];
-    c += (((ent >> 25) ^ (bf >> 17)) & 1u) ? -w : w;
-  }
-  if ((ent >> 26) & (bf >> 18) & 1u) {
-    const R w = s_coef[(bf >> 8) & 0xFFu];
-    c += (((ent >> 27) ^ (bf >> 19)) & 1u) ? -w : w;
-  }
-  return c;
-}
-
-__device__ __forceinline__ RowBlock load_block(const RowBlock* p) {
-  const uint4* q = reinterpret_cast<const uint4*>(p);
-  const uint4 a = __ldg(q), b = __ldg(q + 1);
-  RowBlock r;
-  r.base = a.x; r.size = a.y; r.lst = a.z; r.ebeg = a.w;
-  r.nh = b.x; r.combo = b.y;
-  r.dh = __hiloint2double(int(b.w), int(b.z));
-  return r;
-}
-
-// Next visiting position for this CTA from the per-die queues (wq[0], wq[1];
-// wq[2] counts CTAs that are done, the last one resets all three for the
-// next launch).  Returns nblocks when both queues are empty.
-__device__ __forceinline__ uint32_t wq_fetch(const SpinPlan& p, uint32_t* wq, int die) {
-  for (int k = 0; k < 2; ++k) {
-    const int q = die ^ k;
-    const uint32_t beg = q ? p.qsplit : 0u, n = q ? p.nblocks - p.qsplit : p.qsplit;
-    const uint32_t i = atomicAdd(wq + q, 1u);
-    if (i < n) return beg + i;
-  }
-  return p.nblocks;
-}
-
-__device__ __forceinline__ int sm_die_of(const SpinPlan& p) {
-  uint32_t s;
-  asm volatile("mov.u32 %0, %%smid;" : "=r"(s));
-  return (p.sm_die && s < p.nsmid) ? int(__ldg(p.sm_die + s)) : 0;
-}
-
-__device__ __forceinline__ void wq_done(uint32_t* wq) {
-  if (threadIdx.x == 0) {
-    __threadfence();
-    if (atomicAdd(wq + 2, 1u) == gridDim.x - 1) {
-      atomicExch(wq, 0u);
-      atomicExch(wq + 1, 0u);
-      atomicExch(wq + 2, 0u);
-    }
-  }
-}
 
 template <int DT, bool DOT, bool GEN>
 __global__ void __launch_bounds__(kRowNT<DT>, kRowMinCta<DT, GEN>)
@@ -887,6 +735,7 @@ struct SpinHandle {
   uint32_t* wq = nullptr;  // per-die work queues (8 u32: row kernel, block kernel; zero between launches)
   int n0 = 0, n1 = 0;      // SMs of each die
   bool lean = false;       // every bond conserves the charge: row kernel
+  GroupHandle* grp = nullptr;  // the grouped row kernel's plan, or null
   // per-tile column-dot partials of the queued block kernel, sized on first use
   mutable std::mutex tp_mu;
   mutable double* tile_part = nullptr;
@@ -895,6 +744,7 @@ struct SpinHandle {
 
 void spin_plan_destroy(SpinHandle* h) {
   if (!h) return;
+  group_plan_destroy(h->grp);
   for (void* b : h->bufs) cudaFree(b);
   cudaFree(h->tile_part);
   cudaFree(h->wq);
@@ -1007,6 +857,88 @@ static std::vector<uint32_t> record_order(const std::vector<uint32_t>& rec_h, in
   return o;
 }
 
+// Warp tiles of the grouped row kernel from the low targets of every position
+// (ent[off[pos] .. off[pos + 1])): per class of low parts, runs of 32
+// positions; per run and coefficient class one slot for every bond with a
+// target in at least one row.  tile0[key]: first tile of the class.
+struct LowEnt { uint16_t bond, cls, rank; };
+static bool warp_tiles(const uint32_t* key_off, uint32_t nkeys, const std::vector<uint32_t>& off,
+                       const std::vector<LowEnt>& ent, int nbond, int ncls, uint32_t zero_slot,
+                       std::vector<uint2>& wrec, std::vector<uint2>& wgrp, std::vector<uint32_t>& tile0) {
+  std::vector<uint16_t> slots;  // [class * nbond + bond][lane]
+  std::vector<uint8_t> used(size_t(ncls) * nbond);
+  slots.resize(size_t(ncls) * nbond * 32);
+  tile0.assign(nkeys, 0);
+  for (uint32_t key = 0; key < nkeys; ++key) {
+    tile0[key] = uint32_t(wrec.size());
+    for (uint32_t p0 = key_off[key]; p0 < key_off[key + 1]; p0 += 32) {
+      const uint32_t n = std::min(32u, key_off[key + 1] - p0);
+      std::fill(used.begin(), used.end(), uint8_t(0));
+      std::fill(slots.begin(), slots.end(), uint16_t(zero_slot));
+      for (uint32_t i = 0; i < n; ++i)
+        for (uint32_t e = off[p0 + i]; e < off[p0 + i + 1]; ++e) {
+          const size_t q = size_t(ent[e].cls) * nbond + ent[e].bond;
+          used[q] = 1;
+          slots[q * 32 + i] = ent[e].rank;
+        }
+      uint2 rec = make_uint2(uint32_t(wgrp.size() / 32), 0u);
+      for (int c = 0; c < ncls; ++c) {
+        std::vector<size_t> on;
+        for (int b = 0; b < nbond; ++b)
+          if (used[size_t(c) * nbond + b]) on.push_back(size_t(c) * nbond + b);
+        const uint32_t ng = uint32_t((on.size() + 3) / 4);
+        if (ng > 255) return false;
+        rec.y |= ng << (8 * c);
+        for (uint32_t g = 0; g < ng; ++g)
+          for (uint32_t i = 0; i < 32; ++i) {
+            uint32_t t[4];
+            for (uint32_t u = 0; u < 4; ++u) t[u] = 4 * g + u < on.size() ? slots[on[4 * g + u] * 32 + i] : zero_slot;
+            wgrp.push_back(make_uint2(t[0] | (t[1] << 16), t[2] | (t[3] << 16)));
+          }
+      }
+      wrec.push_back(rec);
+    }
+  }
+  if (wrec.empty()) wrec.push_back(make_uint2(0, 0));
+  if (wgrp.empty()) wgrp.push_back(make_uint2(0, 0));
+  return true;
+}
+
+// The grouped kernel's plan from the tables of a row plan whose device
+// copies are in place; wrec / wgrp go to bufs[8] and bufs[9].
+static void add_groups(SpinHandle* out, const SpinPlan& h, const std::vector<RowBlock>& brec,
+                       const std::vector<uint32_t>& tile_of, const std::vector<uint32_t>& order,
+                       const std::vector<uint2>& bent, const std::vector<uint2>& wrec, const std::vector<uint2>& wgrp,
+                       size_t* dev_bytes) {
+  auto up = [&](int slot, const std::vector<uint2>& v) {
+    if (cudaMalloc(&out->bufs[slot], v.size() * sizeof(uint2)) != cudaSuccess) return false;
+    *dev_bytes += v.size() * sizeof(uint2);
+    return cudaMemcpy(out->bufs[slot], v.data(), v.size() * sizeof(uint2), cudaMemcpyHostToDevice) == cudaSuccess;
+  };
+  if (!up(8, wrec) || !up(9, wgrp)) {
+    (void)cudaGetLastError();
+    return;
+  }
+  GroupPlan g{};
+  g.bent = h.bent;
+  g.wrec = static_cast<const uint2*>(out->bufs[8]);
+  g.wgrp = static_cast<const uint2*>(out->bufs[9]);
+  g.crk = h.crk; g.dtab = h.dtab; g.crk32 = h.crk32; g.crm = h.crm;
+  g.sm_die = h.sm_die; g.nsmid = h.nsmid;
+  g.nllist = h.nllist; g.zero_slot = h.zero_slot;
+  g.ncross = h.ncross; g.ncls = h.ncls; g.cpad = h.cpad;
+  g.dim = h.dim;
+  for (int k = 0; k < kRowCoef && k < h.ncoef; ++k) g.coef[k] = h.coef[k];
+  for (int k = 0; k < kRowCls; ++k) g.lcls[k] = h.lcls[k];
+  std::vector<GroupBlock> blocks;
+  for (uint32_t i = 0; i < uint32_t(brec.size()); ++i) {
+    const uint32_t r = order.empty() ? i : order[i];
+    const RowBlock& b = brec[r];
+    blocks.push_back(GroupBlock{b.base, b.size, b.lst, tile_of[r], b.ebeg, b.nh, b.combo, b.dh});
+  }
+  out->grp = group_plan_create(g, blocks, bent, out->n0 + out->n1 ? out->n0 : 1, out->n0 + out->n1 ? out->n1 : 0, dev_bytes);
+}
+
 // Host side: decide eligibility from the compiled plan and build the
 // specialised tables.  Returns nullptr when the operator does not qualify.
 SpinHandle* spin_plan_create(const qk_plan_desc* d, size_t* dev_bytes) {
@@ -1091,7 +1023,7 @@ SpinHandle* spin_plan_create(const qk_plan_desc* d, size_t* dev_bytes) {
   }
 
   // coefficient table and the per-part target lists the row tables are built from
-  std::vector<uint32_t> loff, lent, hoff, hlst;
+  std::vector<uint32_t> loff, lent, lbond, hoff, hlst;
   std::vector<uint2> hent;
   if (lean) {
     auto coef_index = [&](double c) -> uint32_t {
@@ -1108,6 +1040,7 @@ SpinHandle* spin_plan_create(const qk_plan_desc* d, size_t* dev_bytes) {
         if (v == 0 || v == m) continue;
         const double c = ((v >> h.low_i[q]) & 1u) ? h.low_c10[q] : h.low_c01[q];
         lent.push_back(((d->B[l ^ m] & 0xFFFFu) << 8) | coef_index(c));
+        lbond.push_back(uint32_t(q));
       }
     }
     loff[d->nllist] = uint32_t(lent.size());
@@ -1140,7 +1073,8 @@ SpinHandle* spin_plan_create(const qk_plan_desc* d, size_t* dev_bytes) {
   // diagonal table at most 16 MB, a free u16 index for the zero slot, and
   // every high-bond partner block of the same size as the block (which is
   // what keeps the coalesced high-bond loads in bounds).
-  std::vector<uint2> rrec, lgrp, bent;
+  std::vector<uint2> rrec, lgrp, bent, wrec, wgrp;
+  std::vector<uint32_t> tile0, tile_of;
   std::vector<uint16_t> crk;
   std::vector<double> dtab;
   std::vector<RowBlock> brec;
@@ -1196,6 +1130,14 @@ SpinHandle* spin_plan_create(const qk_plan_desc* d, size_t* dev_bytes) {
       if (lgrp.empty()) lgrp.push_back(make_uint2(0, 0));
     }
     if (h.rows_ok) {
+      std::vector<LowEnt> ent(loff[d->nllist]);
+      for (size_t e = 0; e < ent.size(); ++e)
+        ent[e] = LowEnt{uint16_t(lbond[e]), uint16_t(cls_of[lent[e] & 0xFFu]), uint16_t(lent[e] >> 8)};
+      if (!warp_tiles(d->key_off, d->nkeys, loff, ent, std::max(1, h.nlow), std::max(1, h.ncls), h.zero_slot, wrec, wgrp, tile0))
+        wrec.clear();
+      tile_of.assign(d->nA, 0);
+    }
+    if (h.rows_ok) {
       crk.assign(std::max<uint64_t>(2, d->nllist * uint64_t(h.cpad)), 0);
       for (uint64_t pos = 0; pos < d->nllist; ++pos) {
         const uint32_t l = d->llist[pos];
@@ -1228,6 +1170,7 @@ SpinHandle* spin_plan_create(const qk_plan_desc* d, size_t* dev_bytes) {
         b.base = uint32_t(d->A[hh] & qkb::kOffsetMask);
         b.size = need == qkb::kEmptyBlockKey ? 0 : d->key_off[need + 1] - d->key_off[need];
         b.lst = hlst[hh];
+        if (need != qkb::kEmptyBlockKey) tile_of[hh] = tile0[need];
         b.ebeg = uint32_t(bent.size());
         b.nh = hoff[hh + 1] - hoff[hh];
         b.dh = dhi[hh];
@@ -1307,6 +1250,7 @@ SpinHandle* spin_plan_create(const qk_plan_desc* d, size_t* dev_bytes) {
       out->bt[1] = static_cast<const uint4*>(out->bufs[6]); out->nbt[1] = uint32_t(bt1.size());
       out->bt[2] = static_cast<const uint4*>(out->bufs[7]); out->nbt[2] = uint32_t(bt2.size());
       set_die_queues(out, h, brec, bord, dev_bytes);
+      if (!wrec.empty()) add_groups(out, h, brec, tile_of, bord, bent, wrec, wgrp, dev_bytes);
     }
     out->host = h;
     ok = cudaMalloc(reinterpret_cast<void**>(&out->dev), sizeof(SpinPlan)) == cudaSuccess &&
@@ -1389,12 +1333,15 @@ SpinHandle* gen_plan_create(const qk_plan_desc* d, size_t* dev_bytes) {
   std::vector<uint32_t> crm(std::max<uint64_t>(1, nll), 0);
   std::vector<double> cls;
   std::vector<uint16_t> bucket[kRowCls];
+  std::vector<LowEnt> went;
+  std::vector<uint32_t> woff(nll + 1, 0);
   for (uint64_t pos = 0; pos < nll; ++pos) {
     const uint32_t l = d->llist[pos];
     const uint32_t key = d->B[l] >> 24;
     for (auto& b : bucket) b.clear();
-    for (uint32_t gi : lowg) {
-      const qk_group_t& g = d->groups[gi];
+    woff[pos] = uint32_t(went.size());
+    for (size_t q = 0; q < lowg.size(); ++q) {
+      const qk_group_t& g = d->groups[lowg[q]];
       const double c = group_value(g, l, true);
       if (c == 0.0) continue;
       const uint32_t lt = l ^ lo(g.flip);
@@ -1407,6 +1354,7 @@ SpinHandle* gen_plan_create(const qk_plan_desc* d, size_t* dev_bytes) {
         ci = int(cls.size()) - 1;
       }
       bucket[ci].push_back(uint16_t(d->B[lt] & 0xFFFFu));
+      went.push_back(LowEnt{uint16_t(q), uint16_t(ci), uint16_t(d->B[lt] & 0xFFFFu)});
     }
     rrec[pos].x = uint32_t(lgrp.size());
     uint32_t counts = 0;
@@ -1439,6 +1387,12 @@ SpinHandle* gen_plan_create(const qk_plan_desc* d, size_t* dev_bytes) {
   if (lgrp.empty()) lgrp.push_back(make_uint2(0, 0));
   h.ncls = int(cls.size());
   for (int c = 0; c < h.ncls; ++c) h.lcls[c] = cls[c];
+  woff[nll] = uint32_t(went.size());
+  std::vector<uint2> wrec, wgrp;
+  std::vector<uint32_t> tile0, tile_of;
+  if (!warp_tiles(d->key_off, d->nkeys, woff, went, std::max<int>(1, int(lowg.size())), std::max(1, h.ncls), h.zero_slot,
+                  wrec, wgrp, tile0))
+    wrec.clear();
   // block records of the non-empty blocks
   std::vector<RowBlock> brec;
   std::vector<uint2> bent;
@@ -1453,6 +1407,7 @@ SpinHandle* gen_plan_create(const qk_plan_desc* d, size_t* dev_bytes) {
     b.base = uint32_t(d->A[hh] & qkb::kOffsetMask);
     b.size = size;
     b.lst = d->key_off[need];
+    tile_of.push_back(tile0.empty() ? 0u : tile0[need]);
     b.ebeg = uint32_t(bent.size());
     b.dh = 0.0;
     for (uint32_t gi : highg) {
@@ -1526,6 +1481,7 @@ SpinHandle* gen_plan_create(const qk_plan_desc* d, size_t* dev_bytes) {
     out->bt[1] = static_cast<const uint4*>(out->bufs[6]); out->nbt[1] = uint32_t(t1.size());
     out->bt[2] = static_cast<const uint4*>(out->bufs[7]); out->nbt[2] = uint32_t(t2.size());
     set_die_queues(out, h, brec, rord, dev_bytes);
+    if (!wrec.empty()) add_groups(out, h, brec, tile_of, rord, bent, wrec, wgrp, dev_bytes);
     out->host = h;
     ok = cudaMalloc(reinterpret_cast<void**>(&out->dev), sizeof(SpinPlan)) == cudaSuccess &&
          cudaMemcpy(out->dev, &h, sizeof(SpinPlan), cudaMemcpyHostToDevice) == cudaSuccess;
@@ -1544,8 +1500,14 @@ int spin_apply_rows(const SpinHandle* h, qk_dtype t, const void* x, void* y, cud
   if (!h->host.rows_ok || (h->host.gen && !h->host.diag_full)) return QKD_EINVAL;
   const size_t es = (t == QK_C128) ? 16 : (t == QK_F32 ? 4 : 8);
   const size_t smem = es * (h->host.max_block + 1);  // staged block and the zero slot
-  if (smem > 200 * 1024) return QKD_EINVAL;
   uint32_t* const wq = g_die_queues ? h->wq : nullptr;
+  if (h->grp) {
+    const int rc = group_apply(h->grp, h->host.gen, t, x, y, s, w, dot_out, wq, h->host.diag_full,
+                               uint32_t(std::min<uint64_t>(row_lo, 0xFFFFFFFFull)),
+                               uint32_t(std::min<uint64_t>(row_hi, 0xFFFFFFFFull)));
+    if (rc != QKD_EINVAL) return rc;
+  }
+  if (smem > 200 * 1024) return QKD_EINVAL;
   if (dot_out && size_t(h->host.nblocks) > size_t(kMaxK) * kMaxG) return QKD_EINVAL;  // one partial per block
   const uint32_t rlo = uint32_t(std::min<uint64_t>(row_lo, 0xFFFFFFFFull));
   const uint32_t rhi = uint32_t(std::min<uint64_t>(row_hi, 0xFFFFFFFFull));
