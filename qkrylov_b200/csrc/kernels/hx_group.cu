@@ -24,9 +24,10 @@
 // float32 and complex128, 48 registers and 40 warps for the 8-byte types; more
 // entries in flight, tables or slots loaded a row ahead and unconditional
 // crossing loads were each slower.  us per apply, one-block kernel -> this one:
-// Heisenberg N=24 float32 46.6 -> 36.2, N=25 float64 99 -> 75, N=24 complex128
-// 86 -> 69, N=28 float32 437 -> 345, float64 590 -> 531; J1-J2 N=24 float32 81 -> 60; t-J N=19
-// float64 177 -> 103, N=20 float64 329 -> 285, complex128 529 -> 463.
+// Heisenberg N=24 float32 46.6 -> 35.1, N=25 float64 99 -> 73, N=24 complex128
+// 86 -> 66, N=28 float32 437 -> 331, float64 590 -> 529, complex128 980 -> 922;
+// J1-J2 N=24 float32 81 -> 57; t-J N=19 float64 177 -> 102, N=20 float64 329 ->
+// 278, complex128 529 -> 453.
 #include <algorithm>
 #include <cstring>
 #include <map>
@@ -74,16 +75,21 @@ k_hx_group(const __grid_constant__ GroupPlan p, const void* __restrict__ x, void
   __shared__ R s_cc[kRowCross], s_coef[kRowCoef], s_lc[kRowCls];
   __shared__ double s_dot[2 * (NT / 32)];
   const uint32_t tid = threadIdx.x, lane = tid & 31;
-  const uint32_t stride = p.zero_slot + 1, nll = p.nllist;
+  const uint32_t stride = p.zero_slot + 8, nll = p.nllist;
   const int ncross = p.ncross, ncls = p.ncls;
   for (int i = tid; i < kRowCoef; i += NT) s_coef[i] = R(p.coef[i]);
   if (tid < kRowCls) s_lc[tid] = R(p.lcls[tid]);
-  if (tid < PL) {
+  if (tid < 8 * PL) {
     Pack z;
     #pragma unroll
     for (int u = 0; u < EPP; ++u) szero(z.v[u]);
-    sx[tid * stride + p.zero_slot] = z;
+    sx[(tid / 8) * stride + p.zero_slot + tid % 8] = z;
   }
+  // one coefficient for every high entry (uniform chains): summed, then scaled;
+  // complex128 alone gains (Heisenberg N=28 959 -> 924 us), the others need the
+  // registers (float64 531 -> 580)
+  const bool uni = DT == QK_C128 && !GEN && p.uniform_high;
+  const R high = R(p.high_coef);
   int die = 0;
   if (wq) {
     uint32_t sid;
@@ -166,9 +172,14 @@ k_hx_group(const __grid_constant__ GroupPlan p, const void* __restrict__ x, void
     const double* __restrict__ dtab = p.dtab + size_t(rec.combo) * nll + lst;
     const uint32_t* __restrict__ ckw = reinterpret_cast<const uint32_t*>(p.crk);
     const uint32_t cw = uint32_t(p.cpad) >> 1;
-    uint32_t nmax = 0;
+    // entries per block: in registers for exchange tables (Heisenberg N=26
+    // float64 151.5 -> 147.4 us), re-read from shared memory for two-part ones,
+    // whose crossing loop needs the registers (t-J N=20 float32 202 -> 183 us)
+    uint32_t nhr[G], nmax = 0;
     #pragma unroll
-    for (int g = 0; g < G; ++g) nmax = max(nmax, rec.nh[g]);
+    for (int g = 0; g < G; ++g) { nhr[g] = rec.nh[g]; nmax = max(nmax, nhr[g]); }
+    const uint32_t* const nhs = rec.nh;
+    auto nh = [&](int g) { return GEN ? nhs[g] : nhr[g]; };
     for (uint32_t l = tid; any && l < size; l += NT) {
       if (p.prefetch) {  // the partner rows two chunks ahead go to L2
         const uint32_t ahead = l - tid + 2u * NT;
@@ -196,16 +207,22 @@ k_hx_group(const __grid_constant__ GroupPlan p, const void* __restrict__ x, void
         #pragma unroll
         for (int g = 0; g < G; ++g)
           #pragma unroll
-          for (int u = 0; u < U; ++u) T::ld(x, uint64_t(s_ent[g][e0 + u].base) + l, vr[g][u], vi[g][u]);
+          for (int u = 0; u < U; ++u) {
+            T::ld(x, uint64_t(s_ent[g][e0 + u].base) + l, vr[g][u], vi[g][u]);
+          }
         #pragma unroll
         for (int g = 0; g < G; ++g)
           #pragma unroll
           for (int u = 0; u < U; ++u)
-            if (e0 + u < rec.nh[g]) {
-              const R c = s_ent[g][e0 + u].c;
+            if (e0 + u < nh(g)) {
+              const R c = uni ? R(1) : s_ent[g][e0 + u].c;
               ar[g] += c * vr[g][u];
               if (T::cplx) ai[g] += c * vi[g][u];
             }
+      }
+      if (uni) {
+        #pragma unroll
+        for (int g = 0; g < G; ++g) { ar[g] *= high; if (T::cplx) ai[g] *= high; }
       }
       if constexpr (GEN) {
         // two-part crossing groups whose low and high masks both allow a term,
@@ -349,7 +366,7 @@ int launch(const GroupPlan& p, const void* x, void* y, cudaStream_t s, qk_worksp
            uint32_t rlo, uint32_t rhi) {
   using E = typename VT<DT>::E;
   constexpr int EPP = 16 / int(sizeof(E)), PL = (G + EPP - 1) / EPP;
-  const size_t smem = size_t(PL) * 16 * (p.zero_slot + 1);
+  const size_t smem = size_t(PL) * 16 * (p.zero_slot + 8);
   auto go = [&](auto k, unsigned cap, double* part, unsigned* tick) -> int {
     if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess) {
       (void)cudaGetLastError();
@@ -456,16 +473,13 @@ int group_apply(const GroupHandle* h, bool gen, qk_dtype t, const void* x, void*
                 double* dot_out, uint32_t* wq, const double* diag_full, uint32_t row_lo, uint32_t row_hi) {
   if (!h || t < QK_C128 || t > QK_F32) return QKD_EINVAL;
   const size_t es = qk_dtype_size(t);
-  const size_t rows = size_t(h->plan[0].zero_slot) + 1;
+  const size_t rows = size_t(h->plan[0].zero_slot) + 8;
   // blocks per group: 16 bytes per position for float32 (4), two planes of
   // 16 bytes or one for the others (2); complex128 alone (1) where two staged
-  // blocks would leave room for fewer than three CTAs, and there only two-part
-  // operators (t-J N=20 529 -> 463 us): exchange operators of that size are
-  // bound by the DRAM traffic of their partner rows and stay on the one-block
-  // kernel (Heisenberg N=28, three vectors in turn: 1052 us, here 1060)
+  // blocks would leave room for fewer than three CTAs (Heisenberg N=28: 1071
+  // us with two, 922 with one)
   int gi = t == QK_F32 ? 0 : 1;
   if (t == QK_C128) gi = rows * 32 > 60 * 1024 ? 2 : gen ? 1 : 3;
-  if (gi == 2 && !gen) return QKD_EINVAL;
   GroupPlan p = h->plan[gi];
   p.diag_full = diag_full;
   const size_t smem = std::max<size_t>(16, (gi == 3 ? 2u : 4u >> gi) * es) * rows;
@@ -487,8 +501,7 @@ int group_apply(const GroupHandle* h, bool gen, qk_dtype t, const void* x, void*
   switch (t) {
     case QK_C128:
       if (gi != 2) QKD_GRP1(QK_C128, 2, 2, 4, 4, 512, 2, 512, 2)
-      return big ? launch<QK_C128, true, 1, 1, 512, 3>(p, x, y, s, w, dot_out, wq, row_lo, row_hi)
-                 : launch<QK_C128, true, 1, 1, 256, 4>(p, x, y, s, w, dot_out, wq, row_lo, row_hi);
+      QKD_GRP1(QK_C128, 1, 1, 4, 4, 512, 3, 512, 3)
     case QK_C64: QKD_GRP1(QK_C64, 2, 2, 5, 5, 384, 3, 384, 3)
     case QK_F64: QKD_GRP1(QK_F64, 2, 2, 5, 5, 384, 3, 384, 3)
     case QK_F32: QKD_GRP1(QK_F32, 4, 2, 4, 5, 512, 2, 384, 3)

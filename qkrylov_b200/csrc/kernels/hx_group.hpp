@@ -24,7 +24,7 @@ struct GroupPlan {
   const uint2* bent;   // per block: high entries (base, coef) then crossing (base, flags)
   // warp tiles (32 consecutive positions of a low class): first 4-slot group
   // and groups per coefficient class (8 bits each); four slots of a row per
-  // uint2 ([group][lane], in-class ranks; zero_slot where a row has no target)
+  // uint2 ([group][lane], in-class ranks; zero_slot .. zero_slot + 7: no target)
   const uint2* wrec;
   const uint2* wgrp;
   const uint16_t* crk;
@@ -37,6 +37,8 @@ struct GroupPlan {
   int ncross, ncls, cpad;
   uint64_t dim;
   double coef[32], lcls[4];
+  int uniform_high;   // every high entry has the coefficient high_coef
+  double high_coef;
 };
 
 struct GroupBlock { uint32_t base, size, lst, tile0, ebeg, nh, combo; double dh; };

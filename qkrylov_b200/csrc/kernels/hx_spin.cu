@@ -865,6 +865,7 @@ struct LowEnt { uint16_t bond, cls, rank; };
 static bool warp_tiles(const uint32_t* key_off, uint32_t nkeys, const std::vector<uint32_t>& off,
                        const std::vector<LowEnt>& ent, int nbond, int ncls, uint32_t zero_slot,
                        std::vector<uint2>& wrec, std::vector<uint2>& wgrp, std::vector<uint32_t>& tile0) {
+  if (zero_slot + 8 > 0xFFFFu) return false;
   std::vector<uint16_t> slots;  // [class * nbond + bond][lane]
   std::vector<uint8_t> used(size_t(ncls) * nbond);
   slots.resize(size_t(ncls) * nbond * 32);
@@ -874,7 +875,7 @@ static bool warp_tiles(const uint32_t* key_off, uint32_t nkeys, const std::vecto
     for (uint32_t p0 = key_off[key]; p0 < key_off[key + 1]; p0 += 32) {
       const uint32_t n = std::min(32u, key_off[key + 1] - p0);
       std::fill(used.begin(), used.end(), uint8_t(0));
-      std::fill(slots.begin(), slots.end(), uint16_t(zero_slot));
+      std::fill(slots.begin(), slots.end(), uint16_t(0xFFFFu));
       for (uint32_t i = 0; i < n; ++i)
         for (uint32_t e = off[p0 + i]; e < off[p0 + i + 1]; ++e) {
           const size_t q = size_t(ent[e].cls) * nbond + ent[e].bond;
@@ -886,6 +887,17 @@ static bool warp_tiles(const uint32_t* key_off, uint32_t nkeys, const std::vecto
         std::vector<size_t> on;
         for (int b = 0; b < nbond; ++b)
           if (used[size_t(c) * nbond + b]) on.push_back(size_t(c) * nbond + b);
+        // rows without the bond point at the one of eight zero packs whose
+        // 16-byte bank group no target of their quarter warp uses
+        for (size_t q : on)
+          for (uint32_t ph = 0; ph < 32; ph += 8) {
+            uint32_t banks = 0, z = 0;
+            for (uint32_t i = ph; i < ph + 8; ++i)
+              if (slots[q * 32 + i] != 0xFFFFu) banks |= 1u << (slots[q * 32 + i] & 7u);
+            while (z < 7 && (banks >> ((zero_slot + z) & 7u) & 1u)) ++z;
+            for (uint32_t i = ph; i < ph + 8; ++i)
+              if (slots[q * 32 + i] == 0xFFFFu) slots[q * 32 + i] = uint16_t(zero_slot + z);
+          }
         const uint32_t ng = uint32_t((on.size() + 3) / 4);
         if (ng > 255) return false;
         rec.y |= ng << (8 * c);
@@ -930,6 +942,15 @@ static void add_groups(SpinHandle* out, const SpinPlan& h, const std::vector<Row
   g.dim = h.dim;
   for (int k = 0; k < kRowCoef && k < h.ncoef; ++k) g.coef[k] = h.coef[k];
   for (int k = 0; k < kRowCls; ++k) g.lcls[k] = h.lcls[k];
+  uint32_t hc = ~0u;
+  g.uniform_high = 1;
+  for (const RowBlock& b : brec)
+    for (uint32_t e = b.ebeg; e < b.ebeg + b.nh; ++e) {
+      const uint32_t c = bent[e].y & 0xFFFFu;
+      if (hc == ~0u) hc = c;
+      if (c != hc) g.uniform_high = 0;
+    }
+  g.high_coef = hc == ~0u ? 0.0 : h.coef[hc];
   std::vector<GroupBlock> blocks;
   for (uint32_t i = 0; i < uint32_t(brec.size()); ++i) {
     const uint32_t r = order.empty() ? i : order[i];
