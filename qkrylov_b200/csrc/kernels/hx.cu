@@ -40,7 +40,7 @@ void flip_plan_destroy(FlipHandle* h);
 int flip_apply(const FlipHandle* h, qk_dtype t, const void* x, void* y, cudaStream_t s, qk_workspace* w,
                double* dot_out, uint64_t row_lo, uint64_t row_hi);
 struct ListHandle;
-ListHandle* list_plan_create(const DevPlan& p, uint64_t dim, const double* diag, size_t* dev_bytes);
+ListHandle* list_plan_create(const DevPlan& p, uint64_t dim, const double* diag, bool two_part, size_t* dev_bytes);
 void list_plan_destroy(ListHandle* h);
 int list_apply(const ListHandle* h, qk_dtype t, const void* x, void* y, cudaStream_t s, qk_workspace* w,
                double* dot_out, uint64_t row_lo, uint64_t row_hi);
@@ -423,11 +423,12 @@ const double* real_diag(qk_plan* p) {
 // sector, with the real diagonal they need.
 void make_lists(qk_plan* p, const qk_plan_desc* d) {
   const bool flips = flip_eligible(d);
-  if (!flips && size_t(p->dim) * 16 > (size_t(64) << 20)) return;  // no list of that many rows fits
+  if (!flips && size_t(p->dim) * 16 > (size_t(96) << 20)) return;  // no list of that many rows fits
   const double* diag = real_diag(p);
   if (p->has_diag && !diag) return;
   if (flips) p->flip = flip_plan_create(d, diag, &p->bytes);
-  if (!p->flip) p->list = list_plan_create(dev(p), p->dim, diag, &p->bytes);
+  const bool two_part = !p->pair && (!p->spin || qkd::spin_plan_is_gen(p->spin));
+  if (!p->flip) p->list = list_plan_create(dev(p), p->dim, diag, two_part, &p->bytes);
   if (!p->list && !p->flip && p->list_diag) {
     cudaFree(p->list_diag);
     p->list_diag = nullptr;

@@ -33,16 +33,21 @@ namespace qkd {
 constexpr int kListClasses = 64;   // coefficient values (class 0 is zero); 8 bits of the word
 constexpr int kListThreads = 128;  // four slices per CTA: a 2^14-row sector still spreads over every SM
 constexpr uint64_t kListMaxDim = 1ull << 24;  // 24-bit ranks
-// Largest table: about one die's L2 (63 MB), so that with the vectors it stays
-// in the caches from apply to apply; beyond it the words stream from DRAM.
-// Measured against the row / pair kernels (us per apply): Heisenberg N=22 c128
-// 34.5 -> 23.3 (41 MB), N=24 87 -> 100 (165 MB); transverse Ising N=20 c64
-// 31.6 -> 34.8 (80 MB); 4x3 Hubbard f32 30.7 -> 34.7 (93 MB).
-constexpr size_t kListMaxBytes = size_t(64) << 20;
+constexpr uint32_t kListSmall = 148 * 16;     // slices whose CTAs are all resident at once (k_hx_list_small);
+// 148 * 60 instead: Heisenberg N=20 float64 8.2 -> 10.3 us
+// Largest table.  The words have to stay in the L2 caches (126 MB, lines read
+// by both dies held twice) from apply to apply.  Where the line lies depends on
+// what runs instead, us per apply with lists / without: exchange tables
+// Heisenberg N=22 c128 (41 MB) 23.3 / 24.6, float32 16.3 / 18.1, N=23 (85 MB)
+// float64 31.5 / 27.0: 64 MB; spin-product 4x3 Hubbard float32 (93 MB) 34.7 /
+// 28.7: 64 MB; two-part tables, whose rows decode slowest, t-J N=17 (72 MB)
+// float64 26 / 38: 96 MB.
+constexpr size_t kListMaxBytes = size_t(96) << 20;
 
 struct ListPlan {
   uint32_t dim, nslice;
   uint32_t row_lo, row_hi, slice0;  // rows written; first slice that holds one of them
+  uint32_t width;         // groups of every slice where they are padded to one width, else 0
   const uint32_t* start;  // per slice: first 4-slot group (nslice + 1)
   const uint4* words;     // four slots of a row per 16 bytes: [slot / 4][lane]
   const double* diag;     // or null
@@ -353,6 +358,83 @@ __global__ void __launch_bounds__(256) k_sum_items(const double* __restrict__ pa
   if (threadIdx.x == 0) { out[2 * blockIdx.x] = re; out[2 * blockIdx.x + 1] = im; }
 }
 
+// The smallest sectors: a CTA of four warps per slice, each warp every fourth
+// group of slots, partial sums added in warp order through shared memory.  The
+// slices have one width, so the words are the first loads of the kernel and
+// their targets the second: nothing else is on the path (Heisenberg N=16
+// complex128, launches back to back: 5.4 us with k_hx_list, 4.3 us here).
+template <int DT, bool DOT>
+__global__ void __launch_bounds__(kListThreads) k_hx_list_small(const __grid_constant__ ListPlan p,
+                                                                const void* __restrict__ x, void* __restrict__ y,
+                                                                double* partials, unsigned* ticket, double* dot_out) {
+  using T = VT<DT>;
+  using R = typename T::R;
+  constexpr int NW = kListThreads / 32;
+  __shared__ R s_coef[kListClasses];
+  __shared__ R s_sum[2][NW][32];
+  const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  double dr = 0.0, di = 0.0;
+  bool first = true;
+  for (uint32_t sl = p.slice0 + blockIdx.x; sl < p.nslice; sl += gridDim.x) {
+    const uint4* __restrict__ w = p.words + size_t(sl) * p.width * 32 + lane;
+    uint4 q = warp < p.width ? __ldg(w + warp * 32) : make_uint4(0u, 0u, 0u, 0u);
+    const uint32_t row = sl * 32 + lane;
+    const bool in = row >= p.row_lo && row < p.row_hi;
+    R xr = R(0), xi = R(0), d = R(0);
+    if (warp == 0 && in) {
+      T::ld(x, row, xr, xi);
+      if (p.diag) d = R(__ldg(p.diag + row));
+    }
+    if (first && threadIdx.x < kListClasses) s_coef[threadIdx.x] = R(p.coef[threadIdx.x]);
+    __syncthreads();  // the coefficients; the previous slice's sums have been read
+    first = false;
+    R ar = R(0), ai = R(0);
+    for (uint32_t j = warp; j < p.width; j += NW) {
+      const uint32_t e[4] = {q.x, q.y, q.z, q.w};
+      if (j + NW < p.width) q = __ldg(w + (j + NW) * 32);
+      R vr[4], vi[4];
+      #pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        vr[u] = R(0);
+        vi[u] = R(0);
+        if (e[u] >> 24) T::ld(x, e[u] & 0xFFFFFFu, vr[u], vi[u]);
+      }
+      #pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (e[u] >> 24) {
+          const R c = s_coef[e[u] >> 24];
+          ar += c * vr[u];
+          if (T::cplx) ai += c * vi[u];
+        }
+    }
+    s_sum[0][warp][lane] = ar;
+    if (T::cplx) s_sum[1][warp][lane] = ai;
+    __syncthreads();
+    if (warp == 0) {
+      ar = d * xr;
+      ai = d * xi;
+      #pragma unroll
+      for (int k = 0; k < NW; ++k) {
+        ar += s_sum[0][k][lane];
+        if (T::cplx) ai += s_sum[1][k][lane];
+      }
+      if (in) {
+        T::st(y, row, ar, ai);
+        if (DOT) {
+          dr += double(xr) * double(ar) + double(xi) * double(ai);
+          di += double(xr) * double(ai) - double(xi) * double(ar);
+        }
+      }
+    }
+  }
+  if (DOT) {
+    __shared__ double sbuf[2 * NW];
+    block_sum2(dr, di, sbuf);
+    if (threadIdx.x == 0) { partials[2 * blockIdx.x] = dr; partials[2 * blockIdx.x + 1] = di; }
+    grid_finish(partials, ticket, 1, dot_out);
+  }
+}
+
 template <int DT, bool DOT>
 __global__ void __launch_bounds__(kListThreads) k_hx_list(const __grid_constant__ ListPlan p,
                                                           const void* __restrict__ x, void* __restrict__ y,
@@ -428,12 +510,14 @@ void list_plan_destroy(ListHandle* h) {
 }
 
 // Row lists of a real operator with its real diagonal (diag: dim device
-// doubles, or null for none); null when they do not fit kListMaxBytes, the
+// doubles, or null for none); two_part: the operator would run on the two-part
+// tables or the generic kernel.  Null when they do not fit the limit, the
 // ranks 24 bits or the coefficients the class table.
-ListHandle* list_plan_create(const DevPlan& p, uint64_t dim, const double* diag, size_t* dev_bytes) {
+ListHandle* list_plan_create(const DevPlan& p, uint64_t dim, const double* diag, bool two_part, size_t* dev_bytes) {
+  const size_t max_bytes = two_part ? kListMaxBytes : kListMaxBytes * 2 / 3;
   const uint32_t nslice = uint32_t((dim + 31) / 32);
   // at least one slot per slice: cheap refusal of sectors that cannot fit
-  if (dim == 0 || dim > kListMaxDim || p.ngroups == 0 || size_t(nslice) * 512 > kListMaxBytes) return nullptr;
+  if (dim == 0 || dim > kListMaxDim || p.ngroups == 0 || size_t(nslice) * 512 > max_bytes) return nullptr;
   uint64_t* st = nullptr;
   unsigned long long* table = nullptr;  // kListClasses values, then the overflow flag
   uint32_t *start = nullptr, *words = nullptr;
@@ -457,11 +541,20 @@ ListHandle* list_plan_create(const DevPlan& p, uint64_t dim, const double* diag,
     const uint32_t n = hs[i];
     hs[i] = uint32_t(total);
     total += n;
-    ok = total * 512 <= kListMaxBytes;
+    ok = total * 512 <= max_bytes;
   }
   hs[nslice] = uint32_t(total);
+  // small sectors: every slice padded to the widest one
+  uint32_t width = 0;
+  for (uint32_t i = 0; ok && i < nslice; ++i) width = std::max(width, hs[i + 1] - hs[i]);
+  if (nslice > kListSmall || width == 0) width = 0;
+  if (width) {
+    for (uint32_t i = 0; i <= nslice; ++i) hs[i] = i * width;
+    total = size_t(nslice) * width;
+  }
   ok = ok && cudaMalloc(&words, std::max<size_t>(total, 1) * 512) == cudaSuccess &&
        cudaMemcpy(start, hs.data(), hs.size() * 4, cudaMemcpyHostToDevice) == cudaSuccess;
+  if (ok && width) ok = cudaMemset(words, 0, total * 512) == cudaSuccess;
   if (ok) {
     k_list_build<true><<<g, 256>>>(p, uint32_t(dim), st, start, words, table,
                                    reinterpret_cast<int*>(table + kListClasses));
@@ -483,6 +576,7 @@ ListHandle* list_plan_create(const DevPlan& p, uint64_t dim, const double* diag,
   l.dim = uint32_t(dim);
   l.nslice = nslice;
   l.start = start;
+  l.width = width;
   l.words = reinterpret_cast<const uint4*>(words);
   l.diag = diag;
   l.ncoef = kListClasses;
@@ -502,13 +596,13 @@ int list_apply(const ListHandle* h, qk_dtype t, const void* x, void* y, cudaStre
   p.row_hi = uint32_t(row_hi);
   p.slice0 = p.row_lo / 32;
   p.nslice = (p.row_hi + 31) / 32;
-  const unsigned g = (p.nslice - p.slice0 + kListThreads / 32 - 1) / (kListThreads / 32);
-  if (dot_out) {
-    QKD_DISPATCH(t, (k_hx_list<DT, true><<<std::min<unsigned>(g, kMaxG), kListThreads, 0, s>>>(
-                        p, x, y, w->partials, w->ticket, dot_out)));
-  } else {
-    QKD_DISPATCH(t, (k_hx_list<DT, false><<<g, kListThreads, 0, s>>>(p, x, y, nullptr, nullptr, nullptr)));
-  }
+  const unsigned n = p.nslice - p.slice0, g = p.width ? n : (n + kListThreads / 32 - 1) / (kListThreads / 32);
+  QKD_DISPATCH(t, {
+    auto kd = p.width ? k_hx_list_small<DT, true> : k_hx_list<DT, true>;
+    auto kn = p.width ? k_hx_list_small<DT, false> : k_hx_list<DT, false>;
+    if (dot_out) kd<<<std::min<unsigned>(g, kMaxG), kListThreads, 0, s>>>(p, x, y, w->partials, w->ticket, dot_out);
+    else kn<<<g, kListThreads, 0, s>>>(p, x, y, nullptr, nullptr, nullptr);
+  });
   QKD_LAUNCH_CHECK();
   return QKD_OK;
 }
