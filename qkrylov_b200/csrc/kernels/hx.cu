@@ -516,6 +516,13 @@ int qkd_plan_create(const qk_plan_desc* d, int device, qk_plan** out) {
   }
   if (d->pair_sites && p->diag_re) p->pair = qkd::pair_plan_create(d, p->A, p->B, p->diag_re, &p->bytes);
   if (d->all_real && !d->transient && d->dim > 0) make_lists(p, d);
+  // the uploads from pageable memory and the cleared counters above may still
+  // be on their way, and an apply on a non-blocking stream would not wait
+  if (cudaStreamSynchronize(nullptr) != cudaSuccess) {
+    (void)cudaGetLastError();
+    qkd_plan_destroy(p);
+    return QKD_ECUDA;
+  }
   *out = p;
   return QKD_OK;
 }

@@ -671,7 +671,9 @@ BlockListHandle* block_list_create(const DevPlan& p, uint64_t dim, const double*
   }
   const uint8_t* map = nullptr;
   int nsmid = 0, n0 = 0, n1 = 0;
-  if (die_map(&map, &nsmid, &n0, &n1) && cudaMalloc(&wq, 16) == cudaSuccess && cudaMemset(wq, 0, 16) == cudaSuccess) {
+  // the first apply may run on a stream that does not wait for the memset
+  if (die_map(&map, &nsmid, &n0, &n1) && cudaMalloc(&wq, 16) == cudaSuccess && cudaMemset(wq, 0, 16) == cudaSuccess &&
+      cudaStreamSynchronize(nullptr) == cudaSuccess) {
     h->plan.wq = wq;
     h->plan.sm_die = map;
     h->plan.nsmid = uint32_t(nsmid);
