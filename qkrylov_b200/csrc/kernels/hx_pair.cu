@@ -33,15 +33,21 @@ namespace qkd {
 
 struct PairPlan {
   uint32_t Du, Dd;         // up and down configurations
+  // elements per row of every product-ordered array (x_p, y_p, D, ranks): Dd
+  // rounded up to 32, so that rows start on 128-byte lines in every type and
+  // can be read as 16-byte packs (what a row holds beyond Dd is never used)
+  uint32_t ld;
   int L;                   // low bits of the sector tables
   uint32_t lmask;
   const uint64_t* A;       // sector tables (device copies owned by the qk_plan)
   const uint32_t* B;
   const uint32_t* ulist;   // up configurations (compressed site bits), ascending
   const uint32_t* dlist;
-  const uint32_t* up_ptr;  // CSR of T_up over configuration indices (Du + 1)
-  const uint32_t* up_col;
-  const double* up_val;
+  // T_up: per row its first quad and its hops; a quad is four hops (target
+  // indices, elements), the last one of a row filled with zeros
+  const uint2* up_rec;
+  const uint4* up_col;
+  const double2* up_val;
   const uint32_t* dn_ptr;  // CSR of T_dn (Dd + 1)
   const uint32_t* dn_col;
   const double* dn_val;
@@ -52,14 +58,14 @@ struct PairPlan {
   // zero pack)
   const uint2 *dn_rec, *dn_slot;
   double dn_mag[4];
-  const double* diag;      // D in product order (Du * Dd)
-  const uint32_t* perm;    // rank(u, d) in product order (Du * Dd), or null: computed from A, B
+  const double* diag;      // D in product order (Du * ld)
+  const uint32_t* perm;    // rank(u, d) in product order (Du * ld), or null: computed from A, B
 };
 
 namespace {
 
 constexpr int kMags = 4;  // magnitudes of the by-hop tables
-constexpr int kPT = 256;  // threads per CTA; k_pair_up takes row slabs of 2 * kPT elements
+constexpr int kPT = 256;  // threads per CTA of the gather
 constexpr int kDT = 1024; // k_pair_dn: one staged row shared by 32 warps (two CTAs per SM)
 
 __device__ __forceinline__ uint32_t spread16(uint32_t x) {  // bit i -> bit 2i (16 -> 32 bits)
@@ -84,6 +90,13 @@ __device__ __forceinline__ uint32_t pair_rank(const PairPlan& p, uint32_t u, uin
   return uint32_t(__ldg(p.A + (s >> p.L)) & qkb::kOffsetMask) + (__ldg(p.B + (s & p.lmask)) & qkb::kRankMask);
 }
 
+// Work items of the gather: (u, kInCols * kPT columns), kInCols columns per
+// thread so that as many ranks, then as many gathers, are in flight.
+constexpr int kInCols = 4;
+__host__ __device__ inline uint64_t in_items(uint32_t Du, uint32_t Dd) {
+  return uint64_t(Du) * ((Dd + kInCols * kPT - 1) / (kInCols * kPT));
+}
+
 // SIGN false: the plain gather (the diagonal, on which S acts twice)
 template <int DT, bool SIGN>
 __global__ void __launch_bounds__(kPT) k_pair_in(const PairPlan* __restrict__ pp, const void* __restrict__ x,
@@ -91,79 +104,126 @@ __global__ void __launch_bounds__(kPT) k_pair_in(const PairPlan* __restrict__ pp
   using T = VT<DT>;
   using R = typename T::R;
   const PairPlan& p = *pp;
-  const uint64_t n = uint64_t(p.Du) * p.Dd;
-  for (uint64_t i = blockIdx.x * uint64_t(kPT) + threadIdx.x; i < n; i += uint64_t(gridDim.x) * kPT) {
-    const uint32_t iu = uint32_t(i / p.Dd), id = uint32_t(i - uint64_t(iu) * p.Dd);
-    const uint32_t u = __ldg(p.ulist + iu), d = __ldg(p.dlist + id);
-    R re, im;
-    T::ld(x, p.perm ? __ldg(p.perm + i) : pair_rank(p, u, d), re, im);
-    const R sg = SIGN ? R(pair_sign(u, d)) : R(1);
-    T::st(xp, i, sg * re, sg * im);
+  const uint32_t Dd = p.Dd, nc = (Dd + kInCols * kPT - 1) / (kInCols * kPT);
+  const uint64_t items = in_items(p.Du, Dd);
+  for (uint64_t it = blockIdx.x; it < items; it += gridDim.x) {
+    const uint32_t iu = uint32_t(it / nc), c0 = uint32_t(it - uint64_t(iu) * nc) * (kInCols * kPT) + threadIdx.x;
+    const uint64_t row = uint64_t(iu) * p.ld;
+    const uint32_t u = __ldg(p.ulist + iu);
+    uint32_t d[kInCols], rk[kInCols];
+    #pragma unroll
+    for (int k = 0; k < kInCols; ++k) {  // spare columns of the last item repeat column Dd - 1
+      const uint32_t c = min(c0 + k * kPT, Dd - 1);
+      d[k] = __ldg(p.dlist + c);
+      rk[k] = p.perm ? __ldg(p.perm + row + c) : pair_rank(p, u, d[k]);
+    }
+    R re[kInCols], im[kInCols];
+    #pragma unroll
+    for (int k = 0; k < kInCols; ++k) T::ld(x, rk[k], re[k], im[k]);
+    #pragma unroll
+    for (int k = 0; k < kInCols; ++k) {
+      const R sg = SIGN ? R(pair_sign(u, d[k])) : R(1);
+      if (c0 + k * kPT < Dd) T::st(xp, row + c0 + k * kPT, sg * re[k], sg * im[k]);
+    }
   }
 }
 
-// perm[i] = rank(u, d) for the product index i = iu * Dd + id
+// perm[u][d] = rank(u, d)
 __global__ void __launch_bounds__(kPT) k_pair_perm(const PairPlan* __restrict__ pp, uint32_t* __restrict__ perm) {
   const PairPlan& p = *pp;
-  const uint64_t n = uint64_t(p.Du) * p.Dd;
-  for (uint64_t i = blockIdx.x * uint64_t(kPT) + threadIdx.x; i < n; i += uint64_t(gridDim.x) * kPT) {
-    const uint32_t iu = uint32_t(i / p.Dd), id = uint32_t(i - uint64_t(iu) * p.Dd);
-    perm[i] = pair_rank(p, __ldg(p.ulist + iu), __ldg(p.dlist + id));
-  }
-}
-
-// y_p[u][c0 .. c0 + 2 kPT) = sum_u' T_up[u][u'] x_p[u'][...]: work item
-// (slab, u) in slab-major order, two elements per thread
-template <int DT>
-__global__ void __launch_bounds__(kPT) k_pair_up(const PairPlan* __restrict__ pp, const void* __restrict__ xp,
-                                                 void* __restrict__ yp) {
-  using T = VT<DT>;
-  using R = typename T::R;
-  const PairPlan& p = *pp;
-  const uint32_t slab_elems = 2 * kPT;
-  const uint32_t nslab = (p.Dd + slab_elems - 1) / slab_elems;
-  const uint64_t items = uint64_t(nslab) * p.Du;
-  for (uint64_t it = blockIdx.x; it < items; it += gridDim.x) {
-    const uint32_t slab = uint32_t(it / p.Du), iu = uint32_t(it - uint64_t(slab) * p.Du);
-    const uint32_t c0 = slab * slab_elems + threadIdx.x, c1 = c0 + kPT;
-    const uint32_t k0 = __ldg(p.up_ptr + iu), k1 = __ldg(p.up_ptr + iu + 1);
-    R a0r = R(0), a0i = R(0), a1r = R(0), a1i = R(0);
-    const bool in0 = c0 < p.Dd, in1 = c1 < p.Dd;
-    uint32_t k = k0;
-    for (; k + 4 <= k1; k += 4) {  // four partner rows in flight
-      uint32_t col[4];
-      R w[4], v0r[4], v0i[4], v1r[4], v1i[4];
-      #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        col[j] = __ldg(p.up_col + k + j);
-        w[j] = R(__ldg(p.up_val + k + j));
-        const uint64_t rb = uint64_t(col[j]) * p.Dd;
-        v0r[j] = v0i[j] = v1r[j] = v1i[j] = R(0);
-        if (in0) T::ld(xp, rb + c0, v0r[j], v0i[j]);
-        if (in1) T::ld(xp, rb + c1, v1r[j], v1i[j]);
-      }
-      #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        a0r += w[j] * v0r[j]; a1r += w[j] * v1r[j];
-        if (T::cplx) { a0i += w[j] * v0i[j]; a1i += w[j] * v1i[j]; }
-      }
-    }
-    for (; k < k1; ++k) {
-      const uint64_t rb = uint64_t(__ldg(p.up_col + k)) * p.Dd;
-      const R w = R(__ldg(p.up_val + k));
-      R vr = R(0), vi = R(0);
-      if (in0) { T::ld(xp, rb + c0, vr, vi); a0r += w * vr; if (T::cplx) a0i += w * vi; }
-      if (in1) { T::ld(xp, rb + c1, vr, vi); a1r += w * vr; if (T::cplx) a1i += w * vi; }
-    }
-    const uint64_t ob = uint64_t(iu) * p.Dd;
-    if (in0) T::st(yp, ob + c0, a0r, a0i);
-    if (in1) T::st(yp, ob + c1, a1r, a1i);
+  for (uint32_t iu = blockIdx.x; iu < p.Du; iu += gridDim.x) {
+    const uint32_t u = __ldg(p.ulist + iu);
+    for (uint32_t c = threadIdx.x; c < p.Dd; c += kPT) perm[uint64_t(iu) * p.ld + c] = pair_rank(p, u, __ldg(p.dlist + c));
   }
 }
 
 // A 16-byte pack of NE elements that a hop reads with one load.
 template <class E, int NE>
 struct alignas(sizeof(E) * NE) RowPack { E v[NE]; };
+
+template <class P>
+__device__ __forceinline__ P ldg_pack(const P* p) {
+  static_assert(sizeof(P) == 16, "one 16-byte load");
+  const uint4 q = __ldg(reinterpret_cast<const uint4*>(p));
+  return *reinterpret_cast<const P*>(&q);
+}
+
+// y_p[u][...] = sum_u' T_up[u][u'] x_p[u'][...]: work item (slab of columns,
+// u) in slab-major order, so that a slab of x_p (4 KB per row, 53 MB at 12,870
+// rows) stays in L2 while its rows are combined.  The hops re-read x_p from
+// L2, and the loads bound the kernel: L1 wavefronts (88% of its rate with
+// 8-byte loads of unaligned rows and four one-word loads of index and element
+// per hop and warp) and the bytes in flight.  So: 16-byte loads of aligned
+// rows, four hops of two packs in flight per thread, three 16-byte loads for
+// the indices and elements of four hops.  Whole apply, before -> after:
+// Hubbard 4x4 float64 5.59 -> 4.86 ms, float32 3.81 -> 2.82 ms, 13 sites
+// complex64 74.1 -> 70 us.  One pack per thread with 256 threads costs
+// complex128 7% (7x2: 515 us against 480); eight hops in flight at fewer
+// CTAs, 64 x 2 and 64 x 4 threads x packs are equal or slower.
+constexpr int kUT = 128;  // threads
+constexpr int kUP = 2;    // packs per thread
+template <int DT>
+__global__ void __launch_bounds__(kUT, 8) k_pair_up(const PairPlan* __restrict__ pp, const void* __restrict__ xp,
+                                                 void* __restrict__ yp) {
+  using T = VT<DT>;
+  using R = typename T::R;
+  constexpr int NR = 16 / int(sizeof(R));  // reals per pack
+  using Pack = RowPack<R, NR>;
+  const PairPlan& p = *pp;
+  const uint32_t npk = p.ld / (16 / uint32_t(sizeof(typename T::E)));  // packs per row
+  const uint32_t nslab = (npk + kUP * kUT - 1) / (kUP * kUT);
+  const uint32_t items = nslab * p.Du;
+  for (uint32_t it = blockIdx.x; it < items; it += gridDim.x) {
+    const uint32_t slab = it / p.Du, iu = it - slab * p.Du;
+    const uint32_t c = slab * kUP * kUT + threadIdx.x;
+    const uint2 rec = __ldg(p.up_rec + iu);
+    const uint4* __restrict__ col = p.up_col + rec.x;
+    const double2* __restrict__ val = p.up_val + size_t(rec.x) * 2;
+    const Pack* x[kUP];
+    #pragma unroll
+    for (int k = 0; k < kUP; ++k) x[k] = static_cast<const Pack*>(xp) + min(c + k * kUT, npk - 1);
+    R a[kUP][NR];
+    #pragma unroll
+    for (int k = 0; k < kUP; ++k)
+      #pragma unroll
+      for (int r = 0; r < NR; ++r) a[k][r] = R(0);
+    auto add = [&](const Pack (&v)[kUP], double w) {
+      #pragma unroll
+      for (int k = 0; k < kUP; ++k)
+        #pragma unroll
+        for (int r = 0; r < NR; ++r) a[k][r] += R(w) * v[k].v[r];
+    };
+    auto ld = [&](Pack (&v)[kUP], uint32_t row) {
+      #pragma unroll
+      for (int k = 0; k < kUP; ++k) v[k] = ldg_pack(x[k] + uint64_t(row) * npk);
+    };
+    uint32_t left = rec.y;
+    Pack v[4][kUP];
+    for (; left >= 4; left -= 4, ++col, val += 2) {
+      const uint4 t = __ldg(col);
+      ld(v[0], t.x); ld(v[1], t.y); ld(v[2], t.z); ld(v[3], t.w);
+      const double2 w0 = __ldg(val), w1 = __ldg(val + 1);
+      add(v[0], w0.x); add(v[1], w0.y); add(v[2], w1.x); add(v[3], w1.y);
+    }
+    if (left) {
+      const uint4 t = __ldg(col);
+      ld(v[0], t.x);
+      if (left > 1) ld(v[1], t.y);
+      if (left > 2) ld(v[2], t.z);
+      const double2 w0 = __ldg(val), w1 = __ldg(val + 1);
+      add(v[0], w0.x);
+      if (left > 1) add(v[1], w0.y);
+      if (left > 2) add(v[2], w1.x);
+    }
+    #pragma unroll
+    for (int k = 0; k < kUP; ++k) {
+      Pack o;
+      #pragma unroll
+      for (int r = 0; r < NR; ++r) o.v[r] = a[k][r];
+      if (c + k * kUT < npk) static_cast<Pack*>(yp)[uint64_t(iu) * npk + c + k * kUT] = o;
+    }
+  }
+}
 
 __device__ __forceinline__ double flip_sign(double v, uint32_t e) {  // -v when bit 15 of e is set
   return __hiloint2double(__double2hiint(v) ^ int((e & 0x8000u) << 16), __double2loint(v));
@@ -271,7 +331,7 @@ __global__ void __launch_bounds__(NT) k_pair_dn(const PairPlan* __restrict__ pp,
         #pragma unroll
         for (int r = 0; r < NE; ++r) {
           const uint32_t k = pl * NE + r;
-          v.v[r] = k < nr ? __ldg(reinterpret_cast<const E*>(xp) + uint64_t(iu0 + k) * Dd + c) : E{};
+          v.v[r] = k < nr ? __ldg(reinterpret_cast<const E*>(xp) + uint64_t(iu0 + k) * p.ld + c) : E{};
         }
         xs[pl * stride + c] = v;
       }
@@ -286,7 +346,7 @@ __global__ void __launch_bounds__(NT) k_pair_dn(const PairPlan* __restrict__ pp,
       #pragma unroll
       for (int r = 0; r < NR; ++r) {
         const uint32_t u = iu0 + (uint32_t(r) < nr ? r : 0);
-        const uint64_t i = uint64_t(u) * Dd + c;
+        const uint64_t i = uint64_t(u) * p.ld + c;
         T::ld(yp, i, ar[r], ai[r]);
         dg[r] = __ldg(p.diag + i);
         rk[r] = p.perm ? __ldg(p.perm + i) : pair_rank(p, __ldg(p.ulist + u), d);
@@ -533,7 +593,8 @@ PairHandle* pair_plan_create(const qk_plan_desc* d, const uint64_t* A_dev, const
     }
     return true;
   };
-  std::vector<uint32_t> uptr(1, 0), ucol, dptr(1, 0), dcol;
+  std::vector<uint2> urec;
+  std::vector<uint32_t> ucol, dptr(1, 0), dcol;
   std::vector<double> uval, dval;
   std::vector<uint16_t> dhop;
   std::vector<std::pair<uint32_t, double>> r, r2;
@@ -547,14 +608,18 @@ PairHandle* pair_plan_create(const qk_plan_desc* d, const uint64_t* A_dev, const
       for (int k = 0; k < 2; ++k) {  // the row must not depend on the other species
         if (!row(up, a, o_chk[sp][k], r2) || r2 != r) return nullptr;
       }
+      if (up) urec.push_back(make_uint2(uint32_t(ucol.size() / 4), uint32_t(r.size())));
       for (auto& e : r) {
         (up ? ucol : dcol).push_back(e.first);
         (up ? uval : dval).push_back(e.second);
       }
+      for (; up && ucol.size() % 4; uval.push_back(0.0)) ucol.push_back(0);
       // the last call above was for another configuration of the other
       // species with the same result, so its hops are this row's
-      if (!up) dhop.insert(dhop.end(), hop.begin(), hop.end());
-      (up ? uptr : dptr).push_back(uint32_t((up ? ucol : dcol).size()));
+      if (!up) {
+        dhop.insert(dhop.end(), hop.begin(), hop.end());
+        dptr.push_back(uint32_t(dcol.size()));
+      }
     }
   }
   std::vector<uint2> drec, dslot;
@@ -574,13 +639,15 @@ PairHandle* pair_plan_create(const qk_plan_desc* d, const uint64_t* A_dev, const
   };
   PairPlan& h = out->host;
   h.Du = uint32_t(ul.size()); h.Dd = uint32_t(dl.size());
+  h.ld = (h.Dd + 31u) & ~31u;
+  const size_t np = size_t(h.Du) * h.ld;
   h.L = d->L; h.lmask = uint32_t((1ull << d->L) - 1);
   h.A = A_dev; h.B = B_dev;
   h.ulist = static_cast<const uint32_t*>(up_(ul.data(), ul.size() * 4));
   h.dlist = static_cast<const uint32_t*>(up_(dl.data(), dl.size() * 4));
-  h.up_ptr = static_cast<const uint32_t*>(up_(uptr.data(), uptr.size() * 4));
-  h.up_col = static_cast<const uint32_t*>(up_(ucol.data(), ucol.size() * 4));
-  h.up_val = static_cast<const double*>(up_(uval.data(), uval.size() * 8));
+  h.up_rec = static_cast<const uint2*>(up_(urec.data(), urec.size() * sizeof(uint2)));
+  h.up_col = static_cast<const uint4*>(up_(ucol.data(), ucol.size() * 4));
+  h.up_val = static_cast<const double2*>(up_(uval.data(), uval.size() * 8));
   h.dn_ptr = static_cast<const uint32_t*>(up_(dptr.data(), dptr.size() * 4));
   if (dslots) {
     h.dn_rec = static_cast<const uint2*>(up_(drec.data(), drec.size() * sizeof(uint2)));
@@ -590,7 +657,7 @@ PairHandle* pair_plan_create(const qk_plan_desc* d, const uint64_t* A_dev, const
     h.dn_val = static_cast<const double*>(up_(dval.data(), dval.size() * 8));
   }
   for (int m = 0; m < kMags; ++m) h.dn_mag[m] = dmag[m];
-  double* dp = static_cast<double*>(up_(nullptr, d->dim * 8));
+  double* dp = static_cast<double*>(up_(nullptr, np * 8));
   h.diag = dp;
   if (ok) {
     out->dev = nullptr;
@@ -599,7 +666,7 @@ PairHandle* pair_plan_create(const qk_plan_desc* d, const uint64_t* A_dev, const
     if (ok) *dev_bytes += sizeof(PairPlan);
   }
   if (ok) {  // the diagonal in product order (no sign: S D S = D)
-    const unsigned g = resident_grid(k_pair_in<QK_F64, false>, kPT, 0, 4096);
+    const unsigned g = resident_grid(k_pair_in<QK_F64, false>, kPT, 0, unsigned(std::min<uint64_t>(4096, in_items(h.Du, h.Dd))));
     k_pair_in<QK_F64, false><<<g, kPT>>>(out->dev, diag_ref, dp);
     ok = cudaGetLastError() == cudaSuccess && cudaDeviceSynchronize() == cudaSuccess;
   }
@@ -608,9 +675,9 @@ PairHandle* pair_plan_create(const qk_plan_desc* d, const uint64_t* A_dev, const
     // gather and the scatter instead of two scattered table lookups per
     // element (4 bytes per state; without the memory the kernels compute it)
     uint32_t* pm = nullptr;
-    if (cudaMalloc(&pm, d->dim * 4) == cudaSuccess) {
+    if (cudaMalloc(&pm, np * 4) == cudaSuccess) {
       out->bufs.push_back(pm);
-      *dev_bytes += d->dim * 4;
+      *dev_bytes += np * 4;
       k_pair_perm<<<resident_grid(k_pair_perm, kPT, 0, 4096), kPT>>>(out->dev, pm);
       ok = cudaGetLastError() == cudaSuccess && cudaDeviceSynchronize() == cudaSuccess;
       h.perm = pm;
@@ -633,8 +700,8 @@ PairHandle* pair_plan_create(const qk_plan_desc* d, const uint64_t* A_dev, const
 int pair_apply(const PairHandle* h, qk_dtype t, const void* x, void* y, cudaStream_t s, qk_workspace* w,
                double* dot_out) {
   if (!h || !x || !y || x == y) return QKD_EINVAL;
-  const size_t es = qk_dtype_size(t), n = size_t(h->host.Du) * h->host.Dd;
-  const size_t half = (n * es + 255) & ~size_t(255);  // x_p and y_p both on 256-byte boundaries
+  const size_t es = qk_dtype_size(t);
+  const size_t half = (size_t(h->host.Du) * h->host.ld * es + 255) & ~size_t(255);  // x_p and y_p on 256-byte boundaries
   void* scr = nullptr;
   {
     std::lock_guard<std::mutex> lk(h->mu);
@@ -694,8 +761,9 @@ int pair_apply(const PairHandle* h, qk_dtype t, const void* x, void* y, cudaStre
   }
 #define QKD_PAIR(DT)                                                                                       \
   {                                                                                                        \
-    k_pair_in<DT, true><<<resident_grid(k_pair_in<DT, true>, kPT, 0, 1u << 20), kPT, 0, s>>>(h->dev, x, xp); \
-    k_pair_up<DT><<<resident_grid(k_pair_up<DT>, kPT, 0, 1u << 20), kPT, 0, s>>>(h->dev, xp, yp);          \
+    const unsigned gi = unsigned(std::min<uint64_t>(1u << 20, in_items(h->host.Du, h->host.Dd)));          \
+    k_pair_in<DT, true><<<resident_grid(k_pair_in<DT, true>, kPT, 0, gi), kPT, 0, s>>>(h->dev, x, xp);     \
+    k_pair_up<DT><<<resident_grid(k_pair_up<DT>, kUT, 0, 1u << 20), kUT, 0, s>>>(h->dev, xp, yp);          \
     if (dot_out) QKD_PAIR_DNS(DT, true) else QKD_PAIR_DNS(DT, false)                                       \
   }
   switch (t) {
