@@ -51,11 +51,10 @@ struct PairPlan {
   const uint32_t* dn_ptr;  // CSR of T_dn (Dd + 1)
   const uint32_t* dn_col;
   const double* dn_val;
-  // T_dn by hop, when its elements have at most kMags magnitudes: per tile of
-  // 32 rows the first group and the groups of each magnitude (8 bits each); a
-  // slot is one hop, four slots of a row per uint2 ([group][lane]), each the
-  // target index with the sign in bit 15 (indices Dd .. Dd + 7: no target, a
-  // zero pack)
+  // T_dn in slots, when its elements have at most kMags magnitudes: per tile
+  // of 32 rows the first group and the groups of each magnitude (8 bits each);
+  // four slots of a row per uint2 ([group][lane]), each the target index with
+  // the sign in bit 15 (indices Dd .. Dd + 7: no target, a zero pack)
   const uint2 *dn_rec, *dn_slot;
   double dn_mag[4];
   const double* diag;      // D in product order (Du * ld)
@@ -64,7 +63,7 @@ struct PairPlan {
 
 namespace {
 
-constexpr int kMags = 4;  // magnitudes of the by-hop tables
+constexpr int kMags = 4;  // magnitudes of the slot tables
 constexpr int kPT = 256;  // threads per CTA of the gather
 constexpr int kDT = 1024; // k_pair_dn: one staged row shared by 32 warps (two CTAs per SM)
 
@@ -234,9 +233,9 @@ __device__ __forceinline__ float flip_sign(float v, uint32_t e) {
 
 // The hops of row c (tile c / 32) on the staged packs: sum over magnitudes of
 // magnitude * (sum of +-pack).  kAhead slot groups are loaded together, the
-// next ones while these are summed (Hubbard 4x4 float64, the whole kernel:
-// one group ahead 2.90 ms, four 2.67 ms).
-constexpr int kAhead = 4;
+// next ones while these are summed (whole apply, Hubbard 4x4 complex64: two
+// 4.40 ms, three 4.48, four 4.60; 7x2 float64: 262, 263, 269, six 281 us).
+constexpr int kAhead = 2;
 template <class T, class Pack, int NE>
 __device__ __forceinline__ void hop_sum(const uint2* __restrict__ rec, const uint2* __restrict__ slot,
                                         const double* mag, uint32_t c, const Pack* xs, typename T::R (&sr)[NE],
@@ -294,8 +293,9 @@ __device__ __forceinline__ void hop_sum(const uint2* __restrict__ rec, const uin
 // NE * PL rows u of the product order staged in shared memory as PL planes
 // of NE interleaved rows (16 bytes per column), so that one load fetches a
 // column of NE rows; per column d the down hops are decoded once for all rows
-// (SLOTS: from the by-hop tables, one plane; otherwise a CSR walk); per element the hops and the diagonal are added to y_p and the result
-// goes to its reference-order slot with the sign S.  DOT: <x, y> summed per
+// (SLOTS: from the slot tables, one plane; otherwise a CSR walk); per element the
+// hops and the diagonal are added to y_p and the result goes to its
+// reference-order place with the sign S.  DOT: <x, y> summed per
 // CTA in a fixed order, then over CTAs (deterministic for a given grid).
 template <int DT, bool DOT, int NE, int PL, int NT, bool SLOTS>
 __global__ void __launch_bounds__(NT) k_pair_dn(const PairPlan* __restrict__ pp, const void* __restrict__ xp,
@@ -353,7 +353,7 @@ __global__ void __launch_bounds__(NT) k_pair_dn(const PairPlan* __restrict__ pp,
       }
       R sr[NR], si[NR];
       if constexpr (SLOTS) {
-        static_assert(PL == 1, "the by-hop tables serve one plane");
+        static_assert(PL == 1, "the slot tables serve one plane");
         hop_sum<T, Pack, NE>(p.dn_rec, p.dn_slot, p.dn_mag, c, xs, sr, si);
       } else {
         const uint32_t k0 = __ldg(p.dn_ptr + c), k1 = __ldg(p.dn_ptr + c + 1);
@@ -442,17 +442,58 @@ int host_pair_sign(uint32_t u, uint32_t d, int nsites) {
 }
 }  // namespace
 
-// By-hop tables of a sparse matrix in CSR form (hop[k]: the hop of entry k,
-// at most one entry per row and hop): per tile of 32 rows and magnitude one
-// slot for every hop with an entry in at least one row.  Rows without the hop
-// point at one of eight zero packs behind the staged rows, the one whose
-// 16-byte bank group no target of their quarter warp uses, so they cost no
-// extra wavefront (4x4 torus, 8 particles: 120 wavefronts per warp; one shared
-// zero pack 157, lists packed per row 155).  False when the elements have more
-// than kMags magnitudes.
+// The slot (colour) of every entry of a quarter warp: `row[k]`, `bank[k]` (0..7)
+// of entry k, ncol >= the entries of any row and of any bank.  No two entries
+// of a slot share a row or a bank: an edge colouring of the bipartite
+// multigraph of rows and banks, which needs no more colours than its largest
+// degree (an entry without a common free colour swaps two colours along the
+// alternating path from its bank).
+static std::vector<int> quarter_slots(const std::vector<uint8_t>& row, const std::vector<uint8_t>& bank, int ncol) {
+  std::vector<int> slot(row.size(), -1), at_row(size_t(8) * ncol, -1), at_bank(size_t(8) * ncol, -1);
+  for (size_t k = 0; k < row.size(); ++k) {
+    int* r = &at_row[size_t(row[k]) * ncol];
+    int* b = &at_bank[size_t(bank[k]) * ncol];
+    int fr = -1, fb = -1, both = -1;
+    for (int c = 0; c < ncol && both < 0; ++c) {
+      if (r[c] < 0 && fr < 0) fr = c;
+      if (b[c] < 0 && fb < 0) fb = c;
+      if (r[c] < 0 && b[c] < 0) both = c;
+    }
+    if (both < 0) {
+      std::vector<int> path;
+      int c = fr;  // the path leaves the bank by the row's free colour, then by the bank's
+      for (int e = b[c]; e >= 0;) {
+        path.push_back(e);
+        const bool to_row = path.size() & 1;
+        c = c == fr ? fb : fr;
+        e = to_row ? at_row[size_t(row[e]) * ncol + c] : at_bank[size_t(bank[e]) * ncol + c];
+      }
+      for (int e : path) at_row[size_t(row[e]) * ncol + slot[e]] = at_bank[size_t(bank[e]) * ncol + slot[e]] = -1;
+      for (int e : path) {
+        slot[e] = slot[e] == fr ? fb : fr;
+        at_row[size_t(row[e]) * ncol + slot[e]] = at_bank[size_t(bank[e]) * ncol + slot[e]] = e;
+      }
+      both = fr;
+    }
+    slot[k] = both;
+    r[both] = b[both] = int(k);
+  }
+  return slot;
+}
+
+// Slot tables of a sparse matrix in CSR form: per tile of 32 rows and
+// magnitude, the entries of each row spread over slots so that the eight rows
+// of a quarter warp read eight different 16-byte bank groups in every slot:
+// a 16-byte load is then four wavefronts, the least it can take.  Rows without
+// an entry in a slot point at that one of the eight zero packs behind the
+// staged rows whose bank group is still free.  The slots of a tile are the
+// entries of its fullest row or bank, to a multiple of four: 4x4 torus, 8
+// particles, 17.1 entries per row, 24 slots and 96 wavefronts per warp (one
+// slot per hop of the lattice: 28.9 slots and 134 wavefronts, the whole kernel
+// 2.69 -> 2.35 ms; the same slots by position in the row: 155 wavefronts).
+// False when the elements have more than kMags magnitudes.
 static bool hop_slots(const std::vector<uint32_t>& ptr, const std::vector<uint32_t>& col,
-                      const std::vector<double>& val, const std::vector<uint16_t>& hop, size_t nhop, double* mag,
-                      std::vector<uint2>& rec, std::vector<uint2>& slot) {
+                      const std::vector<double>& val, double* mag, std::vector<uint2>& rec, std::vector<uint2>& slot) {
   const uint32_t n = uint32_t(ptr.size() - 1);
   if (n + 8 > 0x8000u) return false;
   int nmag = 0;
@@ -464,9 +505,6 @@ static bool hop_slots(const std::vector<uint32_t>& ptr, const std::vector<uint32
     if (m == nmag) mag[nmag++] = std::abs(val[k]);
     cls[k] = uint8_t(m);
   }
-  constexpr uint16_t kNone = 0xFFFFu;
-  std::vector<uint16_t> s(std::max<size_t>(nhop, 1) * 32);  // [hop][lane] of one magnitude
-  std::vector<uint8_t> used(std::max<size_t>(nhop, 1));
   for (uint32_t r0 = 0; r0 < n; r0 += 32) {
     uint2 rc = make_uint2(uint32_t(slot.size() / 32), 0u);
     int out = 0;
@@ -476,34 +514,43 @@ static bool hop_slots(const std::vector<uint32_t>& ptr, const std::vector<uint32
     int last = -1;
     for (uint32_t k = ptr[r0]; k < ptr[std::min(n, r0 + 32)]; ++k) last = std::max(last, int(cls[k]));
     for (int m = 0; m <= last; ++m, ++out) {
-      std::fill(s.begin(), s.end(), kNone);
-      std::fill(used.begin(), used.end(), uint8_t(0));
-      for (uint32_t i = 0; i < 32 && r0 + i < n; ++i)
-        for (uint32_t k = ptr[r0 + i]; k < ptr[r0 + i + 1]; ++k)
-          if (cls[k] == m) {
-            s[size_t(hop[k]) * 32 + i] = uint16_t(col[k] | (val[k] < 0 ? 0x8000u : 0u));
-            used[hop[k]] = 1;
-          }
-      std::vector<uint32_t> on;
-      for (uint32_t q = 0; q < nhop; ++q) if (used[q]) on.push_back(q);
-      for (uint32_t q : on)
-        for (uint32_t ph = 0; ph < 32; ph += 8) {  // quarter warps
-          uint32_t banks = 0, z = 0;
-          for (uint32_t i = ph; i < ph + 8; ++i)
-            if (s[q * 32 + i] != kNone) banks |= 1u << (s[q * 32 + i] & 7u);
-          while (z < 7 && (banks >> ((n + z) & 7u) & 1u)) ++z;
-          for (uint32_t i = ph; i < ph + 8; ++i)
-            if (s[q * 32 + i] == kNone) s[q * 32 + i] = uint16_t(n + z);
-        }
-      const uint32_t ng = std::max<uint32_t>(1, uint32_t((on.size() + 3) / 4));
+      std::vector<uint8_t> row[4], bank[4];
+      std::vector<uint32_t> ent[4];
+      int need = 1;
+      for (uint32_t q = 0; q < 4; ++q) {
+        int nr[8] = {}, nb[8] = {};
+        for (uint32_t i = 0; i < 8 && r0 + 8 * q + i < n; ++i)
+          for (uint32_t k = ptr[r0 + 8 * q + i]; k < ptr[r0 + 8 * q + i + 1]; ++k)
+            if (cls[k] == m) {
+              row[q].push_back(uint8_t(i));
+              bank[q].push_back(uint8_t(col[k] & 7u));
+              ent[q].push_back(col[k] | (val[k] < 0 ? 0x8000u : 0u));
+              need = std::max({need, ++nr[i], ++nb[col[k] & 7u]});
+            }
+      }
+      const uint32_t ng = uint32_t(need + 3) / 4;
       if (ng > 255) return false;
       rc.y |= ng << (8 * out);
+      std::vector<uint32_t> t(size_t(ng) * 4 * 32, ~0u);  // [slot][lane]
+      for (uint32_t q = 0; q < 4; ++q) {
+        const std::vector<int> s = quarter_slots(row[q], bank[q], int(ng) * 4);
+        for (size_t k = 0; k < s.size(); ++k) t[size_t(s[k]) * 32 + 8 * q + row[q][k]] = ent[q][k];
+        for (uint32_t c = 0; c < ng * 4; ++c) {
+          uint32_t banks = 0, z = 0;
+          uint32_t* l = &t[size_t(c) * 32 + 8 * q];
+          for (int i = 0; i < 8; ++i)
+            if (l[i] != ~0u) banks |= 1u << (l[i] & 7u);
+          for (int i = 0; i < 8; ++i)
+            if (l[i] == ~0u) {
+              while (banks >> ((n + z) & 7u) & 1u) ++z;
+              l[i] = n + z++;
+            }
+        }
+      }
       for (uint32_t g = 0; g < ng; ++g)
         for (uint32_t i = 0; i < 32; ++i) {
-          uint32_t t[4];
-          for (uint32_t u = 0; u < 4; ++u)  // padding: one address, a broadcast
-            t[u] = 4 * g + u < on.size() ? s[size_t(on[4 * g + u]) * 32 + i] : n;
-          slot.push_back(make_uint2(t[0] | (t[1] << 16), t[2] | (t[3] << 16)));
+          const uint32_t* u = &t[size_t(g) * 128 + i];
+          slot.push_back(make_uint2(u[0] | (u[32] << 16), u[64] | (u[96] << 16)));
         }
     }
     rec.push_back(rc);
@@ -565,15 +612,13 @@ PairHandle* pair_plan_create(const qk_plan_desc* d, const uint64_t* A_dev, const
   for (uint32_t i = 0; i < dl.size(); ++i) didx[dl[i]] = i;
   // row `a` of T_species at a fixed configuration `o` of the other species:
   // (column index, value) pairs in term order
-  std::vector<uint16_t> hop;  // of each pair: its position among the species' groups
   auto row = [&](bool up, uint32_t a, uint32_t o, std::vector<std::pair<uint32_t, double>>& out) -> bool {
     out.clear();
-    hop.clear();
     const uint64_t s = up ? interleave(a, o, ns) : interleave(o, a, ns);
     const int ss = up ? host_pair_sign(a, o, ns) : host_pair_sign(o, a, ns);
     const std::vector<uint32_t>& groups = up ? gup : gdn;
-    for (size_t gq = 0; gq < groups.size(); ++gq) {
-      const qk_group_t& g = d->groups[groups[gq]];
+    for (uint32_t gi : groups) {
+      const qk_group_t& g = d->groups[gi];
       const uint64_t t = s ^ g.flip;
       double c = 0.0;
       for (uint32_t q = g.first; q < g.first + g.count; ++q) {
@@ -589,14 +634,12 @@ PairHandle* pair_plan_create(const qk_plan_desc* d, const uint64_t* A_dev, const
       if (idx == ~0u) return false;
       const int ts = up ? host_pair_sign(a2, o, ns) : host_pair_sign(o, a2, ns);
       out.push_back({idx, double(ss * ts) * c});
-      hop.push_back(uint16_t(gq));
     }
     return true;
   };
   std::vector<uint2> urec;
   std::vector<uint32_t> ucol, dptr(1, 0), dcol;
   std::vector<double> uval, dval;
-  std::vector<uint16_t> dhop;
   std::vector<std::pair<uint32_t, double>> r, r2;
   const uint32_t o_chk[2][2] = {{dl[dl.size() / 2], dl.back()}, {ul[ul.size() / 2], ul.back()}};
   for (int sp = 0; sp < 2; ++sp) {
@@ -614,17 +657,12 @@ PairHandle* pair_plan_create(const qk_plan_desc* d, const uint64_t* A_dev, const
         (up ? uval : dval).push_back(e.second);
       }
       for (; up && ucol.size() % 4; uval.push_back(0.0)) ucol.push_back(0);
-      // the last call above was for another configuration of the other
-      // species with the same result, so its hops are this row's
-      if (!up) {
-        dhop.insert(dhop.end(), hop.begin(), hop.end());
-        dptr.push_back(uint32_t(dcol.size()));
-      }
+      if (!up) dptr.push_back(uint32_t(dcol.size()));
     }
   }
   std::vector<uint2> drec, dslot;
   double dmag[kMags] = {0.0, 0.0, 0.0, 0.0};
-  const bool dslots = hop_slots(dptr, dcol, dval, dhop, gdn.size(), dmag, drec, dslot);
+  const bool dslots = hop_slots(dptr, dcol, dval, dmag, drec, dslot);
   auto* out = new PairHandle;
   bool ok = true;
   auto up_ = [&](const void* src, size_t bytes) -> void* {

@@ -37,7 +37,7 @@ def magnitudes(n, k):
     (9, 2, 7, O.hubbard_square(9, 1, 1.0, 4.0)),     # 36 x 36
     (11, 5, 6, O.hubbard_square(11, 1, 1.0, 4.0)),   # 462 x 462
     (8, 4, 4, magnitudes(8, 3)),                     # three hop amplitudes
-    (9, 5, 4, magnitudes(9, 9)),                     # nine: more than the by-hop tables hold
+    (9, 5, 4, magnitudes(9, 9)),                     # nine: more than the slot tables hold
     (8, 3, 4, O.hubbard_square(2, 4, 1.0, 4.0)),     # doubled bonds: two amplitudes
 ])
 def test_spin_product_kernels_match_the_oracle(N, nup, ndn, terms):
