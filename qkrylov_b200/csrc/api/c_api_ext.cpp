@@ -190,6 +190,7 @@ int qkrylov_hamiltonian_apply_device(qkrylov_hamiltonian_h h, int dtype, const v
   if (!h || !h->op || !x || !y || !valid_dtype(dtype)) return QKRYLOV_ERROR_INVALID_ARG;
   return guarded([&] {
     auto& c = h->op->ctx();
+    if (!stream) h->op->first_use(qk_dtype(dtype));
     const int rc = qkd_apply(h->op->plan(), qk_dtype(dtype), x, y, stream ? cudaStream_t(stream) : c.stream);
     if (rc == QKD_EINVAL) { qkapi::set_error("invalid dtype for this operator or aliased x/y"); return QKRYLOV_ERROR_INVALID_ARG; }
     qkb::qkd_check(rc, "H.x");
