@@ -11,9 +11,11 @@
 //   staging  x of the G blocks interleaved in 16-byte packs ([plane][position],
 //            16 / sizeof(element) blocks per pack), so that a low target is one
 //            16-byte load per plane
-//   low      slots by bond: a slot holds one bond's targets of 32 consecutive
-//            positions (a warp), so its addresses are nearly consecutive; four
-//            slots per 8-byte table load, grouped by coefficient class
+//   low      the targets of 32 consecutive positions (a warp) in slots without
+//            bank conflicts (hx_slots.hpp), four slots per 8-byte table load,
+//            grouped by coefficient class; one slot per bond instead, half of its
+//            rows without the bond: t-J N=20 complex128 424 -> 451 us, J1-J2
+//            N=24 float64 71.7 -> 76.0, Heisenberg N=28 complex128 893 -> 918
 //   high     per block, its entries (partner block, coefficient) from shared
 //            memory; U entries of every block in flight, without branches
 //   crossing per row table words shared by the G blocks
@@ -24,10 +26,10 @@
 // float32 and complex128, 48 registers and 40 warps for the 8-byte types; more
 // entries in flight, tables or slots loaded a row ahead and unconditional
 // crossing loads were each slower.  us per apply, one-block kernel -> this one:
-// Heisenberg N=24 float32 46.6 -> 35.1, N=25 float64 99 -> 73, N=24 complex128
-// 86 -> 66, N=28 float32 437 -> 331, float64 590 -> 529, complex128 980 -> 922;
-// J1-J2 N=24 float32 81 -> 57; t-J N=19 float64 177 -> 102, N=20 float64 329 ->
-// 278, complex128 529 -> 453.
+// Heisenberg N=24 float32 46.6 -> 33.9, N=25 float64 99 -> 70, N=24 complex128
+// 86 -> 63, N=28 float32 437 -> 323, float64 590 -> 522, complex128 980 -> 893;
+// J1-J2 N=24 float32 81 -> 54; t-J N=19 float64 177 -> 96, N=20 float64 329 ->
+// 264, complex128 529 -> 424.
 #include <algorithm>
 #include <cstring>
 #include <map>
@@ -272,7 +274,7 @@ k_hx_group(const __grid_constant__ GroupPlan p, const void* __restrict__ x, void
           tw = twn;
         }
       }
-      // low bonds: slot groups two ahead, summed per coefficient class
+      // low bonds: summed per coefficient class
       uint32_t left = wr.y & 0xFFu;
       int cls = 0;
       R sr[G], si[G];

@@ -26,6 +26,7 @@
 #include <mutex>
 #include <vector>
 
+#include "hx_slots.hpp"
 #include "reduce.cuh"
 #include "../engine/sector.hpp"
 
@@ -442,56 +443,11 @@ int host_pair_sign(uint32_t u, uint32_t d, int nsites) {
 }
 }  // namespace
 
-// The slot (colour) of every entry of a quarter warp: `row[k]`, `bank[k]` (0..7)
-// of entry k, ncol >= the entries of any row and of any bank.  No two entries
-// of a slot share a row or a bank: an edge colouring of the bipartite
-// multigraph of rows and banks, which needs no more colours than its largest
-// degree (an entry without a common free colour swaps two colours along the
-// alternating path from its bank).
-static std::vector<int> quarter_slots(const std::vector<uint8_t>& row, const std::vector<uint8_t>& bank, int ncol) {
-  std::vector<int> slot(row.size(), -1), at_row(size_t(8) * ncol, -1), at_bank(size_t(8) * ncol, -1);
-  for (size_t k = 0; k < row.size(); ++k) {
-    int* r = &at_row[size_t(row[k]) * ncol];
-    int* b = &at_bank[size_t(bank[k]) * ncol];
-    int fr = -1, fb = -1, both = -1;
-    for (int c = 0; c < ncol && both < 0; ++c) {
-      if (r[c] < 0 && fr < 0) fr = c;
-      if (b[c] < 0 && fb < 0) fb = c;
-      if (r[c] < 0 && b[c] < 0) both = c;
-    }
-    if (both < 0) {
-      std::vector<int> path;
-      int c = fr;  // the path leaves the bank by the row's free colour, then by the bank's
-      for (int e = b[c]; e >= 0;) {
-        path.push_back(e);
-        const bool to_row = path.size() & 1;
-        c = c == fr ? fb : fr;
-        e = to_row ? at_row[size_t(row[e]) * ncol + c] : at_bank[size_t(bank[e]) * ncol + c];
-      }
-      for (int e : path) at_row[size_t(row[e]) * ncol + slot[e]] = at_bank[size_t(bank[e]) * ncol + slot[e]] = -1;
-      for (int e : path) {
-        slot[e] = slot[e] == fr ? fb : fr;
-        at_row[size_t(row[e]) * ncol + slot[e]] = at_bank[size_t(bank[e]) * ncol + slot[e]] = e;
-      }
-      both = fr;
-    }
-    slot[k] = both;
-    r[both] = b[both] = int(k);
-  }
-  return slot;
-}
-
-// Slot tables of a sparse matrix in CSR form: per tile of 32 rows and
-// magnitude, the entries of each row spread over slots so that the eight rows
-// of a quarter warp read eight different 16-byte bank groups in every slot:
-// a 16-byte load is then four wavefronts, the least it can take.  Rows without
-// an entry in a slot point at that one of the eight zero packs behind the
-// staged rows whose bank group is still free.  The slots of a tile are the
-// entries of its fullest row or bank, to a multiple of four: 4x4 torus, 8
-// particles, 17.1 entries per row, 24 slots and 96 wavefronts per warp (one
-// slot per hop of the lattice: 28.9 slots and 134 wavefronts, the whole kernel
-// 2.69 -> 2.35 ms; the same slots by position in the row: 155 wavefronts).
-// False when the elements have more than kMags magnitudes.
+// Slot tables (SlotTile) of a sparse matrix in CSR form, per tile of 32 rows
+// and magnitude.  4x4 torus, 8 particles, 17.1 entries per row: 24 slots and 96
+// wavefronts per warp (one slot per hop of the lattice: 28.9 slots and 134
+// wavefronts, the whole kernel 2.69 -> 2.35 ms; by position in the row: 155
+// wavefronts).  False when the elements have more than kMags magnitudes.
 static bool hop_slots(const std::vector<uint32_t>& ptr, const std::vector<uint32_t>& col,
                       const std::vector<double>& val, double* mag, std::vector<uint2>& rec, std::vector<uint2>& slot) {
   const uint32_t n = uint32_t(ptr.size() - 1);
@@ -514,44 +470,14 @@ static bool hop_slots(const std::vector<uint32_t>& ptr, const std::vector<uint32
     int last = -1;
     for (uint32_t k = ptr[r0]; k < ptr[std::min(n, r0 + 32)]; ++k) last = std::max(last, int(cls[k]));
     for (int m = 0; m <= last; ++m, ++out) {
-      std::vector<uint8_t> row[4], bank[4];
-      std::vector<uint32_t> ent[4];
-      int need = 1;
-      for (uint32_t q = 0; q < 4; ++q) {
-        int nr[8] = {}, nb[8] = {};
-        for (uint32_t i = 0; i < 8 && r0 + 8 * q + i < n; ++i)
-          for (uint32_t k = ptr[r0 + 8 * q + i]; k < ptr[r0 + 8 * q + i + 1]; ++k)
-            if (cls[k] == m) {
-              row[q].push_back(uint8_t(i));
-              bank[q].push_back(uint8_t(col[k] & 7u));
-              ent[q].push_back(col[k] | (val[k] < 0 ? 0x8000u : 0u));
-              need = std::max({need, ++nr[i], ++nb[col[k] & 7u]});
-            }
-      }
-      const uint32_t ng = uint32_t(need + 3) / 4;
+      SlotTile t(0x7FFFu);
+      for (uint32_t i = 0; i < 32 && r0 + i < n; ++i)
+        for (uint32_t k = ptr[r0 + i]; k < ptr[r0 + i + 1]; ++k)
+          if (cls[k] == m) t.add(i, col[k] | (val[k] < 0 ? 0x8000u : 0u));
+      const uint32_t ng = std::max(1u, t.groups());
       if (ng > 255) return false;
       rc.y |= ng << (8 * out);
-      std::vector<uint32_t> t(size_t(ng) * 4 * 32, ~0u);  // [slot][lane]
-      for (uint32_t q = 0; q < 4; ++q) {
-        const std::vector<int> s = quarter_slots(row[q], bank[q], int(ng) * 4);
-        for (size_t k = 0; k < s.size(); ++k) t[size_t(s[k]) * 32 + 8 * q + row[q][k]] = ent[q][k];
-        for (uint32_t c = 0; c < ng * 4; ++c) {
-          uint32_t banks = 0, z = 0;
-          uint32_t* l = &t[size_t(c) * 32 + 8 * q];
-          for (int i = 0; i < 8; ++i)
-            if (l[i] != ~0u) banks |= 1u << (l[i] & 7u);
-          for (int i = 0; i < 8; ++i)
-            if (l[i] == ~0u) {
-              while (banks >> ((n + z) & 7u) & 1u) ++z;
-              l[i] = n + z++;
-            }
-        }
-      }
-      for (uint32_t g = 0; g < ng; ++g)
-        for (uint32_t i = 0; i < 32; ++i) {
-          const uint32_t* u = &t[size_t(g) * 128 + i];
-          slot.push_back(make_uint2(u[0] | (u[32] << 16), u[64] | (u[96] << 16)));
-        }
+      t.write(ng, n, slot);
     }
     rec.push_back(rc);
   }

@@ -19,6 +19,7 @@
 
 #include "hx_group.hpp"
 #include "hx_rows.cuh"
+#include "hx_slots.hpp"
 
 namespace qkd {
 
@@ -859,54 +860,28 @@ static std::vector<uint32_t> record_order(const std::vector<uint32_t>& rec_h, in
 
 // Warp tiles of the grouped row kernel from the low targets of every position
 // (ent[off[pos] .. off[pos + 1])): per class of low parts, runs of 32
-// positions; per run and coefficient class one slot for every bond with a
-// target in at least one row.  tile0[key]: first tile of the class.
-struct LowEnt { uint16_t bond, cls, rank; };
+// positions; per run and coefficient class the targets in conflict-free slots
+// (SlotTile).  tile0[key]: first tile of the class.
+struct LowEnt { uint16_t cls, rank; };
 static bool warp_tiles(const uint32_t* key_off, uint32_t nkeys, const std::vector<uint32_t>& off,
-                       const std::vector<LowEnt>& ent, int nbond, int ncls, uint32_t zero_slot,
+                       const std::vector<LowEnt>& ent, int ncls, uint32_t zero_slot,
                        std::vector<uint2>& wrec, std::vector<uint2>& wgrp, std::vector<uint32_t>& tile0) {
   if (zero_slot + 8 > 0xFFFFu) return false;
-  std::vector<uint16_t> slots;  // [class * nbond + bond][lane]
-  std::vector<uint8_t> used(size_t(ncls) * nbond);
-  slots.resize(size_t(ncls) * nbond * 32);
   tile0.assign(nkeys, 0);
   for (uint32_t key = 0; key < nkeys; ++key) {
     tile0[key] = uint32_t(wrec.size());
     for (uint32_t p0 = key_off[key]; p0 < key_off[key + 1]; p0 += 32) {
       const uint32_t n = std::min(32u, key_off[key + 1] - p0);
-      std::fill(used.begin(), used.end(), uint8_t(0));
-      std::fill(slots.begin(), slots.end(), uint16_t(0xFFFFu));
-      for (uint32_t i = 0; i < n; ++i)
-        for (uint32_t e = off[p0 + i]; e < off[p0 + i + 1]; ++e) {
-          const size_t q = size_t(ent[e].cls) * nbond + ent[e].bond;
-          used[q] = 1;
-          slots[q * 32 + i] = ent[e].rank;
-        }
       uint2 rec = make_uint2(uint32_t(wgrp.size() / 32), 0u);
       for (int c = 0; c < ncls; ++c) {
-        std::vector<size_t> on;
-        for (int b = 0; b < nbond; ++b)
-          if (used[size_t(c) * nbond + b]) on.push_back(size_t(c) * nbond + b);
-        // rows without the bond point at the one of eight zero packs whose
-        // 16-byte bank group no target of their quarter warp uses
-        for (size_t q : on)
-          for (uint32_t ph = 0; ph < 32; ph += 8) {
-            uint32_t banks = 0, z = 0;
-            for (uint32_t i = ph; i < ph + 8; ++i)
-              if (slots[q * 32 + i] != 0xFFFFu) banks |= 1u << (slots[q * 32 + i] & 7u);
-            while (z < 7 && (banks >> ((zero_slot + z) & 7u) & 1u)) ++z;
-            for (uint32_t i = ph; i < ph + 8; ++i)
-              if (slots[q * 32 + i] == 0xFFFFu) slots[q * 32 + i] = uint16_t(zero_slot + z);
-          }
-        const uint32_t ng = uint32_t((on.size() + 3) / 4);
+        SlotTile t(0xFFFFu);
+        for (uint32_t i = 0; i < n; ++i)
+          for (uint32_t e = off[p0 + i]; e < off[p0 + i + 1]; ++e)
+            if (ent[e].cls == c) t.add(i, ent[e].rank);
+        const uint32_t ng = t.groups();
         if (ng > 255) return false;
         rec.y |= ng << (8 * c);
-        for (uint32_t g = 0; g < ng; ++g)
-          for (uint32_t i = 0; i < 32; ++i) {
-            uint32_t t[4];
-            for (uint32_t u = 0; u < 4; ++u) t[u] = 4 * g + u < on.size() ? slots[on[4 * g + u] * 32 + i] : zero_slot;
-            wgrp.push_back(make_uint2(t[0] | (t[1] << 16), t[2] | (t[3] << 16)));
-          }
+        t.write(ng, zero_slot, wgrp);
       }
       wrec.push_back(rec);
     }
@@ -1044,7 +1019,7 @@ SpinHandle* spin_plan_create(const qk_plan_desc* d, size_t* dev_bytes) {
   }
 
   // coefficient table and the per-part target lists the row tables are built from
-  std::vector<uint32_t> loff, lent, lbond, hoff, hlst;
+  std::vector<uint32_t> loff, lent, hoff, hlst;
   std::vector<uint2> hent;
   if (lean) {
     auto coef_index = [&](double c) -> uint32_t {
@@ -1061,7 +1036,6 @@ SpinHandle* spin_plan_create(const qk_plan_desc* d, size_t* dev_bytes) {
         if (v == 0 || v == m) continue;
         const double c = ((v >> h.low_i[q]) & 1u) ? h.low_c10[q] : h.low_c01[q];
         lent.push_back(((d->B[l ^ m] & 0xFFFFu) << 8) | coef_index(c));
-        lbond.push_back(uint32_t(q));
       }
     }
     loff[d->nllist] = uint32_t(lent.size());
@@ -1153,8 +1127,8 @@ SpinHandle* spin_plan_create(const qk_plan_desc* d, size_t* dev_bytes) {
     if (h.rows_ok) {
       std::vector<LowEnt> ent(loff[d->nllist]);
       for (size_t e = 0; e < ent.size(); ++e)
-        ent[e] = LowEnt{uint16_t(lbond[e]), uint16_t(cls_of[lent[e] & 0xFFu]), uint16_t(lent[e] >> 8)};
-      if (!warp_tiles(d->key_off, d->nkeys, loff, ent, std::max(1, h.nlow), std::max(1, h.ncls), h.zero_slot, wrec, wgrp, tile0))
+        ent[e] = LowEnt{uint16_t(cls_of[lent[e] & 0xFFu]), uint16_t(lent[e] >> 8)};
+      if (!warp_tiles(d->key_off, d->nkeys, loff, ent, std::max(1, h.ncls), h.zero_slot, wrec, wgrp, tile0))
         wrec.clear();
       tile_of.assign(d->nA, 0);
     }
@@ -1375,7 +1349,7 @@ SpinHandle* gen_plan_create(const qk_plan_desc* d, size_t* dev_bytes) {
         ci = int(cls.size()) - 1;
       }
       bucket[ci].push_back(uint16_t(d->B[lt] & 0xFFFFu));
-      went.push_back(LowEnt{uint16_t(q), uint16_t(ci), uint16_t(d->B[lt] & 0xFFFFu)});
+      went.push_back(LowEnt{uint16_t(ci), uint16_t(d->B[lt] & 0xFFFFu)});
     }
     rrec[pos].x = uint32_t(lgrp.size());
     uint32_t counts = 0;
@@ -1411,7 +1385,7 @@ SpinHandle* gen_plan_create(const qk_plan_desc* d, size_t* dev_bytes) {
   woff[nll] = uint32_t(went.size());
   std::vector<uint2> wrec, wgrp;
   std::vector<uint32_t> tile0, tile_of;
-  if (!warp_tiles(d->key_off, d->nkeys, woff, went, std::max<int>(1, int(lowg.size())), std::max(1, h.ncls), h.zero_slot,
+  if (!warp_tiles(d->key_off, d->nkeys, woff, went, std::max(1, h.ncls), h.zero_slot,
                   wrec, wgrp, tile0))
     wrec.clear();
   // block records of the non-empty blocks
