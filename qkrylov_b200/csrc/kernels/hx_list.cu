@@ -62,6 +62,7 @@ struct ListHandle {
 
 struct BlockListPlan {
   uint32_t dim;
+  uint32_t tile;          // rows per tile
   const uint32_t* start;  // per row: first 4-word group (dim + 1)
   const uint4* words;
   const double* diag;     // or null
@@ -189,7 +190,13 @@ __global__ void __launch_bounds__(256) k_packed_build(DevPlan p, uint32_t dim, c
 // 1117 -> 624 and 2173 -> 1514 us; t-J N=20, 64 vectors float32 4.97 -> 3.41,
 // float64 9.24 -> 6.60 ms; t-J N=13, 64 float32 56 -> 18 us.  Tiles of
 // kBlockTile rows from a queue per die; column dots per tile (sum_items).
+// Sectors with fewer than kBlockTiles tiles (two per resident CTA) take tiles
+// of 64 or 32 rows, so that a warp's rows, one after the other, are not the
+// length of the kernel: J1-J2 N=16, 64 float32 vectors 20.5 -> 12.5 us, t-J
+// N=14, 64 float64 101 -> 82 us; a limit of 148 * 20 or 148 * 40 costs J1-J2
+// N=22, 32 float64 0 and 4%.
 constexpr uint32_t kBlockTile = 128;
+constexpr uint32_t kBlockTileMin = 32, kBlockTiles = 148 * 10;
 template <class E, int VPL> struct alignas(sizeof(E) * VPL >= 16 ? 16 : sizeof(E) * VPL) ListPack { E v[VPL]; };
 template <int DT> __device__ __forceinline__ void unpk(const typename VT<DT>::E& e, typename VT<DT>::R& re, typename VT<DT>::R& im) {
   if constexpr (VT<DT>::cplx) { re = e.x; im = e.y; } else { re = e; im = typename VT<DT>::R(0); }
@@ -235,11 +242,11 @@ k_hx_block_list(const __grid_constant__ BlockListPlan p, const void* __restrict_
   for (int v = 0; v < VPL; ++v) gcol[v] = gacc ? R(gacc[l * VPL + v]) : R(1);
   for (uint32_t it = 1; tile < ntiles; ++it) {
     if (threadIdx.x == 0) s_tile[it & 1] = fetch(tile);
-    const uint32_t r1 = min(p.dim, (tile + 1) * kBlockTile);
+    const uint32_t r1 = min(p.dim, (tile + 1) * p.tile);
     double dr[VPL], di[VPL];
     #pragma unroll
     for (int v = 0; v < VPL; ++v) { dr[v] = 0.0; di[v] = 0.0; }
-    uint32_t r = tile * kBlockTile + warp * RPW + sub;
+    uint32_t r = tile * p.tile + warp * RPW + sub;
     uint32_t b0 = 0, b1 = 0;
     if (r < r1) { b0 = __ldg(p.start + r); b1 = __ldg(p.start + r + 1); }
     for (; r < r1; r += (256 / 32) * RPW) {
@@ -687,6 +694,8 @@ BlockListHandle* block_list_create(const DevPlan& p, uint64_t dim, const double*
   h->bufs[2] = wq;
   *dev_bytes += hs.size() * 4 + std::max<uint64_t>(total, 1) * 16;
   h->plan.dim = uint32_t(dim);
+  h->plan.tile = kBlockTile;
+  while (h->plan.tile > kBlockTileMin && dim / h->plan.tile < kBlockTiles) h->plan.tile /= 2;
   h->plan.start = start;
   h->plan.words = reinterpret_cast<const uint4*>(words);
   h->plan.diag = diag;
@@ -704,7 +713,7 @@ int block_list_apply(const BlockListHandle* h, qk_dtype t, int R, int lpr, bool 
                      double* dots, cudaStream_t s, const double* gacc) {
   BlockListPlan p = h->plan;
   if (!queues) p.wq = nullptr;
-  const uint32_t ntiles = (p.dim + kBlockTile - 1) / kBlockTile;
+  const uint32_t ntiles = (p.dim + p.tile - 1) / p.tile;
   const uint32_t qsplit = uint32_t(uint64_t(ntiles) * p.n0 / std::max(1, p.n0 + p.n1));
   double* part = nullptr;
   if (dots) {
