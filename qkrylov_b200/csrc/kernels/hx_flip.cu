@@ -111,6 +111,10 @@ k_hx_flip(const FlipPlan p, const void* __restrict__ x, void* __restrict__ y, do
       for (int k = 0; k < K; ++k) T::ld(x, (r0 + k * NT) ^ flip, vr[k], vi[k]);
       add(g, vr, vi);
     }
+    // the low flips in a sum of their own: half the terms, half the rounding
+    R hr[K], hi[K];
+    #pragma unroll
+    for (int k = 0; k < K; ++k) { hr[k] = ar[k]; hi[k] = ai[k]; ar[k] = R(0); ai[k] = R(0); }
     for (uint32_t g = 0; g < nlow; ++g) {
       const uint32_t flip = s_m[g].x;
       R vr[K], vi[K];
@@ -121,8 +125,8 @@ k_hx_flip(const FlipPlan p, const void* __restrict__ x, void* __restrict__ y, do
     #pragma unroll
     for (int k = 0; k < K; ++k) {
       const uint32_t row = r0 + k * NT;
-      ar[k] += R(d[k]) * xr[k];
-      if (T::cplx) ai[k] += R(d[k]) * xi[k];
+      ar[k] = ar[k] + hr[k] + R(d[k]) * xr[k];
+      if (T::cplx) ai[k] = ai[k] + hi[k] + R(d[k]) * xi[k];
       if (row >= p.row_lo && row < p.row_hi) {
         T::st(y, row, ar[k], ai[k]);
         if (DOT) {

@@ -259,11 +259,7 @@ k_hx_block_list(const __grid_constant__ BlockListPlan p, const void* __restrict_
       if (rn < r1) { b0 = __ldg(p.start + rn); b1 = __ldg(p.start + rn + 1); }
       R ar[VPL], ai[VPL];
       #pragma unroll
-      for (int v = 0; v < VPL; ++v) {
-        unpk<DT>(own.v[v], ar[v], ai[v]);
-        ar[v] *= d;
-        if (T::cplx) ai[v] *= d;
-      }
+      for (int v = 0; v < VPL; ++v) { ar[v] = R(0); ai[v] = R(0); }
       for (uint32_t j = 0; j < n; ++j) {
         const uint32_t e[4] = {q.x, q.y, q.z, q.w};
         Pack t[4];
@@ -283,6 +279,14 @@ k_hx_block_list(const __grid_constant__ BlockListPlan p, const void* __restrict_
               if (T::cplx) ai[v] += c * vi;
             }
           }
+      }
+      // the diagonal last: the hops are rounded against their own sum
+      #pragma unroll
+      for (int v = 0; v < VPL; ++v) {
+        R xr, xi;
+        unpk<DT>(own.v[v], xr, xi);
+        ar[v] += d * xr;
+        if (T::cplx) ai[v] += d * xi;
       }
       Pack* yp = reinterpret_cast<Pack*>(Ye + size_t(r) * RV);
       if (gacc) {
@@ -366,7 +370,7 @@ __global__ void __launch_bounds__(256) k_sum_items(const double* __restrict__ pa
 }
 
 // The smallest sectors: a CTA of four warps per slice, each warp every fourth
-// group of slots, partial sums added in warp order through shared memory.  The
+// group of slots, partial sums added in pairs through shared memory.  The
 // slices have one width, so the words are the first loads of the kernel and
 // their targets the second: nothing else is on the path (Heisenberg N=16
 // complex128, launches back to back: 5.4 us with k_hx_list, 4.3 us here).
@@ -418,13 +422,11 @@ __global__ void __launch_bounds__(kListThreads) k_hx_list_small(const __grid_con
     if (T::cplx) s_sum[1][warp][lane] = ai;
     __syncthreads();
     if (warp == 0) {
-      ar = d * xr;
-      ai = d * xi;
-      #pragma unroll
-      for (int k = 0; k < NW; ++k) {
-        ar += s_sum[0][k][lane];
-        if (T::cplx) ai += s_sum[1][k][lane];
-      }
+      static_assert(NW == 4, "four partial sums");
+      ar = (s_sum[0][0][lane] + s_sum[0][1][lane]) + (s_sum[0][2][lane] + s_sum[0][3][lane]);
+      if (T::cplx) ai = (s_sum[1][0][lane] + s_sum[1][1][lane]) + (s_sum[1][2][lane] + s_sum[1][3][lane]);
+      ar += d * xr;
+      if (T::cplx) ai += d * xi;
       if (in) {
         T::st(y, row, ar, ai);
         if (DOT) {
