@@ -38,10 +38,10 @@ constexpr uint32_t kListSmall = 148 * 16;     // slices whose CTAs are all resid
 // Largest table.  The words have to stay in the L2 caches (126 MB, lines read
 // by both dies held twice) from apply to apply.  Where the line lies depends on
 // what runs instead, us per apply with lists / without: exchange tables
-// Heisenberg N=22 c128 (41 MB) 23.3 / 24.6, float32 16.3 / 18.1, N=23 (85 MB)
-// float64 31.5 / 27.0: 64 MB; spin-product 4x3 Hubbard float32 (93 MB) 34.7 /
-// 28.7: 64 MB; two-part tables, whose rows decode slowest, t-J N=17 (72 MB)
-// float64 26 / 38: 96 MB.
+// Heisenberg N=22 c128 (41 MB) 25.6 / 24.0, float64 16.4 / 19.7, N=23 (85 MB)
+// float64 31.5 / 25.9: 64 MB; spin-product 4x3 Hubbard float32 (93 MB) 34.7 /
+// 23.3: 64 MB; two-part tables, whose rows decode slowest, t-J N=17 (72 MB)
+// float64 24.6 / 35.4, c128 47.1 / 44.9: 96 MB.
 constexpr size_t kListMaxBytes = size_t(96) << 20;
 
 struct ListPlan {
