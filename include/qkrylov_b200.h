@@ -102,7 +102,12 @@ int qkrylov_hamiltonian_diagonal_complex_f64(qkrylov_hamiltonian_h h, double* di
 
 /* y = H x on device pointers of `dtype` (any precision handle; real dtypes
  * need a real operator), issued on `stream` (NULL: the library stream)
- * without synchronising.  MatrixFreeHamiltonian::apply(VectorView, VectorView)
+ * without synchronising.  A NULL-stream call (of this and the other functions
+ * with a stream argument) starts after the work the legacy default stream
+ * holds at that moment, except while that stream cannot be named because the
+ * library stream or a blocking stream is in capture.  The default stream does
+ * not wait for the call: before it reads y or writes x again, synchronise or
+ * make it wait for qkrylov_hamiltonian_stream.  MatrixFreeHamiltonian::apply(VectorView, VectorView)
  * (matrix_free_hamiltonian.hpp:38) as a C entry point. */
 int qkrylov_hamiltonian_apply_device(qkrylov_hamiltonian_h h, int dtype, const void* x, void* y, void* stream);
 int qkrylov_hamiltonian_diagonal_device(qkrylov_hamiltonian_h h, int dtype, void* diag, void* stream);

@@ -190,7 +190,7 @@ int qkrylov_hamiltonian_apply_device(qkrylov_hamiltonian_h h, int dtype, const v
   if (!h || !h->op || !x || !y || !valid_dtype(dtype)) return QKRYLOV_ERROR_INVALID_ARG;
   return guarded([&] {
     auto& c = h->op->ctx();
-    if (!stream) h->op->first_use(qk_dtype(dtype));
+    if (!stream) c.after_default_stream();
     const int rc = qkd_apply(h->op->plan(), qk_dtype(dtype), x, y, stream ? cudaStream_t(stream) : c.stream);
     if (rc == QKD_EINVAL) { qkapi::set_error("invalid dtype for this operator or aliased x/y"); return QKRYLOV_ERROR_INVALID_ARG; }
     qkb::qkd_check(rc, "H.x");
@@ -217,6 +217,7 @@ int qkrylov_hamiltonian_apply_range_device(qkrylov_hamiltonian_h h, int dtype, c
   }
   return guarded([&] {
     auto& c = h->op->ctx();
+    if (!stream) c.after_default_stream();
     const int rc = qkd_apply_range(h->op->plan(), qk_dtype(dtype), x, y, row_lo, row_hi,
                                    stream ? cudaStream_t(stream) : c.stream);
     if (rc == QKD_EINVAL) { qkapi::set_error("invalid dtype for this operator or aliased x/y"); return QKRYLOV_ERROR_INVALID_ARG; }
@@ -238,6 +239,7 @@ int qkrylov_b200_apply_block_device(qkrylov_hamiltonian_h h, int dtype, int R, i
   return guarded([&] {
     auto& c = h->op->ctx();
     c.activate();
+    if (!stream) c.after_default_stream();
     const cudaStream_t s = stream ? cudaStream_t(stream) : c.stream;
     qk_plan* plan = const_cast<qk_plan*>(h->op->plan());
     const qk_dtype t = qk_dtype(dtype);
@@ -272,6 +274,7 @@ int qkrylov_hamiltonian_diagonal_device(qkrylov_hamiltonian_h h, int dtype, void
   if (!h || !h->op || !d || !valid_dtype(dtype)) return QKRYLOV_ERROR_INVALID_ARG;
   return guarded([&] {
     auto& c = h->op->ctx();
+    if (!stream) c.after_default_stream();
     const int rc = qkd_diagonal(h->op->plan(), qk_dtype(dtype), d, stream ? cudaStream_t(stream) : c.stream);
     if (rc == QKD_EINVAL) return QKRYLOV_ERROR_INVALID_ARG;
     qkb::qkd_check(rc, "diagonal");
@@ -360,6 +363,7 @@ int qkrylov_b200_multi_dot(int device, int dtype, size_t n, int k, const void* c
     if (!V[j]) return QKRYLOV_ERROR_INVALID_ARG;
   return guarded([&] {
     auto& c = qkb::Context::get(device);
+    c.after_default_stream();
     qkb::PtrArray P(size_t(k), device);
     for (int j = 0; j < k; ++j) P.set(size_t(j), V[j], c.stream);
     qkb::DevVec res(2 * size_t(k), QK_F64, device, false);

@@ -39,15 +39,6 @@ void Operator::apply_dot(qk_dtype t, const void* x, void* y, double* dot_dev) co
   qkd_check(qkd_apply_dot(plan_, c.ws, t, x, y, dot_dev, c.stream), "H.x");
 }
 
-void Operator::first_use(qk_dtype t) const {
-  const unsigned bit = 1u << unsigned(t);
-  if ((used_.load(std::memory_order_relaxed) & bit) || (used_.fetch_or(bit) & bit)) return;
-  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(ctx().stream, &st) == cudaSuccess && st == cudaStreamCaptureStatusNone)
-    cudaStreamSynchronize(cudaStreamLegacy);
-  (void)cudaGetLastError();
-}
-
 void Operator::diagonal(qk_dtype t, void* d) const {
   qkd_check(qkd_diagonal(plan_, t, d, ctx().stream), "diagonal");
 }

@@ -4,7 +4,6 @@
 // (src/hamiltonian/matrix_free_hamiltonian.cpp:12-135), without the CSR.
 #pragma once
 
-#include <atomic>
 #include <memory>
 #include <vector>
 
@@ -36,15 +35,7 @@ class Operator {
   void apply_dot(qk_dtype t, const void* x, void* y, double* dot_dev) const;
   void diagonal(qk_dtype t, void* d) const;
 
-  // Called before an apply on caller memory that names no stream.  The first
-  // one of a vector type waits for the default stream, where that memory was
-  // usually just filled: the library stream does not wait for it, and a small
-  // sector's kernel reads x 1 us after its launch.  Ordering further work is
-  // the caller's part (an event per call would cost half of such an apply).
-  void first_use(qk_dtype t) const;
-
  private:
-  mutable std::atomic<unsigned> used_{0};  // vector types seen by first_use
   std::shared_ptr<const SectorTable> basis_;
   CompiledOp op_;
   qk_plan* plan_ = nullptr;

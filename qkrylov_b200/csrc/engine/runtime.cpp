@@ -27,6 +27,7 @@ Context::Context(int dev) : device(dev) {
   if (dev < 0 || dev >= n) throw DeviceError("qkrylov_b200: no CUDA device " + std::to_string(dev));
   cuda_check(cudaSetDevice(dev), "cudaSetDevice");
   cuda_check(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking), "cudaStreamCreate");
+  cuda_check(cudaEventCreateWithFlags(&def_ev, cudaEventDisableTiming), "cudaEventCreate");
   qkd_check(qkd_workspace_create(dev, &ws), "workspace");
   cuda_check(cudaMallocHost(&host, sizeof(double) * kHost), "cudaMallocHost");
   // Solver vectors come from the device's stream-ordered pool, which keeps
@@ -86,6 +87,20 @@ const double* Context::fetch2(const double* a, int na, const double* b, int nb) 
 }
 
 void Context::sync() { cuda_check(cudaStreamSynchronize(stream), "stream sync"); }
+
+void Context::after_default_stream() const {
+  cudaStreamCaptureStatus own = cudaStreamCaptureStatusNone, def = cudaStreamCaptureStatusNone;
+  cuda_check(cudaStreamIsCapturing(stream, &own), "stream");
+  if (own != cudaStreamCaptureStatusNone) return;
+  // an error here says that a blocking stream is in capture (and leaves it intact)
+  if (cudaStreamIsCapturing(cudaStreamLegacy, &def) != cudaSuccess) {
+    (void)cudaGetLastError();
+    return;
+  }
+  // threads may share the event: a later record covers an earlier one's work
+  cuda_check(cudaEventRecord(def_ev, cudaStreamLegacy), "default stream");
+  cuda_check(cudaStreamWaitEvent(stream, def_ev, 0), "default stream");
+}
 
 DevVec::DevVec(size_t n, qk_dtype t, int device, bool zero) : n_(n), t_(t), dev_(device) {
   if (n == 0) return;

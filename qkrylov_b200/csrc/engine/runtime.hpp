@@ -31,6 +31,7 @@ class Context {
   qk_workspace* ws = nullptr;
   double* host = nullptr;  // pinned, kHost doubles
   static constexpr int kHost = 4096;
+  cudaEvent_t def_ev = nullptr;  // after_default_stream
 
   double* dres(int i = 0) const { return qkd_workspace_results(ws) + i; }
   // Copy n doubles from device memory to the pinned buffer and wait.
@@ -39,6 +40,14 @@ class Context {
   const double* fetch2(const double* a, int na, const double* b, int nb);
   void sync();
   void activate() const;
+  // Makes the library stream wait for the work the default stream holds now.
+  // Called by every entry point that runs on caller memory without a stream of
+  // the caller's: that memory was usually just written on the default stream,
+  // which a non-blocking stream does not wait for, and a small sector's kernel
+  // reads it 1 us after its launch.  An event pair: 0.3 us of host time, 0.6 us
+  // of a call waited for by itself.  No-op while the library stream or any
+  // blocking stream is in capture, where the default stream cannot be named.
+  void after_default_stream() const;
   // Stream-ordered device memory on this context's stream (the device's
   // default pool, which keeps freed blocks); release() is ordered after all
   // work already issued on the stream.

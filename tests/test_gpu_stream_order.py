@@ -1,0 +1,112 @@
+"""Ordering of device-pointer calls with other streams: every call without a
+stream starts after what the default stream holds (not only the first of its
+vector type), for each entry point, and leaves a capture on another stream
+alone."""
+import ctypes
+
+import numpy as np
+import pytest
+
+import oracle as O
+import qkrylov_b200 as qk
+from test_gpu_hx import ham, rel
+
+pytestmark = pytest.mark.gpu
+torch = pytest.importorskip("torch")
+
+N, SEC, TERMS = 14, dict(use_sz=1, sz2=0), O.heisenberg_chain(14)
+
+
+@pytest.fixture(scope="module")
+def case():
+    H = ham("spin", N, SEC, TERMS)
+    rng = np.random.default_rng(1)
+    x = rng.standard_normal(H.dimension)
+    return H, x, O.port().hamiltonian("spin", N, SEC, TERMS).apply(x.astype(np.complex128)).real
+
+
+def busy():
+    """Some milliseconds of work on the current stream."""
+    a = torch.ones(4096, 4096, device="cuda")
+    for _ in range(8):
+        a = a @ a * 1e-4
+    return a
+
+
+@pytest.mark.parametrize("entry", ["apply", "range", "block", "diagonal", "multi_dot"])
+def test_calls_without_a_stream_follow_the_default_stream(case, entry):
+    H, xh, want = case
+    src = torch.tensor(xh, device="cuda")
+    D = H.dimension
+    ptr = lambda t: ctypes.c_void_p(t.data_ptr())
+    if entry == "block":
+        X, Y = (torch.zeros(D, 32, dtype=torch.float64, device="cuda") for _ in range(2))
+        H.apply_block_device(X.data_ptr(), Y.data_ptr(), qk.DTYPE_F64, 32)  # tunes
+    for _ in range(4):
+        shape = (D, 32) if entry == "block" else (D,)
+        x = torch.full(shape, 9.0, dtype=torch.float64, device="cuda")
+        y = torch.full(shape, 9.0, dtype=torch.float64, device="cuda")
+        torch.cuda.synchronize()
+        keep = busy()
+        x.copy_(src[:, None].expand(D, 32) if entry == "block" else src)
+        y.fill_(float("nan"))
+        if entry == "apply":
+            H.apply_device(x.data_ptr(), y.data_ptr(), qk.DTYPE_F64)
+        elif entry == "range":
+            assert qk.lib().qkrylov_hamiltonian_apply_range_device(H._h, qk.DTYPE_F64, ptr(x), ptr(y), 0, D, None) == 0
+        elif entry == "block":
+            H.apply_block_device(x.data_ptr(), y.data_ptr(), qk.DTYPE_F64, 32)
+        elif entry == "diagonal":
+            assert qk.lib().qkrylov_hamiltonian_diagonal_device(H._h, qk.DTYPE_F64, ptr(y), None) == 0
+        else:
+            out = np.zeros(2)
+            V = (ctypes.c_void_p * 1)(x.data_ptr())
+            assert qk.lib().qkrylov_b200_multi_dot(0, qk.DTYPE_F64, D, 1, V, ptr(x), out.ctypes.data) == 0
+            assert abs(out[0] - xh @ xh) < 1e-12 * (xh @ xh)
+        torch.cuda.synchronize()
+        del keep
+        got = y.cpu().numpy()
+        if entry == "diagonal":
+            assert np.array_equal(got, H.diagonal().real)
+        elif entry == "block":
+            assert rel(got, np.repeat(want[:, None], 32, axis=1)) < 1e-13
+        elif entry != "multi_dot":
+            assert rel(got, want) < 1e-13
+
+
+@pytest.mark.parametrize("mode", ["global", "thread_local", "relaxed"])
+def test_a_capture_on_another_stream_survives(case, mode):
+    """Calls without a stream, on an operator that has been applied before and
+    on a new vector type, while another stream is in capture."""
+    H, xh, want = case
+    x = torch.tensor(xh, device="cuda")
+    x32, y32 = x.float(), torch.empty(len(xh), dtype=torch.float32, device="cuda")
+    y, z = torch.empty_like(x), torch.zeros(8, device="cuda")
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, capture_error_mode=mode):
+        z.add_(1.0)
+        H.apply_device(x.data_ptr(), y.data_ptr(), qk.DTYPE_F64)
+        H.apply_device(x32.data_ptr(), y32.data_ptr(), qk.DTYPE_F32)
+    g.replay()
+    torch.cuda.synchronize()
+    assert (z == 1.0).all() and rel(y.cpu().numpy(), want) < 1e-13 and rel(y32.cpu().numpy(), want) < 2e-6
+    g.reset()
+
+
+def test_a_capture_on_a_blocking_stream_survives(case):
+    """The default stream cannot be named while a stream that synchronises with
+    it is in capture: the call goes ahead and the capture stays valid."""
+    H, xh, want = case
+    x = torch.tensor(xh, device="cuda")
+    y = torch.empty_like(x)
+    torch.cuda.synchronize()
+    rt = ctypes.CDLL(f"libcudart.so.{torch.version.cuda.split('.')[0]}")
+    s, g = ctypes.c_void_p(), ctypes.c_void_p()
+    assert rt.cudaStreamCreate(ctypes.byref(s)) == 0
+    assert rt.cudaStreamBeginCapture(s, 1) == 0
+    H.apply_device(x.data_ptr(), y.data_ptr(), qk.DTYPE_F64)
+    assert rt.cudaStreamEndCapture(s, ctypes.byref(g)) == 0 and g.value
+    assert rt.cudaGraphDestroy(g) == 0 and rt.cudaStreamDestroy(s) == 0
+    torch.cuda.synchronize()
+    assert rel(y.cpu().numpy(), want) < 1e-13
