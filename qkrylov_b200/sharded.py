@@ -53,6 +53,8 @@ def gpu_apply_rows(H, dtype_code: int):
         y = state.get("y")
         if y is None or y.shape != x_full.shape or y.dtype != x_full.dtype:
             y = state["y"] = torch.empty_like(x_full)
+        # x_full was made, and y's last rows are read, on the caller's stream
+        torch.cuda.ExternalStream(H.stream).wait_stream(torch.cuda.current_stream())
         rc = lib().qkrylov_hamiltonian_apply_range_device(H._h, dtype_code, ctypes.c_void_p(x_full.data_ptr()),
                                                           ctypes.c_void_p(y.data_ptr()), int(lo), int(hi), None)
         if rc != 0:

@@ -9,6 +9,7 @@ import pytest
 
 import oracle as O
 import qkrylov_b200 as qk
+from qkrylov_b200 import sharded
 from test_gpu_hx import ham, rel
 
 pytestmark = pytest.mark.gpu
@@ -72,6 +73,25 @@ def test_calls_without_a_stream_follow_the_default_stream(case, entry):
             assert rel(got, np.repeat(want[:, None], 32, axis=1)) < 1e-13
         elif entry != "multi_dot":
             assert rel(got, want) < 1e-13
+
+
+def test_range_hook_follows_the_current_stream(case):
+    """The sharded Lanczos' range apply on a stream other than the default one."""
+    H, xh, want = case
+    src = torch.tensor(xh, device="cuda")
+    apply_rows = sharded.gpu_apply_rows(H, qk.DTYPE_F64)
+    x = torch.empty_like(src)
+    torch.cuda.synchronize()
+    got = []
+    with torch.cuda.stream(torch.cuda.Stream()):
+        for k in (1.0, 2.0, 3.0):
+            keep = busy()
+            torch.mul(src, k, out=x)
+            got.append(apply_rows(x, 0, H.dimension).clone())
+    torch.cuda.synchronize()
+    del keep
+    for k, y in zip((1.0, 2.0, 3.0), got):
+        assert rel(y.cpu().numpy(), k * want) < 1e-13, k
 
 
 @pytest.mark.parametrize("mode", ["global", "thread_local", "relaxed"])
