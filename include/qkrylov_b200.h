@@ -107,7 +107,13 @@ int qkrylov_hamiltonian_diagonal_complex_f64(qkrylov_hamiltonian_h h, double* di
  * holds at that moment, except while that stream cannot be named because the
  * library stream or a blocking stream is in capture.  The default stream does
  * not wait for the call: before it reads y or writes x again, synchronise or
- * make it wait for qkrylov_hamiltonian_stream.  MatrixFreeHamiltonian::apply(VectorView, VectorView)
+ * make it wait for qkrylov_hamiltonian_stream.
+ * Calls on one handle may come from several streams and threads: a call that
+ * uses the handle's own scratch waits on its stream for the handle's previous
+ * call.  Not covered: a replay of a captured call (run none while other calls on
+ * that handle are on the GPU), and results that go through the device's one
+ * set of reduction buffers (dots_out of the block apply, the solvers), of which
+ * one call per device may run at a time.  MatrixFreeHamiltonian::apply(VectorView, VectorView)
  * (matrix_free_hamiltonian.hpp:38) as a C entry point. */
 int qkrylov_hamiltonian_apply_device(qkrylov_hamiltonian_h h, int dtype, const void* x, void* y, void* stream);
 int qkrylov_hamiltonian_diagonal_device(qkrylov_hamiltonian_h h, int dtype, void* diag, void* stream);

@@ -6,10 +6,10 @@ Operator::Operator(Family site_family, std::shared_ptr<const SectorTable> basis,
                    const std::vector<TermIn>& terms, int device, bool transient)
     : basis_(std::move(basis)), device_(device) {
   op_ = compile_opsum(site_family, *basis_, terms);
-  Context::get(device_);
   static_assert(sizeof(CTerm) == sizeof(qk_term_t), "term layout");
   static_assert(sizeof(CGroup) == sizeof(qk_group_t), "group layout");
   qk_plan_desc d{};
+  d.home = Context::get(device_).stream;
   d.nbits = basis_->nbits;
   d.L = basis_->L;
   d.dim = basis_->dim;

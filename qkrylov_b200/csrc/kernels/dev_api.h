@@ -45,6 +45,7 @@ typedef struct {
   int has_diag, all_real;
   int pair_sites;  /* 1: two bits per site, up-spin at the even bit (Hubbard, t-J) */
   int transient;   /* 1: applied once or twice and destroyed; no row lists are built */
+  cudaStream_t home;  /* the stream most calls run on; outlives the plan */
 } qk_plan_desc;
 
 typedef struct qk_plan qk_plan;

@@ -10,11 +10,11 @@
 // consecutive addresses (coalesced); terms that flip low bits stay inside
 // the block, which L1 holds.  Each thread writes only its own y[row].
 #include <algorithm>
-#include <mutex>
 #include <vector>
 
 #include "reduce.cuh"
 #include "hx_terms.cuh"
+#include "stream_order.hpp"
 #include "../engine/sector.hpp"
 
 namespace qkd {
@@ -62,6 +62,7 @@ static bool g_die_queues = true;  // per-die work queues
 static bool g_list_path = true;  // the row lists of small sectors, the flips of complete bases
 
 struct qk_plan {
+  qkd::StreamOrder* order = nullptr;  // calls on different streams
   qkd::SpinHandle* spin = nullptr;
   qkd::PairHandle* pair = nullptr;  // spin-product path (Hubbard-type operators), or null
   qkd::ListHandle* list = nullptr;  // row lists (small sectors of real operators), or null
@@ -461,19 +462,20 @@ int qkd_plan_create(const qk_plan_desc* d, int device, qk_plan** out) {
   if (tiles.size() > 0xFFFFFFFFull) return QKD_EINVAL;
   auto* p = new qk_plan{};
   p->device = device;
+  p->order = new qkd::StreamOrder(d->home);
   p->nbits = d->nbits; p->L = d->L; p->dim = d->dim;
   p->lmask = (d->L >= 64) ? ~0ULL : ((1ULL << d->L) - 1);
   p->nterms = d->nterms; p->ngroups = d->ngroups; p->ntiles = uint32_t(tiles.size());
   p->has_diag = d->has_diag; p->all_real = d->all_real;
   p->smem = size_t(d->nterms) * sizeof(qk_term_t) + size_t(d->ngroups) * sizeof(qk_group_t);
-  if (p->smem > 200 * 1024) { delete p; return QKD_EINVAL; }
+  if (p->smem > 200 * 1024) { qkd_plan_destroy(p); return QKD_EINVAL; }
   auto up = [&](void** dst, const void* src, size_t bytes) -> bool {
     if (bytes == 0) { *dst = nullptr; return true; }
     if (cudaMalloc(dst, bytes) != cudaSuccess) return false;
     p->bytes += bytes;
     return cudaMemcpy(*dst, src, bytes, cudaMemcpyHostToDevice) == cudaSuccess;
   };
-  bool ok = up((void**)&p->A, d->A, d->nA * 8) && up((void**)&p->B, d->B, d->nB * 4) &&
+  bool ok = p->order->init() && up((void**)&p->A, d->A, d->nA * 8) && up((void**)&p->B, d->B, d->nB * 4) &&
             up((void**)&p->llist, d->llist, d->nllist * 4) &&
             up((void**)&p->terms, d->terms, size_t(d->nterms) * sizeof(qk_term_t)) &&
             up((void**)&p->groups, d->groups, size_t(d->ngroups) * sizeof(qk_group_t)) &&
@@ -555,6 +557,7 @@ int qkd_plan_destroy(qk_plan* p) {
   cudaFree(p->list_diag);
   cudaFree(p->A); cudaFree(p->B); cudaFree(p->llist);
   cudaFree(p->terms); cudaFree(p->groups); cudaFree(p->tiles);
+  delete p->order;
   delete p;
   return QKD_OK;
 }
@@ -569,6 +572,7 @@ int qkd_apply(const qk_plan* p, qk_dtype t, const void* x, void* y, cudaStream_t
   if (!qk_dtype_complex(t) && !p->all_real) return QKD_EINVAL;
   if (p->flip && g_kernel_policy == 0 && g_list_path) return qkd::flip_apply(p->flip, t, x, y, s, nullptr, nullptr, 0, p->dim);
   if (p->list && g_kernel_policy == 0 && g_list_path) return qkd::list_apply(p->list, t, x, y, s, nullptr, nullptr, 0, p->dim);
+  StreamOrder::Use use(*p->order, s);
   if (p->pair && g_kernel_policy == 0 && g_pair_path) {
     const int rc = qkd::pair_apply(p->pair, t, x, y, s, nullptr, nullptr);
     if (rc != QKD_EINVAL) return rc;
@@ -590,6 +594,7 @@ int qkd_apply_range(const qk_plan* p, qk_dtype t, const void* x, void* y, uint64
     return qkd::flip_apply(p->flip, t, x, y, s, nullptr, nullptr, row_lo, row_hi);
   if (p->list && g_kernel_policy == 0 && g_list_path)
     return qkd::list_apply(p->list, t, x, y, s, nullptr, nullptr, row_lo, row_hi);
+  StreamOrder::Use use(*p->order, s);
   if (p->spin && g_kernel_policy == 0) {
     const int rc = qkd::spin_apply_range(p->spin, t, x, y, s, row_lo, row_hi);
     if (rc != QKD_EINVAL) return rc;
@@ -607,6 +612,7 @@ int qkd_apply_dot(const qk_plan* p, qk_workspace* w, qk_dtype t, const void* x, 
   if (!qk_dtype_complex(t) && !p->all_real) return QKD_EINVAL;
   if (p->flip && g_kernel_policy == 0 && g_list_path) return qkd::flip_apply(p->flip, t, x, y, s, w, dot_out, 0, p->dim);
   if (p->list && g_kernel_policy == 0 && g_list_path) return qkd::list_apply(p->list, t, x, y, s, w, dot_out, 0, p->dim);
+  StreamOrder::Use use(*p->order, s);
   if (p->pair && g_kernel_policy == 0 && g_pair_path) {
     const int rc = qkd::pair_apply(p->pair, t, x, y, s, w, dot_out);
     if (rc != QKD_EINVAL) return rc;
@@ -650,6 +656,7 @@ static int apply_rows_shape(const qk_plan* p, qk_workspace* w, qk_dtype t, int R
 int qkd_apply_rows(const qk_plan* p, qk_workspace* w, qk_dtype t, int R, int lanes_per_row, const void* X,
                    void* Y, const void* diag, double* dots, cudaStream_t s) {
   if (!p || r_index(R) < 0 || t < QK_C128 || t > QK_F32) return QKD_EINVAL;
+  StreamOrder::Use use(*p->order, s);
   const int lpr = lanes_per_row ? lanes_per_row : (p->rows_lpr[t][r_index(R)] ? p->rows_lpr[t][r_index(R)] : 32);
   const int tilec = lanes_per_row ? 0 : p->rows_tile[t][r_index(R)];
   const int list = lanes_per_row ? 0 : p->rows_list[t][r_index(R)];
@@ -663,6 +670,7 @@ int qkd_apply_rows(const qk_plan* p, qk_workspace* w, qk_dtype t, int R, int lan
 int qkd_apply_rows_acc(const qk_plan* p, qk_workspace* w, qk_dtype t, int R, int lanes_per_row, const void* X,
                        void* Y, const double* g, double* dots, cudaStream_t s) {
   if (!p || !g || r_index(R) < 0 || t < QK_C128 || t > QK_F32) return QKD_EINVAL;
+  StreamOrder::Use use(*p->order, s);
   const int lpr = lanes_per_row ? lanes_per_row : (p->rows_lpr[t][r_index(R)] ? p->rows_lpr[t][r_index(R)] : 32);
   const int tilec = lanes_per_row ? 0 : p->rows_tile[t][r_index(R)];
   const int list = lanes_per_row ? 0 : p->rows_list[t][r_index(R)];
@@ -693,6 +701,7 @@ int qkd_rows_timings(const qk_plan* p, qk_dtype t, int R, float* ms9) {
 static int tune_rows(qk_plan* p, qk_workspace* w, qk_dtype t, int R, const void* X, void* Y, const void* diag,
                      const double* g, cudaStream_t s, int* chosen) {
   if (!p || !w || r_index(R) < 0 || t < QK_C128 || t > QK_F32) return QKD_EINVAL;
+  StreamOrder::Use use(*p->order, s);  // held while tuning: two threads may tune the same plan
   const int lprs[3] = {32, 16, 8};
   const int ntile = (p->spin && g_kernel_policy == 0) ? 3 : 1;
   cudaEvent_t e0, e1;
@@ -730,15 +739,12 @@ static int tune_rows(qk_plan* p, qk_workspace* w, qk_dtype t, int R, const void*
   // the packed lists (4 bytes per target against R elements of its row; at
   // most half a block vector) against the best of those shapes
   int pick_list = 0;
-  static std::mutex build_mu;  // two threads may tune the same plan
-  std::unique_lock<std::mutex> build(build_mu);
   const size_t list_max = size_t(p->dim) * R * qk_dtype_size(t) / 2;
   if (p->all_real && !p->block_list && g_kernel_policy == 0 && g_list_path && list_max > p->block_list_tried) {
     p->block_list_tried = list_max;
     if (const double* dv = real_diag(p); dv || !p->has_diag)
       p->block_list = block_list_create(dev(p), p->dim, dv, list_max, &p->bytes);
   }
-  build.unlock();
   if (p->block_list && g_kernel_policy == 0 && g_list_path) {
     cudaEvent_t s0, s1;
     if (cudaEventCreate(&s0) != cudaSuccess || cudaEventCreate(&s1) != cudaSuccess) return QKD_ECUDA;

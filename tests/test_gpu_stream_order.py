@@ -130,3 +130,55 @@ def test_a_capture_on_a_blocking_stream_survives(case):
     assert rt.cudaGraphDestroy(g) == 0 and rt.cudaStreamDestroy(s) == 0
     torch.cuda.synchronize()
     assert rel(y.cpu().numpy(), want) < 1e-13
+
+
+@pytest.mark.parametrize("kind,n,sec,terms", [
+    ("spin", 24, dict(use_sz=1, sz2=0), O.heisenberg_chain(24)),                    # grouped rows: work queues
+    ("tj", 18, dict(use_nup=1, nup=8, use_ndn=1, ndn=8), O.tj_chain(18)),           # the same, two-part
+    ("hubbard", 13, dict(use_nup=1, nup=6, use_ndn=1, ndn=7), O.hubbard_square(13, 1)),  # product-ordered scratch
+])
+def test_applies_of_one_operator_on_several_streams(kind, n, sec, terms):
+    """Sectors above the row lists' size, whose kernels keep queues or scratch
+    in the operator: applies issued in turn on three streams without waiting."""
+    H = ham(kind, n, sec, terms)
+    g = torch.Generator("cuda").manual_seed(n)
+    xs = [torch.randn(H.dimension, dtype=torch.float64, device="cuda", generator=g) for _ in range(6)]
+    want = [torch.empty_like(x) for x in xs]
+    ys = [torch.full_like(x, float("nan")) for x in xs]
+    for x, w in zip(xs, want):
+        H.apply_device(x.data_ptr(), w.data_ptr(), qk.DTYPE_F64)
+        torch.cuda.synchronize()
+    streams = [0, torch.cuda.Stream().cuda_stream, torch.cuda.Stream().cuda_stream]
+    for rep in range(3):
+        for k, (x, y) in enumerate(zip(xs, ys)):
+            H.apply_device(x.data_ptr(), y.data_ptr(), qk.DTYPE_F64, stream=streams[(k + rep) % 3])
+        torch.cuda.synchronize()
+        assert all(torch.equal(y, w) for y, w in zip(ys, want)), rep
+        for y in ys:
+            y.fill_(float("nan"))
+        torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("kind,n,sec,terms", [
+    ("tj", 14, dict(use_nup=1, nup=6, use_ndn=1, ndn=6), O.tj_chain(14)),
+    ("spin", 16, {}, [(0.5, [("Sz", i), ("Sz", (i + 1) % 16)]) for i in range(16)] + [(0.7, [("Sx", i)]) for i in range(16)]),
+])
+def test_block_applies_of_one_operator_on_several_streams(kind, n, sec, terms):
+    H = ham(kind, n, sec, terms)
+    g = torch.Generator("cuda").manual_seed(n)
+    Xs = [torch.randn(H.dimension, 64, dtype=torch.float64, device="cuda", generator=g) for _ in range(4)]
+    want = [torch.empty_like(X) for X in Xs]
+    Ys = [torch.full_like(X, float("nan")) for X in Xs]
+    torch.cuda.synchronize()
+    for X, W in zip(Xs, want):
+        H.apply_block_device(X.data_ptr(), W.data_ptr(), qk.DTYPE_F64, 64)
+        torch.cuda.synchronize()
+    streams = [torch.cuda.Stream().cuda_stream, 0, torch.cuda.Stream().cuda_stream]
+    for rep in range(3):
+        for k, (X, Y) in enumerate(zip(Xs, Ys)):
+            H.apply_block_device(X.data_ptr(), Y.data_ptr(), qk.DTYPE_F64, 64, stream=streams[(k + rep) % 3])
+        torch.cuda.synchronize()
+        assert all(torch.equal(Y, W) for Y, W in zip(Ys, want)), rep
+        for Y in Ys:
+            Y.fill_(float("nan"))
+        torch.cuda.synchronize()
