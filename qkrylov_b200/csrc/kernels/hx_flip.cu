@@ -125,8 +125,12 @@ k_hx_flip(const FlipPlan p, const void* __restrict__ x, void* __restrict__ y, do
     #pragma unroll
     for (int k = 0; k < K; ++k) {
       const uint32_t row = r0 + k * NT;
-      ar[k] = ar[k] + hr[k] + R(d[k]) * xr[k];
-      if (T::cplx) ai[k] = ai[k] + hi[k] + R(d[k]) * xi[k];
+      ar[k] += hr[k];
+      if (T::cplx) ai[k] += hi[k];
+      if (p.diag) {  // none is not a zero one: an infinite x must not become a NaN
+        ar[k] += R(d[k]) * xr[k];
+        if (T::cplx) ai[k] += R(d[k]) * xi[k];
+      }
       if (row >= p.row_lo && row < p.row_hi) {
         T::st(y, row, ar[k], ai[k]);
         if (DOT) {

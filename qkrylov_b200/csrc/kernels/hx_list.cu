@@ -280,13 +280,16 @@ k_hx_block_list(const __grid_constant__ BlockListPlan p, const void* __restrict_
             }
           }
       }
-      // the diagonal last: the hops are rounded against their own sum
-      #pragma unroll
-      for (int v = 0; v < VPL; ++v) {
-        R xr, xi;
-        unpk<DT>(own.v[v], xr, xi);
-        ar[v] += d * xr;
-        if (T::cplx) ai[v] += d * xi;
+      // the diagonal last: the hops are rounded against their own sum; none is
+      // not a zero one, which would turn an infinite x into a NaN
+      if (p.diag) {
+        #pragma unroll
+        for (int v = 0; v < VPL; ++v) {
+          R xr, xi;
+          unpk<DT>(own.v[v], xr, xi);
+          ar[v] += d * xr;
+          if (T::cplx) ai[v] += d * xi;
+        }
       }
       Pack* yp = reinterpret_cast<Pack*>(Ye + size_t(r) * RV);
       if (gacc) {
@@ -425,8 +428,10 @@ __global__ void __launch_bounds__(kListThreads) k_hx_list_small(const __grid_con
       static_assert(NW == 4, "four partial sums");
       ar = (s_sum[0][0][lane] + s_sum[0][1][lane]) + (s_sum[0][2][lane] + s_sum[0][3][lane]);
       if (T::cplx) ai = (s_sum[1][0][lane] + s_sum[1][1][lane]) + (s_sum[1][2][lane] + s_sum[1][3][lane]);
-      ar += d * xr;
-      if (T::cplx) ai += d * xi;
+      if (p.diag) {
+        ar += d * xr;
+        if (T::cplx) ai += d * xi;
+      }
       if (in) {
         T::st(y, row, ar, ai);
         if (DOT) {
@@ -492,8 +497,10 @@ __global__ void __launch_bounds__(kListThreads) k_hx_list(const __grid_constant_
           if (T::cplx) ai += c * vi[u];
         }
     }
-    ar += d * xr;
-    if (T::cplx) ai += d * xi;
+    if (p.diag) {
+      ar += d * xr;
+      if (T::cplx) ai += d * xi;
+    }
     if (in) T::st(y, row, ar, ai);
     if (DOT) {
       dr += double(xr) * double(ar) + double(xi) * double(ai);

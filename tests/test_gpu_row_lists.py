@@ -92,3 +92,36 @@ def test_tuned_block_apply_on_small_tiles(kind, N, sec, terms, R):
         got = dots[0][0::2] + 1j * dots[0][1::2]
         assert np.abs(got - d).max() <= 10 * tol * np.abs(d).max() + 1e-300, code
         assert np.array_equal(dots[0], dots[1]), code
+
+
+@pytest.mark.parametrize("kind,N,sec,terms", [
+    ("spin", 9, {}, [(0.7, [("Sx", i)]) for i in range(9)]),                        # one warp tile per slice
+    ("fermion", 20, dict(use_n=1, n=10), [(-1.0, [(a, (i + 1) % 20), (b, i)]) for i in range(20)
+                                          for a, b in (("C", "Cdag"), ("Cdag", "C"))]),  # whole slices
+    ("spin", 13, {}, [(0.7, [("Sx", i)]) for i in range(13)]),                      # flips
+])
+def test_no_diagonal_leaves_infinities_to_the_rows_they_couple_to(kind, N, sec, terms):
+    """An operator without a diagonal does not touch a row's own element, as the
+    generic kernel does not: an infinite one stays out of that row."""
+    H = ham(kind, N, sec, terms)
+    for code, tdt in [(qk.DTYPE_F64, torch.float64), (qk.DTYPE_F32, torch.float32), (qk.DTYPE_C128, torch.complex128)]:
+        x = torch.ones(H.dimension, dtype=tdt, device="cuda")
+        j = H.dimension // 3
+        x[j] = float("inf")
+        got = {}
+        try:
+            for pol in ("auto", "generic"):
+                qk.set_kernel_policy(pol)
+                y = torch.empty_like(x)
+                H.apply_device(x.data_ptr(), y.data_ptr(), code)
+                torch.cuda.synchronize()
+                got[pol] = torch.isfinite(torch.view_as_real(y).sum(-1) if tdt.is_complex else y)
+        finally:
+            qk.set_kernel_policy("auto")
+        assert got["auto"][j] and torch.equal(got["auto"], got["generic"]), (kind, code)
+    X = torch.ones(H.dimension, 32, dtype=torch.float64, device="cuda")
+    X[j] = float("inf")
+    Y = torch.empty_like(X)
+    H.apply_block_device(X.data_ptr(), Y.data_ptr(), qk.DTYPE_F64, 32)
+    torch.cuda.synchronize()
+    assert torch.equal(torch.isfinite(Y), got["generic"][:, None].expand(-1, 32))
