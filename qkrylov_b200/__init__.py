@@ -1000,8 +1000,10 @@ def set_kernel_policy(policy: str):
     tables, per-die work queues on a two-die GPU), 'generic' (the term-walk
     kernel only), 'no-die-queues' (auto with one grid-stride order) or
     'no-spin-product' (the row kernels: Hubbard-type operators on the
-    two-part one, small sectors without their row lists), for comparisons."""
-    codes = {"auto": 0, "generic": 1, "no-die-queues": 2, "no-spin-product": 3}
+    two-part one, small sectors without their row lists), 'packed-shapes'
+    (auto, and an explicit lanes_per_row of the block apply names a shape of
+    its packed lists instead of the row kernels), for comparisons."""
+    codes = {"auto": 0, "generic": 1, "no-die-queues": 2, "no-spin-product": 3, "packed-shapes": 4}
     _check(lib().qkrylov_b200_set_kernel_policy(codes[policy]), "set_kernel_policy")
 
 

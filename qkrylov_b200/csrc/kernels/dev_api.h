@@ -60,7 +60,8 @@ size_t qkd_plan_device_bytes(const qk_plan* p);
 /* 0: use specialised kernels where the operator qualifies (default);
  * 1: generic kernel only; 2: as 0 without the per-die work queues of the
  * row kernel; 3: the row kernels without the spin-product path of
- * Hubbard-type operators and without the row lists of small sectors (for
+ * Hubbard-type operators and without the row lists of small sectors; 4: as
+ * 0 with explicit shapes of the block apply on its packed lists (for
  * comparisons). */
 int qkd_set_kernel_policy(int policy);
 /* Dies of the current device as measured by the row kernels' topology probe

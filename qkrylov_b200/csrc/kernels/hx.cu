@@ -29,7 +29,7 @@ int pair_apply(const PairHandle* h, qk_dtype t, const void* x, void* y, cudaStre
                double* dot_out);
 struct BlockListHandle;
 BlockListHandle* block_list_create(const DevPlan& p, uint64_t dim, const double* diag, size_t max_bytes,
-                                   size_t* dev_bytes);
+                                   size_t* list_bytes, size_t* dev_bytes);
 void block_list_destroy(BlockListHandle* h);
 int block_list_apply(const BlockListHandle* h, qk_dtype t, int R, int lpr, bool queues, const void* X, void* Y,
                      double* dots, cudaStream_t s, const double* gacc);
@@ -60,6 +60,7 @@ static int g_kernel_policy = 0;  // 0: specialised kernels where eligible, 1: ge
 static bool g_pair_path = true;  // the spin-product path of Hubbard-type operators
 static bool g_die_queues = true;  // per-die work queues
 static bool g_list_path = true;  // the row lists of small sectors, the flips of complete bases
+static bool g_list_shapes = false;  // explicit shapes of the block apply on its packed lists
 
 struct qk_plan {
   qkd::StreamOrder* order = nullptr;  // calls on different streams
@@ -83,8 +84,8 @@ struct qk_plan {
   int rows_lpr[4][3];   // autotuned lanes per row of the block apply, by dtype and R = 32, 64, 128
   int rows_tile[4][3];  // autotuned tile shape of the block apply (row kernels: 256 / 128 / 512 rows)
   int rows_list[4][3];  // lanes per row of the packed-list block kernel where it was the fastest, else 0
-  size_t block_list_tried;  // largest size the packed lists were refused
-  qkd::BlockListHandle* block_list;  // packed lists of the block apply, built by the tuner
+  size_t block_list_bytes;  // size of the packed lists once counted (~0: they cannot be built), 0 before
+  qkd::BlockListHandle* block_list;  // packed lists of the block apply, built on first use
   float rows_ms[4][3][9];  // the tuner's fastest launch (ms) per lanes per row (32/16/8) x tile code; 0: untimed
   double* diag_re;     // real diagonal (generic-kernel operators with a real diagonal), else null
 };
@@ -437,6 +438,44 @@ void make_lists(qk_plan* p, const qk_plan_desc* d) {
   }
 }
 
+// Whether the block apply of R vectors of type t runs on packed lists where
+// they can be built.  The rule is sizes and the operator's form alone, so that a
+// program's results depend neither on timings nor on what was applied before.
+// The words are 4 bytes per target against R elements of its row: at most half
+// a block vector.  us per apply, best row shape / best list shape:
+//   rows up to 512 bytes: t-J N=10, 64 complex64 14.2 / 12.1, Heisenberg N=12, 64
+//     complex64 11.5 / 11.8 (the worst), Hubbard 4x3, 32 float64 several times
+//   rows of 1024 bytes, which leave one list shape (32 bytes per lane), from 3 MB
+//     of block vector: t-J N=10 (3.2 MB) complex128 17.9 / 14.5; J1-J2 N=10 (0.3 MB)
+//     12.4 / 15.2, Heisenberg N=12 (0.9 MB) 13.6 / 14.4
+//   wider rows: the lane would hold more than 32 bytes
+//   flips of a complete basis, whose row kernels decode next to nothing: double
+//     precision up to 256 bytes (Ising N=14, 32 float64 15.5 / 13.9; N=18, 64
+//     float64 220 / 232), single up to 512 (N=14, 128 float32 27.8 / 21.5), 1024
+//     from 2^20 rows (N=20, 64 complex128 2160 / 1836; N=18, 128 float64 439 / 471)
+bool block_list_pays(const qk_plan* p, qk_dtype t, int R) {
+  const size_t row = size_t(R) * qk_dtype_size(t);
+  if (row > 1024) return false;
+  if (p->flip) {
+    if (row == 1024) return p->dim >= (1ull << 20);
+    return row <= (t == QK_C64 || t == QK_F32 ? 512 : 256);
+  }
+  return row < 1024 || p->dim * row >= (3ull << 20);
+}
+
+// The packed lists for R vectors of type t, built here on first use; false
+// where they do not fit or cannot be built.
+bool make_block_list(qk_plan* p, qk_dtype t, int R) {
+  if (!p->all_real || g_kernel_policy != 0 || !g_list_path) return false;
+  const size_t row = size_t(R) * qk_dtype_size(t), limit = size_t(p->dim) * row / 2;
+  if (row > 1024 || p->block_list_bytes > limit) return false;
+  if (p->block_list) return true;
+  const double* dv = real_diag(p);
+  if (dv || !p->has_diag)
+    p->block_list = block_list_create(dev(p), p->dim, dv, limit, &p->block_list_bytes, &p->bytes);
+  return p->block_list != nullptr;
+}
+
 int r_index(int R) { return R == 32 ? 0 : R == 64 ? 1 : R == 128 ? 2 : -1; }
 
 }  // namespace
@@ -530,12 +569,13 @@ int qkd_plan_create(const qk_plan_desc* d, int device, qk_plan** out) {
 }
 
 int qkd_set_kernel_policy(int policy) {
-  if (policy < 0 || policy > 3) return QKD_EINVAL;
+  if (policy < 0 || policy > 4) return QKD_EINVAL;
   g_kernel_policy = policy == 1 ? 1 : 0;
   g_list_path = policy != 3;
   qkd::spin_set_die_queues(policy != 2);
   g_die_queues = policy != 2;
   g_pair_path = policy != 3;
+  g_list_shapes = policy == 4;
   return QKD_OK;
 }
 
@@ -653,14 +693,25 @@ static int apply_rows_shape(const qk_plan* p, qk_workspace* w, qk_dtype t, int R
   return QKD_EINVAL;
 }
 
+// Lanes per row of the packed lists for this block apply, 0 for the row
+// kernels: the tuner's, or under policy 4 the caller's.
+static int list_lanes(const qk_plan* p, qk_dtype t, int R, int lanes_per_row, cudaStream_t s) {
+  if (g_kernel_policy != 0 || !g_list_path) return 0;
+  if (!lanes_per_row) return p->rows_list[t][r_index(R)];
+  if (!g_list_shapes) return 0;
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  if (!p->block_list && (cudaStreamIsCapturing(s, &st) != cudaSuccess || st != cudaStreamCaptureStatusNone)) return 0;
+  return make_block_list(const_cast<qk_plan*>(p), t, R) ? lanes_per_row : 0;
+}
+
 int qkd_apply_rows(const qk_plan* p, qk_workspace* w, qk_dtype t, int R, int lanes_per_row, const void* X,
                    void* Y, const void* diag, double* dots, cudaStream_t s) {
   if (!p || r_index(R) < 0 || t < QK_C128 || t > QK_F32) return QKD_EINVAL;
   StreamOrder::Use use(*p->order, s);
   const int lpr = lanes_per_row ? lanes_per_row : (p->rows_lpr[t][r_index(R)] ? p->rows_lpr[t][r_index(R)] : 32);
   const int tilec = lanes_per_row ? 0 : p->rows_tile[t][r_index(R)];
-  const int list = lanes_per_row ? 0 : p->rows_list[t][r_index(R)];
-  if (list && w && X && Y && X != Y && g_kernel_policy == 0 && g_list_path) {
+  const int list = list_lanes(p, t, R, lanes_per_row, s);
+  if (list && w && X && Y && X != Y) {
     const int rc = block_list_apply(p->block_list, t, R, list, g_die_queues, X, Y, dots, s, nullptr);
     if (rc != QKD_EINVAL) return rc;
   }
@@ -673,8 +724,8 @@ int qkd_apply_rows_acc(const qk_plan* p, qk_workspace* w, qk_dtype t, int R, int
   StreamOrder::Use use(*p->order, s);
   const int lpr = lanes_per_row ? lanes_per_row : (p->rows_lpr[t][r_index(R)] ? p->rows_lpr[t][r_index(R)] : 32);
   const int tilec = lanes_per_row ? 0 : p->rows_tile[t][r_index(R)];
-  const int list = lanes_per_row ? 0 : p->rows_list[t][r_index(R)];
-  if (list && w && X && Y && X != Y && p->spin && g_kernel_policy == 0 && g_list_path) {
+  const int list = list_lanes(p, t, R, lanes_per_row, s);
+  if (list && w && X && Y && X != Y && p->spin) {
     const int rc = block_list_apply(p->block_list, t, R, list, g_die_queues, X, Y, dots, s, g);
     if (rc != QKD_EINVAL) return rc;
   }
@@ -736,17 +787,10 @@ static int tune_rows(qk_plan* p, qk_workspace* w, qk_dtype t, int R, const void*
   for (int q = 0; q < 3; ++q)
     for (int tc = 0; tc < 3; ++tc)
       p->rows_ms[t][r_index(R)][q * 3 + tc] = (tc < ntile && fastest[q][tc] < 1e29f) ? fastest[q][tc] : 0.f;
-  // the packed lists (4 bytes per target against R elements of its row; at
-  // most half a block vector) against the best of those shapes
-  int pick_list = 0;
-  const size_t list_max = size_t(p->dim) * R * qk_dtype_size(t) / 2;
-  if (p->all_real && !p->block_list && g_kernel_policy == 0 && g_list_path && list_max > p->block_list_tried) {
-    p->block_list_tried = list_max;
-    if (const double* dv = real_diag(p); dv || !p->has_diag)
-      p->block_list = block_list_create(dev(p), p->dim, dv, list_max, &p->bytes);
-  }
-  if (p->block_list && g_kernel_policy == 0 && g_list_path) {
+  int pick_list = 0;  // lanes per row of the packed lists, where the rule takes them
+  if (block_list_pays(p, t, R) && make_block_list(p, t, R)) {
     cudaEvent_t s0, s1;
+    float best_list = 1e30f;
     if (cudaEventCreate(&s0) != cudaSuccess || cudaEventCreate(&s1) != cudaSuccess) return QKD_ECUDA;
     for (int q = 0; q < 3; ++q) {
       if (R / lprs[q] > 8) continue;
@@ -757,7 +801,7 @@ static int tune_rows(qk_plan* p, qk_workspace* w, qk_dtype t, int R, const void*
         cudaEventRecord(s1, s);
         float ms = 0.f;
         if (cudaEventSynchronize(s1) != cudaSuccess || cudaEventElapsedTime(&ms, s0, s1) != cudaSuccess) break;
-        if (i && ms < best) { best = ms; pick_list = lprs[q]; }
+        if (i && ms < best_list) { best_list = ms; pick_list = lprs[q]; }
       }
     }
     cudaEventDestroy(s0);

@@ -639,10 +639,14 @@ void block_list_destroy(BlockListHandle* h) {
 
 // Packed lists of a real operator (diag as in list_plan_create); null when
 // they exceed max_bytes, the ranks 24 bits, the coefficients the class table,
-// or the memory is not there.
+// or the memory is not there.  *list_bytes: the size of the words once they are
+// counted, ~0 when the ranks or the class table are too small for them.
 BlockListHandle* block_list_create(const DevPlan& p, uint64_t dim, const double* diag, size_t max_bytes,
-                                   size_t* dev_bytes) {
-  if (dim == 0 || dim > kListMaxDim || p.ngroups == 0) return nullptr;
+                                   size_t* list_bytes, size_t* dev_bytes) {
+  if (dim == 0 || dim > kListMaxDim || p.ngroups == 0) {
+    *list_bytes = ~size_t(0);
+    return nullptr;
+  }
   uint64_t* st = nullptr;
   unsigned long long* table = nullptr;
   uint32_t *start = nullptr, *words = nullptr, *wq = nullptr;
@@ -659,7 +663,11 @@ BlockListHandle* block_list_create(const DevPlan& p, uint64_t dim, const double*
                                       reinterpret_cast<int*>(table + kListClasses));
     ok = cudaGetLastError() == cudaSuccess &&
          cudaMemcpy(hs.data(), start, dim * 4, cudaMemcpyDeviceToHost) == cudaSuccess &&
-         cudaMemcpy(ht.data(), table, ht.size() * 8, cudaMemcpyDeviceToHost) == cudaSuccess && ht[kListClasses] == 0;
+         cudaMemcpy(ht.data(), table, ht.size() * 8, cudaMemcpyDeviceToHost) == cudaSuccess;
+    if (ok && ht[kListClasses] != 0) {
+      *list_bytes = ~size_t(0);
+      ok = false;
+    }
   }
   uint64_t total = 0;
   for (uint64_t i = 0; ok && i < dim; ++i) {
@@ -668,6 +676,7 @@ BlockListHandle* block_list_create(const DevPlan& p, uint64_t dim, const double*
     total += n;
   }
   hs[dim] = uint32_t(total);
+  if (ok) *list_bytes = size_t(total) * 16;
   ok = ok && total < (1ull << 32) && total * 16 <= max_bytes &&
        cudaMalloc(&words, std::max<uint64_t>(total, 1) * 16) == cudaSuccess &&
        cudaMemcpy(start, hs.data(), hs.size() * 4, cudaMemcpyHostToDevice) == cudaSuccess;

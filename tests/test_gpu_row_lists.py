@@ -125,3 +125,59 @@ def test_no_diagonal_leaves_infinities_to_the_rows_they_couple_to(kind, N, sec, 
     H.apply_block_device(X.data_ptr(), Y.data_ptr(), qk.DTYPE_F64, 32)
     torch.cuda.synchronize()
     assert torch.equal(torch.isfinite(Y), got["generic"][:, None].expand(-1, 32))
+
+
+@pytest.mark.parametrize("kind,N,sec,terms", [
+    ("spin", 7, {}, O.heisenberg_chain(7)),                                         # 128 rows: four whole tiles
+    ("spin", 9, dict(use_sz=1, sz2=1), O.j1j2_chain(9, 1.0, 0.5)),                  # 126 rows: ragged last tile
+    ("spin", 9, {}, [(0.7, [("Sx", i)]) for i in range(9)]),                        # no diagonal
+    ("tj", 8, dict(use_nup=1, nup=3, use_ndn=1, ndn=3), O.tj_chain(8)),             # rows of 0 to 12 targets
+])
+def test_every_shape_of_the_packed_lists(kind, N, sec, terms):
+    H = ham(kind, N, sec, terms)
+    ref = O.port().hamiltonian(kind, N, sec, terms)
+    rng = np.random.default_rng(N)
+    Xc = rng.standard_normal((H.dimension, 128)) + 1j * rng.standard_normal((H.dimension, 128))
+    for code, tdt, tol in [(qk.DTYPE_C128, torch.complex128, 1e-12), (qk.DTYPE_C64, torch.complex64, 2e-5),
+                           (qk.DTYPE_F64, torch.float64, 1e-12), (qk.DTYPE_F32, torch.float32, 2e-5)]:
+        for R in (32, 64, 128):
+            X = torch.tensor((Xc if tdt.is_complex else Xc.real)[:, :R], dtype=tdt, device="cuda").contiguous()
+            Xh = X.cpu().numpy().astype(np.complex128)
+            want = np.stack([ref.apply(np.ascontiguousarray(Xh[:, r])) for r in range(R)], axis=1)
+            d = np.einsum("ir,ir->r", Xh.conj(), want)
+            for lanes in (32, 16, 8):
+                if R // lanes > 8:
+                    continue
+                Y = torch.full_like(X, float("nan"))
+                torch.cuda.synchronize()
+                qk.set_kernel_policy("packed-shapes")
+                try:
+                    dots = H.apply_block_device(X.data_ptr(), Y.data_ptr(), code, R, lanes_per_row=lanes, dots=True)
+                finally:
+                    qk.set_kernel_policy("auto")
+                assert rel(Y.cpu().numpy().astype(np.complex128), want) < tol, (code, R, lanes)
+                assert np.abs(dots[0::2] + 1j * dots[1::2] - d).max() <= 10 * tol * np.abs(d).max() + 1e-300, (code, R, lanes)
+
+
+def test_block_results_do_not_depend_on_what_was_applied_before():
+    """Which block kernel runs follows from sizes alone: the same bits from an
+    operator whose packed lists another block size has built already."""
+    n = 20
+    sec, terms = dict(use_sz=1, sz2=0), O.j1j2_chain(n, 1.0, 0.4)
+    Hs = [ham("spin", n, sec, terms) for _ in range(3)]
+    D = Hs[0].dimension
+    X = torch.randn(D, 64, dtype=torch.float64, device="cuda", generator=torch.Generator("cuda").manual_seed(n))
+    x = X[:, :32].float().contiguous()
+    ys = []
+    for k, H in enumerate(Hs):
+        Y, y = torch.empty_like(X), torch.empty_like(x)
+        torch.cuda.synchronize()
+        if k:
+            H.apply_block_device(X.data_ptr(), Y.data_ptr(), qk.DTYPE_F64, 64)
+        H.apply_block_device(x.data_ptr(), y.data_ptr(), qk.DTYPE_F32, 32)
+        if not k:
+            H.apply_block_device(X.data_ptr(), Y.data_ptr(), qk.DTYPE_F64, 64)
+        torch.cuda.synchronize()
+        ys.append((Y, y))
+    for Y, y in ys[1:]:
+        assert torch.equal(Y, ys[0][0]) and torch.equal(y, ys[0][1])
