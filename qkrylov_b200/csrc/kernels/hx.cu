@@ -28,6 +28,7 @@ void pair_plan_destroy(PairHandle* h);
 int pair_apply(const PairHandle* h, qk_dtype t, const void* x, void* y, cudaStream_t s, qk_workspace* w,
                double* dot_out);
 struct BlockListHandle;
+bool block_list_possible(const DevPlan& p, uint64_t dim);
 BlockListHandle* block_list_create(const DevPlan& p, uint64_t dim, const double* diag, size_t max_bytes,
                                    size_t* list_bytes, size_t* dev_bytes);
 void block_list_destroy(BlockListHandle* h);
@@ -421,6 +422,13 @@ const double* real_diag(qk_plan* p) {
   return p->list_diag;
 }
 
+void drop_real_diag(qk_plan* p) {
+  if (!p->list_diag) return;
+  cudaFree(p->list_diag);
+  p->list_diag = nullptr;
+  p->bytes -= p->dim * 8;
+}
+
 // The table-free kernel of unconditional flips, else the row lists of a small
 // sector, with the real diagonal they need.
 void make_lists(qk_plan* p, const qk_plan_desc* d) {
@@ -431,11 +439,7 @@ void make_lists(qk_plan* p, const qk_plan_desc* d) {
   if (flips) p->flip = flip_plan_create(d, diag, &p->bytes);
   const bool two_part = !p->pair && (!p->spin || qkd::spin_plan_is_gen(p->spin));
   if (!p->flip) p->list = list_plan_create(dev(p), p->dim, diag, two_part, &p->bytes);
-  if (!p->list && !p->flip && p->list_diag) {
-    cudaFree(p->list_diag);
-    p->list_diag = nullptr;
-    p->bytes -= p->dim * 8;
-  }
+  if (!p->list && !p->flip) drop_real_diag(p);
 }
 
 // Whether the block apply of R vectors of type t runs on packed lists where
@@ -470,9 +474,15 @@ bool make_block_list(qk_plan* p, qk_dtype t, int R) {
   const size_t row = size_t(R) * qk_dtype_size(t), limit = size_t(p->dim) * row / 2;
   if (row > 1024 || p->block_list_bytes > limit) return false;
   if (p->block_list) return true;
+  if (!block_list_possible(dev(p), p->dim)) {
+    p->block_list_bytes = ~size_t(0);
+    return false;
+  }
+  const bool had_diag = p->list_diag != nullptr;
   const double* dv = real_diag(p);
   if (dv || !p->has_diag)
     p->block_list = block_list_create(dev(p), p->dim, dv, limit, &p->block_list_bytes, &p->bytes);
+  if (!p->block_list && !had_diag) drop_real_diag(p);
   return p->block_list != nullptr;
 }
 

@@ -637,16 +637,14 @@ void block_list_destroy(BlockListHandle* h) {
   delete h;
 }
 
-// Packed lists of a real operator (diag as in list_plan_create); null when
-// they exceed max_bytes, the ranks 24 bits, the coefficients the class table,
-// or the memory is not there.  *list_bytes: the size of the words once they are
-// counted, ~0 when the ranks or the class table are too small for them.
+bool block_list_possible(const DevPlan& p, uint64_t dim) { return dim > 0 && dim <= kListMaxDim && p.ngroups > 0; }
+
+// Packed lists of a real operator (diag as in list_plan_create) for which
+// block_list_possible; null when they exceed max_bytes, the coefficients the
+// class table, or the memory is not there.  *list_bytes: the size of the words
+// once they are counted, ~0 when the class table is too small for them.
 BlockListHandle* block_list_create(const DevPlan& p, uint64_t dim, const double* diag, size_t max_bytes,
                                    size_t* list_bytes, size_t* dev_bytes) {
-  if (dim == 0 || dim > kListMaxDim || p.ngroups == 0) {
-    *list_bytes = ~size_t(0);
-    return nullptr;
-  }
   uint64_t* st = nullptr;
   unsigned long long* table = nullptr;
   uint32_t *start = nullptr, *words = nullptr, *wq = nullptr;

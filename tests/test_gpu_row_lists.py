@@ -181,3 +181,18 @@ def test_block_results_do_not_depend_on_what_was_applied_before():
         ys.append((Y, y))
     for Y, y in ys[1:]:
         assert torch.equal(Y, ys[0][0]) and torch.equal(y, ys[0][1])
+
+
+def test_refused_packed_lists_keep_nothing():
+    """A sector beyond the lists' 24-bit ranks: tuning its block apply must not
+    leave a diagonal (8 bytes per row) behind."""
+    n = 27
+    H = ham("spin", n, dict(use_sz=1, sz2=1), O.heisenberg_chain(n))
+    assert H.dimension > 1 << 24
+    before = qk.lib().qkrylov_hamiltonian_device_bytes(H._h)
+    X = torch.zeros(H.dimension, 32, dtype=torch.float32, device="cuda")
+    Y = torch.empty_like(X)
+    torch.cuda.synchronize()
+    H.apply_block_device(X.data_ptr(), Y.data_ptr(), qk.DTYPE_F32, 32)
+    torch.cuda.synchronize()
+    assert qk.lib().qkrylov_hamiltonian_device_bytes(H._h) == before
