@@ -36,7 +36,8 @@ int qkrylov_b200_device_count(void);
  * on a two-die GPU; 1: the generic kernel everywhere; 2: as 0 with the
  * blocks handed out in one grid-stride order (no per-die queues); 3: the row
  * kernels (Hubbard-type operators on the two-part one instead of their
- * spin-product path, small sectors without their row lists); 4: as 0, and an
+ * spin-product path, small sectors without their row lists, which operators
+ * created under it do not build); 4: as 0, and an
  * explicit lanes_per_row of the block apply names a shape of its packed lists
  * instead of the row kernels.  For comparisons; process-wide.  Other values:
  * QKRYLOV_ERROR_INVALID_ARG. */

@@ -46,6 +46,7 @@ void list_plan_destroy(ListHandle* h);
 int list_apply(const ListHandle* h, qk_dtype t, const void* x, void* y, cudaStream_t s, qk_workspace* w,
                double* dot_out, uint64_t row_lo, uint64_t row_hi);
 bool spin_plan_is_gen(const SpinHandle* h);
+void spin_plan_finish(SpinHandle* h, bool build);
 int spin_plan_set_diag(SpinHandle* h, const double* diag);
 int spin_apply_block(const SpinHandle* h, qk_dtype t, int R, int lpr, const void* X, void* Y, double* dots,
                      cudaStream_t s, qk_workspace* w, const double* gacc = nullptr, int tilec = 0);
@@ -566,7 +567,12 @@ int qkd_plan_create(const qk_plan_desc* d, int device, qk_plan** out) {
     p->spin = nullptr;
   }
   if (d->pair_sites && p->diag_re) p->pair = qkd::pair_plan_create(d, p->A, p->B, p->diag_re, &p->bytes);
-  if (d->all_real && !d->transient && d->dim > 0) make_lists(p, d);
+  // none under the policy without lists
+  if (d->all_real && !d->transient && d->dim > 0 && g_list_path) make_lists(p, d);
+  // One-shot plans and plans served by lists or flips stay on the one-block row
+  // kernel where they use a row kernel at all: the tables of the grouped one
+  // cost more than they save (one apply of t-J N=20 0.3 ms, its tables 29 ms).
+  if (p->spin) qkd::spin_plan_finish(p->spin, !d->transient && !p->list && !p->flip);
   // the uploads from pageable memory and the cleared counters above may still
   // be on their way, and an apply on a non-blocking stream would not wait
   if (cudaStreamSynchronize(nullptr) != cudaSuccess) {

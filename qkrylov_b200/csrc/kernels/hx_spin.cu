@@ -14,6 +14,7 @@
 // state of a row comes from the coalesced low-part list.  One thread per row,
 // 512 rows per tile.
 #include <algorithm>
+#include <functional>
 #include <mutex>
 #include <vector>
 
@@ -737,6 +738,7 @@ struct SpinHandle {
   int n0 = 0, n1 = 0;      // SMs of each die
   bool lean = false;       // every bond conserves the charge: row kernel
   GroupHandle* grp = nullptr;  // the grouped row kernel's plan, or null
+  std::function<void()> add_groups;  // builds it; only while the plan is made
   // per-tile column-dot partials of the queued block kernel, sized on first use
   mutable std::mutex tp_mu;
   mutable double* tile_part = nullptr;
@@ -863,6 +865,11 @@ static std::vector<uint32_t> record_order(const std::vector<uint32_t>& rec_h, in
 // positions; per run and coefficient class the targets in conflict-free slots
 // (SlotTile).  tile0[key]: first tile of the class.
 struct LowEnt { uint16_t cls, rank; };
+struct LowTargets {
+  std::vector<uint32_t> off;  // per position, and the end
+  std::vector<LowEnt> ent;
+  std::vector<uint32_t> key;  // per block record: its class of low parts
+};
 static bool warp_tiles(const uint32_t* key_off, uint32_t nkeys, const std::vector<uint32_t>& off,
                        const std::vector<LowEnt>& ent, int ncls, uint32_t zero_slot,
                        std::vector<uint2>& wrec, std::vector<uint2>& wgrp, std::vector<uint32_t>& tile0) {
@@ -893,10 +900,12 @@ static bool warp_tiles(const uint32_t* key_off, uint32_t nkeys, const std::vecto
 
 // The grouped kernel's plan from the tables of a row plan whose device
 // copies are in place; wrec / wgrp go to bufs[8] and bufs[9].
-static void add_groups(SpinHandle* out, const SpinPlan& h, const std::vector<RowBlock>& brec,
-                       const std::vector<uint32_t>& tile_of, const std::vector<uint32_t>& order,
-                       const std::vector<uint2>& bent, const std::vector<uint2>& wrec, const std::vector<uint2>& wgrp,
-                       size_t* dev_bytes) {
+static void add_groups(SpinHandle* out, const SpinPlan& h, const qk_plan_desc* d, const LowTargets& low,
+                       const std::vector<RowBlock>& brec, const std::vector<uint32_t>& order,
+                       const std::vector<uint2>& bent, size_t* dev_bytes) {
+  std::vector<uint2> wrec, wgrp;
+  std::vector<uint32_t> tile0;
+  if (!warp_tiles(d->key_off, d->nkeys, low.off, low.ent, std::max(1, h.ncls), h.zero_slot, wrec, wgrp, tile0)) return;
   auto up = [&](int slot, const std::vector<uint2>& v) {
     if (cudaMalloc(&out->bufs[slot], v.size() * sizeof(uint2)) != cudaSuccess) return false;
     *dev_bytes += v.size() * sizeof(uint2);
@@ -930,7 +939,7 @@ static void add_groups(SpinHandle* out, const SpinPlan& h, const std::vector<Row
   for (uint32_t i = 0; i < uint32_t(brec.size()); ++i) {
     const uint32_t r = order.empty() ? i : order[i];
     const RowBlock& b = brec[r];
-    blocks.push_back(GroupBlock{b.base, b.size, b.lst, tile_of[r], b.ebeg, b.nh, b.combo, b.dh});
+    blocks.push_back(GroupBlock{b.base, b.size, b.lst, tile0[low.key[r]], b.ebeg, b.nh, b.combo, b.dh});
   }
   out->grp = group_plan_create(g, blocks, bent, out->n0 + out->n1 ? out->n0 : 1, out->n0 + out->n1 ? out->n1 : 0, dev_bytes);
 }
@@ -1068,8 +1077,8 @@ SpinHandle* spin_plan_create(const qk_plan_desc* d, size_t* dev_bytes) {
   // diagonal table at most 16 MB, a free u16 index for the zero slot, and
   // every high-bond partner block of the same size as the block (which is
   // what keeps the coalesced high-bond loads in bounds).
-  std::vector<uint2> rrec, lgrp, bent, wrec, wgrp;
-  std::vector<uint32_t> tile0, tile_of;
+  std::vector<uint2> rrec, lgrp, bent;
+  LowTargets low;
   std::vector<uint16_t> crk;
   std::vector<double> dtab;
   std::vector<RowBlock> brec;
@@ -1125,12 +1134,11 @@ SpinHandle* spin_plan_create(const qk_plan_desc* d, size_t* dev_bytes) {
       if (lgrp.empty()) lgrp.push_back(make_uint2(0, 0));
     }
     if (h.rows_ok) {
-      std::vector<LowEnt> ent(loff[d->nllist]);
-      for (size_t e = 0; e < ent.size(); ++e)
-        ent[e] = LowEnt{uint16_t(cls_of[lent[e] & 0xFFu]), uint16_t(lent[e] >> 8)};
-      if (!warp_tiles(d->key_off, d->nkeys, loff, ent, std::max(1, h.ncls), h.zero_slot, wrec, wgrp, tile0))
-        wrec.clear();
-      tile_of.assign(d->nA, 0);
+      low.off = loff;
+      low.ent.resize(loff[d->nllist]);
+      for (size_t e = 0; e < low.ent.size(); ++e)
+        low.ent[e] = LowEnt{uint16_t(cls_of[lent[e] & 0xFFu]), uint16_t(lent[e] >> 8)};
+      low.key.assign(d->nA, 0);
     }
     if (h.rows_ok) {
       crk.assign(std::max<uint64_t>(2, d->nllist * uint64_t(h.cpad)), 0);
@@ -1165,7 +1173,7 @@ SpinHandle* spin_plan_create(const qk_plan_desc* d, size_t* dev_bytes) {
         b.base = uint32_t(d->A[hh] & qkb::kOffsetMask);
         b.size = need == qkb::kEmptyBlockKey ? 0 : d->key_off[need + 1] - d->key_off[need];
         b.lst = hlst[hh];
-        if (need != qkb::kEmptyBlockKey) tile_of[hh] = tile0[need];
+        if (need != qkb::kEmptyBlockKey) low.key[hh] = need;
         b.ebeg = uint32_t(bent.size());
         b.nh = hoff[hh + 1] - hoff[hh];
         b.dh = dhi[hh];
@@ -1245,7 +1253,7 @@ SpinHandle* spin_plan_create(const qk_plan_desc* d, size_t* dev_bytes) {
       out->bt[1] = static_cast<const uint4*>(out->bufs[6]); out->nbt[1] = uint32_t(bt1.size());
       out->bt[2] = static_cast<const uint4*>(out->bufs[7]); out->nbt[2] = uint32_t(bt2.size());
       set_die_queues(out, h, brec, bord, dev_bytes);
-      if (!wrec.empty()) add_groups(out, h, brec, tile_of, bord, bent, wrec, wgrp, dev_bytes);
+      out->add_groups = [=] { add_groups(out, h, d, low, brec, bord, bent, dev_bytes); };
     }
     out->host = h;
     ok = cudaMalloc(reinterpret_cast<void**>(&out->dev), sizeof(SpinPlan)) == cudaSuccess &&
@@ -1328,13 +1336,13 @@ SpinHandle* gen_plan_create(const qk_plan_desc* d, size_t* dev_bytes) {
   std::vector<uint32_t> crm(std::max<uint64_t>(1, nll), 0);
   std::vector<double> cls;
   std::vector<uint16_t> bucket[kRowCls];
-  std::vector<LowEnt> went;
-  std::vector<uint32_t> woff(nll + 1, 0);
+  LowTargets low;
+  low.off.assign(nll + 1, 0);
   for (uint64_t pos = 0; pos < nll; ++pos) {
     const uint32_t l = d->llist[pos];
     const uint32_t key = d->B[l] >> 24;
     for (auto& b : bucket) b.clear();
-    woff[pos] = uint32_t(went.size());
+    low.off[pos] = uint32_t(low.ent.size());
     for (size_t q = 0; q < lowg.size(); ++q) {
       const qk_group_t& g = d->groups[lowg[q]];
       const double c = group_value(g, l, true);
@@ -1349,7 +1357,7 @@ SpinHandle* gen_plan_create(const qk_plan_desc* d, size_t* dev_bytes) {
         ci = int(cls.size()) - 1;
       }
       bucket[ci].push_back(uint16_t(d->B[lt] & 0xFFFFu));
-      went.push_back(LowEnt{uint16_t(ci), uint16_t(d->B[lt] & 0xFFFFu)});
+      low.ent.push_back(LowEnt{uint16_t(ci), uint16_t(d->B[lt] & 0xFFFFu)});
     }
     rrec[pos].x = uint32_t(lgrp.size());
     uint32_t counts = 0;
@@ -1382,12 +1390,7 @@ SpinHandle* gen_plan_create(const qk_plan_desc* d, size_t* dev_bytes) {
   if (lgrp.empty()) lgrp.push_back(make_uint2(0, 0));
   h.ncls = int(cls.size());
   for (int c = 0; c < h.ncls; ++c) h.lcls[c] = cls[c];
-  woff[nll] = uint32_t(went.size());
-  std::vector<uint2> wrec, wgrp;
-  std::vector<uint32_t> tile0, tile_of;
-  if (!warp_tiles(d->key_off, d->nkeys, woff, went, std::max(1, h.ncls), h.zero_slot,
-                  wrec, wgrp, tile0))
-    wrec.clear();
+  low.off[nll] = uint32_t(low.ent.size());
   // block records of the non-empty blocks
   std::vector<RowBlock> brec;
   std::vector<uint2> bent;
@@ -1402,7 +1405,7 @@ SpinHandle* gen_plan_create(const qk_plan_desc* d, size_t* dev_bytes) {
     b.base = uint32_t(d->A[hh] & qkb::kOffsetMask);
     b.size = size;
     b.lst = d->key_off[need];
-    tile_of.push_back(tile0.empty() ? 0u : tile0[need]);
+    low.key.push_back(need);
     b.ebeg = uint32_t(bent.size());
     b.dh = 0.0;
     for (uint32_t gi : highg) {
@@ -1476,7 +1479,7 @@ SpinHandle* gen_plan_create(const qk_plan_desc* d, size_t* dev_bytes) {
     out->bt[1] = static_cast<const uint4*>(out->bufs[6]); out->nbt[1] = uint32_t(t1.size());
     out->bt[2] = static_cast<const uint4*>(out->bufs[7]); out->nbt[2] = uint32_t(t2.size());
     set_die_queues(out, h, brec, rord, dev_bytes);
-    if (!wrec.empty()) add_groups(out, h, brec, tile_of, rord, bent, wrec, wgrp, dev_bytes);
+    out->add_groups = [=] { add_groups(out, h, d, low, brec, rord, bent, dev_bytes); };
     out->host = h;
     ok = cudaMalloc(reinterpret_cast<void**>(&out->dev), sizeof(SpinPlan)) == cudaSuccess &&
          cudaMemcpy(out->dev, &h, sizeof(SpinPlan), cudaMemcpyHostToDevice) == cudaSuccess;
@@ -1488,6 +1491,14 @@ SpinHandle* gen_plan_create(const qk_plan_desc* d, size_t* dev_bytes) {
     return nullptr;
   }
   return out;
+}
+
+// Ends a plan's creation: the grouped kernel's tables where build, which take
+// longer to make than the others together (Heisenberg N=24: 2.4 of 5.1 ms, t-J
+// N=20: 29 of 58 ms).
+void spin_plan_finish(SpinHandle* h, bool build) {
+  if (build && h->add_groups) h->add_groups();
+  h->add_groups = nullptr;
 }
 
 int spin_apply_rows(const SpinHandle* h, qk_dtype t, const void* x, void* y, cudaStream_t s,
