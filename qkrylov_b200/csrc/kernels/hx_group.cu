@@ -395,27 +395,41 @@ void group_plan_destroy(GroupHandle* h) {
   delete h;
 }
 
-// Groups of at most G blocks of `blocks` (visiting order) that share class,
-// combo and crossing flags.
-static std::vector<GroupRec> make_groups(const std::vector<GroupBlock>& blocks, const std::vector<uint2>& bent,
-                                         int ncross, uint32_t G) {
-  std::vector<GroupRec> out;
-  std::map<std::vector<uint32_t>, uint32_t> open;
-  std::vector<uint32_t> key;
+// Number of every block's kind: blocks that share class, combo and crossing
+// flags have the same one.
+static std::vector<uint32_t> block_kinds(const std::vector<GroupBlock>& blocks, const std::vector<uint2>& bent,
+                                         int ncross) {
+  std::map<std::vector<uint32_t>, uint32_t> known;
+  std::vector<uint32_t> kind, key;
   for (const GroupBlock& k : blocks) {
+    key.clear();
+    if (k.size) {
+      key.assign({k.lst, k.combo});
+      for (int q = 0; q < ncross; ++q) key.push_back(bent[k.ebeg + k.nh + q].y);
+    }
+    kind.push_back(known.emplace(key, uint32_t(known.size())).first->second);
+  }
+  return kind;
+}
+
+// Groups of at most G blocks of `blocks` (visiting order) of one kind.
+static std::vector<GroupRec> make_groups(const std::vector<GroupBlock>& blocks, const std::vector<uint32_t>& kind,
+                                         uint32_t G) {
+  std::vector<GroupRec> out;
+  constexpr uint32_t kNone = ~0u;
+  std::vector<uint32_t> open(blocks.size(), kNone);  // per kind: its group being filled
+  for (size_t i = 0; i < blocks.size(); ++i) {
+    const GroupBlock& k = blocks[i];
     if (k.size == 0) continue;
-    key.assign({k.lst, k.combo});
-    for (int q = 0; q < ncross; ++q) key.push_back(bent[k.ebeg + k.nh + q].y);
-    auto it = open.find(key);
-    if (it == open.end() || out[it->second].count == G) {
+    uint32_t& at = open[kind[i]];
+    if (at == kNone || out[at].count == G) {
       GroupRec r{};
       r.size = k.size; r.lst = k.lst; r.tile0 = k.tile0; r.combo = k.combo;
       for (uint32_t g = 0; g < kGroupMax; ++g) { r.base[g] = k.base; r.ebeg[g] = k.ebeg + k.nh; r.nh[g] = 0; r.dh[g] = k.dh; }
+      at = uint32_t(out.size());
       out.push_back(r);
-      open[key] = uint32_t(out.size() - 1);
-      it = open.find(key);
     }
-    GroupRec& r = out[it->second];
+    GroupRec& r = out[at];
     const uint32_t g = r.count++;
     r.base[g] = k.base; r.ebeg[g] = k.ebeg; r.nh[g] = uint16_t(k.nh); r.dh[g] = k.dh;
   }
@@ -441,8 +455,9 @@ static void largest_first(std::vector<GroupRec>& rec) {
 GroupHandle* group_plan_create(const GroupPlan& tables, const std::vector<GroupBlock>& blocks,
                                const std::vector<uint2>& bent, int n0, int n1, size_t* dev_bytes) {
   auto* h = new GroupHandle;
+  const std::vector<uint32_t> kind = block_kinds(blocks, bent, tables.ncross);
   for (int i = 0; i < 4; ++i) {
-    std::vector<GroupRec> rec = make_groups(blocks, bent, tables.ncross, i == 3 ? 2u : 4u >> i);
+    std::vector<GroupRec> rec = make_groups(blocks, kind, i == 3 ? 2u : 4u >> i);
     if (i < 2 && tables.dim <= 6300000) largest_first(rec);
     GroupPlan& p = h->plan[i];
     p = tables;

@@ -77,35 +77,47 @@ class SlotTile {
   // free ones along the alternating path from the bank; in a bipartite graph
   // that path does not reach the row.
   std::vector<int> colours(const Quarter& q, int ncol) const {
-    const size_t n = q.row.size();
-    std::vector<int> slot(n, -1), at_row(size_t(8) * ncol, -1), at_bank(size_t(8) * ncol, -1);
-    auto row = [&](size_t e, int c) -> int& { return at_row[size_t(q.row[e]) * ncol + c]; };
-    auto bank = [&](size_t e, int c) -> int& { return at_bank[size_t(q.word[e] & mask_ & 7u) * ncol + c]; };
+    const size_t n = q.row.size(), nw = (size_t(ncol) + 63) / 64;
+    std::vector<int> slot(n, -1), at(size_t(16) * ncol, -1);
+    std::vector<uint64_t> open(16 * nw, ~0ull);  // colours free at each row, then at each bank group
+    if (ncol % 64)
+      for (size_t v = 0; v < 16; ++v) open[v * nw + nw - 1] = (1ull << (ncol % 64)) - 1;
+    auto row = [&](size_t e) { return size_t(q.row[e]); };
+    auto bank = [&](size_t e) { return size_t(8 + (q.word[e] & mask_ & 7u)); };
+    auto put = [&](size_t v, int c, int e) {
+      at[v * ncol + c] = e;
+      const uint64_t bit = 1ull << (c & 63);
+      uint64_t& w = open[v * nw + size_t(c) / 64];
+      w = e < 0 ? w | bit : w & ~bit;
+    };
+    auto first = [&](size_t u, size_t v) {  // lowest colour free at both, -1: none
+      for (size_t w = 0; w < nw; ++w)
+        if (const uint64_t m = open[u * nw + w] & open[v * nw + w]) return int(w * 64) + __builtin_ctzll(m);
+      return -1;
+    };
     for (size_t k = 0; k < n; ++k) {
-      int fr = -1, fb = -1, both = -1;
-      for (int c = 0; c < ncol && both < 0; ++c) {
-        const bool r = row(k, c) < 0, b = bank(k, c) < 0;
-        if (r && fr < 0) fr = c;
-        if (b && fb < 0) fb = c;
-        if (r && b) both = c;
-      }
-      if (both < 0) {
+      const size_t r = row(k), b = bank(k);
+      int c = first(r, b);
+      if (c < 0) {
+        const int fr = first(r, r), fb = first(b, b);
         std::vector<int> path;
-        int c = fr;
-        for (int e = bank(k, c); e >= 0;) {
+        int a = fr;
+        for (int e = at[b * ncol + a]; e >= 0;) {
           path.push_back(e);
-          c = c == fr ? fb : fr;
-          e = (path.size() & 1) ? row(e, c) : bank(e, c);
+          a = a == fr ? fb : fr;
+          e = at[((path.size() & 1) ? row(e) : bank(e)) * ncol + a];
         }
-        for (int e : path) row(e, slot[e]) = bank(e, slot[e]) = -1;
+        for (int e : path) { put(row(e), slot[e], -1); put(bank(e), slot[e], -1); }
         for (int e : path) {
           slot[e] = slot[e] == fr ? fb : fr;
-          row(e, slot[e]) = bank(e, slot[e]) = e;
+          put(row(e), slot[e], e);
+          put(bank(e), slot[e], e);
         }
-        both = fr;
+        c = fr;
       }
-      slot[k] = both;
-      row(k, both) = bank(k, both) = int(k);
+      slot[k] = c;
+      put(r, c, int(k));
+      put(b, c, int(k));
     }
     return slot;
   }
