@@ -436,12 +436,15 @@ static std::vector<GroupRec> make_groups(const std::vector<GroupBlock>& blocks, 
   return out;
 }
 
-// Largest groups first, dealt in turn to the two dies' halves: for sectors
-// that the L2 caches hold (up to 6.3 M rows: 50 MB of 8-byte vectors), where a
-// few large groups at the end of the queue would leave SMs idle.  us per apply,
-// visiting order -> this: t-J N=19 float32 90.7 -> 78.1, Heisenberg N=25
-// float32 57.3 -> 55.4, float64 79.7 -> 74.8; complex128 on exchange tables
-// loses (Heisenberg N=25 126 -> 134) and keeps the visiting order.
+// Largest groups first, dealt in turn to the two dies' halves, so that no large
+// group is left for the end of the queue and SMs idle.  For vectors of up to the
+// L2 caches' size (kL2Bytes), which do not need the visiting order's locality.
+// us per apply, visiting order -> this: t-J N=20 (9.2 M rows) float32 173 -> 132,
+// float64 266 -> 220, complex128 425 -> 425; Heisenberg N=25 float32 54.0 ->
+// 49.7, float64 73.4 -> 68.7, N=26 float64 (83 MB) 145 -> 138, N=27 float32
+// (80 MB) 179 -> 171, float64 (160 MB) 259.7 -> 260.6.  complex128 on exchange
+// tables loses (N=25 126 -> 134) and keeps the visiting order.
+constexpr uint64_t kL2Bytes = 126000000;
 static void largest_first(std::vector<GroupRec>& rec) {
   std::stable_sort(rec.begin(), rec.end(), [](const GroupRec& a, const GroupRec& b) {
     return uint64_t(a.size) * a.count > uint64_t(b.size) * b.count;
@@ -458,7 +461,7 @@ GroupHandle* group_plan_create(const GroupPlan& tables, const std::vector<GroupB
   const std::vector<uint32_t> kind = block_kinds(blocks, bent, tables.ncross);
   for (int i = 0; i < 4; ++i) {
     std::vector<GroupRec> rec = make_groups(blocks, kind, i == 3 ? 2u : 4u >> i);
-    if (i < 2 && tables.dim <= 6300000) largest_first(rec);
+    if (i < 2 && tables.dim * (i == 0 ? 4 : 8) <= kL2Bytes) largest_first(rec);  // float32; the 8-byte types
     GroupPlan& p = h->plan[i];
     p = tables;
     void* d = nullptr;
