@@ -231,10 +231,20 @@ CoreOut lanczos_core(const Operator& H, qk_dtype T, const void* start, int maxit
     }
     const double beta = std::sqrt(after);
     const bool more = beta >= 1e-15 && iter + 1 < lim;
-    if (more) {  // the next step's vector and product, while the host checks this one
-      V.push_back(d.vec(false));
+    auto launch_next = [&] {
       d.scale_into(1.0 / beta, w.data(), V.back().data());
       H.apply_dot(T, V.back().data(), w.data(), d.c.dres(0));
+    };
+    // the next step's vector and product, while the host checks this one; a run
+    // that ends here must not fail for want of that vector
+    bool ahead = false;
+    if (more) {
+      try {
+        V.push_back(d.vec(false));
+        ahead = true;
+      } catch (const DeviceError&) {
+      }
+      if (ahead) launch_next();
     }
     std::vector<double> z;
     const double e = tridiag_ground<double>(a, b, int(a.size()), &z);
@@ -249,6 +259,10 @@ CoreOut lanczos_core(const Operator& H, qk_dtype T, const void* start, int maxit
     e_old = e;
     if (!more) break;
     b.push_back(beta);
+    if (!ahead) {
+      V.push_back(d.vec(false));
+      launch_next();
+    }
   }
   if (ritz) {
     std::vector<double> z;
