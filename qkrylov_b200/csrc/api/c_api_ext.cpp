@@ -407,6 +407,7 @@ static int lanczos_two_phase(qkrylov_hamiltonian_h h, bool low_phase, uint64_t s
     const qk_dtype hi = real ? QK_F64 : QK_C128;
     std::unique_ptr<qkb::DevVec> sdev, pdev;
     const void* sptr = start;
+    if (start && start_on_device) H.ctx().after_default_stream();
     if (start && !start_on_device) {
       sdev = std::make_unique<qkb::DevVec>(dim, st, H.device(), false);
       qkb::cuda_check(cudaMemcpyAsync(sdev->data(), start, dim * qk_dtype_size(st), cudaMemcpyHostToDevice,
@@ -510,7 +511,9 @@ int qkrylov_b200_cf_block(qkrylov_hamiltonian_h h, int precision, int complex_ve
     const size_t count = size_t(H.dim()) * n_vectors;
     qkb::DevVec staged;
     const void* dstart = start;
-    if (!start_on_device) {
+    if (start_on_device) {
+      H.ctx().after_default_stream();
+    } else {
       qkb::Context& c = H.ctx();
       c.activate();
       staged = qkb::DevVec(count, t, H.device(), false);
@@ -609,6 +612,7 @@ int qkrylov_b200_mlp_start_vector(qkrylov_b200_mlp_h h, double j2, float* out, i
   return guarded([&] {
     const uint64_t dim = h->net->dim();
     if (out_on_device) {
+      qkb::Context::get(h->net->device()).after_default_stream();
       h->net->start_vector(j2, out);
       return QKRYLOV_SUCCESS;
     }

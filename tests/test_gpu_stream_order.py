@@ -75,6 +75,31 @@ def test_calls_without_a_stream_follow_the_default_stream(case, entry):
             assert rel(got, want) < 1e-13
 
 
+def test_device_start_vectors_follow_the_default_stream(case):
+    """Solvers whose start vectors are the caller's device memory."""
+    H, xh, _ = case
+    src = torch.tensor(xh, device="cuda")
+    blk = torch.randn(H.dimension, 32, dtype=torch.float64, device="cuda", generator=torch.Generator("cuda").manual_seed(2))
+    torch.cuda.synchronize()
+    x, X = src.clone(), blk.clone()
+    torch.cuda.synchronize()
+    want = qk.lanczos_fp64(H, start_device=x.data_ptr(), maxiter=5, tol=1e-3)
+    cf = qk.cf_block(H, X.data_ptr(), 6, n_vectors=32)
+    for _ in range(2):
+        x, X = torch.zeros_like(src), torch.zeros_like(blk)
+        torch.cuda.synchronize()
+        keep = busy()
+        x.copy_(src)
+        got = qk.lanczos_fp64(H, start_device=x.data_ptr(), maxiter=5, tol=1e-3)
+        assert got.energy == want.energy
+        keep = busy()
+        X.copy_(blk)
+        r = qk.cf_block(H, X.data_ptr(), 6, n_vectors=32)
+        torch.cuda.synchronize()
+        del keep
+        assert all(np.array_equal(p.alphas, q.alphas) for p, q in zip(r, cf))
+
+
 def test_range_hook_follows_the_current_stream(case):
     """The sharded Lanczos' range apply on a stream other than the default one."""
     H, xh, want = case
