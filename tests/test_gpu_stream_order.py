@@ -207,3 +207,47 @@ def test_block_applies_of_one_operator_on_several_streams(kind, n, sec, terms):
         for Y in Ys:
             Y.fill_(float("nan"))
         torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("route", ["lists", "groups", "flips", "spin-product", "block"])
+def test_applies_can_be_captured_and_replayed(route):
+    """One apply per kernel family captured on a caller's stream (after a first
+    call outside the capture), replayed on new contents of x; calls without a
+    stream go on beside the capture."""
+    kind, n, sec, terms = {
+        "lists": ("spin", 14, dict(use_sz=1, sz2=0), O.heisenberg_chain(14)),
+        "groups": ("spin", 24, dict(use_sz=1, sz2=0), O.heisenberg_chain(24)),
+        "flips": ("spin", 13, {}, [(0.7, [("Sx", i)]) for i in range(13)]),
+        "spin-product": ("hubbard", 13, dict(use_nup=1, nup=6, use_ndn=1, ndn=6), O.hubbard_square(13, 1)),
+        "block": ("tj", 12, dict(use_nup=1, nup=5, use_ndn=1, ndn=5), O.tj_chain(12)),
+    }[route]
+    H = ham(kind, n, sec, terms)
+    shape = (H.dimension, 32) if route == "block" else (H.dimension,)
+    g = torch.Generator("cuda").manual_seed(n)
+    xs = [torch.randn(shape, dtype=torch.float64, device="cuda", generator=g) for _ in range(2)]
+    x, y, z = xs[0].clone(), torch.empty(shape, dtype=torch.float64, device="cuda"), torch.empty(shape, dtype=torch.float64, device="cuda")
+
+    def call(a, b, stream=0):
+        if route == "block":
+            H.apply_block_device(a.data_ptr(), b.data_ptr(), qk.DTYPE_F64, 32, stream=stream)
+        else:
+            H.apply_device(a.data_ptr(), b.data_ptr(), qk.DTYPE_F64, stream=stream)
+
+    want = []
+    for v in xs:
+        call(v, z)
+        torch.cuda.synchronize()
+        want.append(z.clone())
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        call(x, y, torch.cuda.current_stream().cuda_stream)
+        call(xs[1], z)  # not part of the graph
+    torch.cuda.synchronize()
+    assert torch.equal(z, want[1])
+    for v, w in zip(xs, want):
+        x.copy_(v)
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(y, w), route
+    graph.reset()
