@@ -86,13 +86,16 @@ qkrylov_hamiltonian_h qkrylov_hamiltonian_create_ex(qkrylov_basis_h basis, qkryl
 int qkrylov_hamiltonian_precision(qkrylov_hamiltonian_h h);
 int qkrylov_hamiltonian_all_real(qkrylov_hamiltonian_h h);
 uint64_t qkrylov_hamiltonian_device_bytes(qkrylov_hamiltonian_h h);
-/* The H.x kernel of this handle: 1 the two-site exchange kernel (spin
+/* The H.x kernel family of this handle: 1 the two-site exchange kernel (spin
  * models in a single-charge sector), 2 the two-part kernel (operators whose
  * terms factorise over the sector split: Hubbard, t-J, fermion hops with
  * Jordan-Wigner signs), 3 the spin-product path (Hubbard-type operators with
  * N_up and N_dn conserved: T_up x 1 + 1 x T_dn + D in the (up, down) order,
  * the vector permuted at the boundary; block applies stay on the two-part
- * kernel), 0 the generic term-table kernel. */
+ * kernel), 0 the generic term-table kernel.  It follows from the operator's
+ * form: small sectors apply from row lists, complete bases with unconditional
+ * flips without tables, whatever family this names; it is what runs under
+ * policy 3 and in larger sectors. */
 int qkrylov_hamiltonian_kernel(qkrylov_hamiltonian_h h);
 /* The CUDA stream (cudaStream_t) the library uses on the handle's device. */
 void* qkrylov_hamiltonian_stream(qkrylov_hamiltonian_h h);
@@ -137,7 +140,9 @@ int qkrylov_hamiltonian_apply_range_device(qkrylov_hamiltonian_h h, int dtype, c
  * for each shape it tried on this operator, dtype and block size R (32, 64
  * or 128), ms9[3*i + j] for lanes per row 32, 16, 8 (i) and tile code j
  * (CTA tiles of 256, 128, 512 rows); 0 where a shape was not timed or the
- * tuner has not run (it runs on the first batched FTLM or sweep). */
+ * tuner has not run (it runs on the first batched FTLM or sweep).  Shapes of
+ * the row kernels: the packed lists, which a rule on sizes prefers where it
+ * takes them, are not in the table. */
 int qkrylov_b200_block_shape_timings(qkrylov_hamiltonian_h h, int dtype, int R, double* ms9);
 /* Block H.X on R vectors stored row-interleaved (element (i, r) at
  * X[i*R + r]; R = 32, 64 or 128; device memory, 16-byte aligned, X != Y):

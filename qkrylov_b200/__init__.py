@@ -435,7 +435,9 @@ class MatrixFreeHamiltonian:
         """The block apply's autotuner table for this operator: fastest timed
         launch in ms, rows = lanes per row 32, 16, 8, columns = CTA tiles of
         256, 128, 512 rows; 0 where not timed (the tuner runs on the first
-        batched FTLM or sweep with this precision and block size)."""
+        batched FTLM or sweep with this precision and block size).  The packed
+        lists, which a rule on sizes prefers where it takes them, are not in
+        the table."""
         dt = {64: DTYPE_F64, 32: DTYPE_F32}[precision]
         out = np.zeros(9)
         _check(lib().qkrylov_b200_block_shape_timings(self._h, dt, int(R), out.ctypes.data), "block_shape_timings")
@@ -443,7 +445,9 @@ class MatrixFreeHamiltonian:
 
     @property
     def kernel(self) -> str:
-        """The H.x kernel this operator uses: 'spin-exchange' (two-site
+        """The H.x kernel family of this operator's form (small sectors apply
+        from row lists, unconditional flips of a complete basis without
+        tables, whatever it names): 'spin-exchange' (two-site
         exchange in a single-charge sector), 'spin-product' (Hubbard-type
         operators with N_up and N_dn conserved: hops of one species applied
         as T_up x 1 + 1 x T_dn in the (up, down) order), 'two-part' (any

@@ -26,10 +26,12 @@
 // float32 and complex128, 48 registers and 40 warps for the 8-byte types; more
 // entries in flight, tables or slots loaded a row ahead and unconditional
 // crossing loads were each slower.  us per apply, one-block kernel -> this one:
-// Heisenberg N=24 float32 46.6 -> 33.9, N=25 float64 99 -> 70, N=24 complex128
-// 86 -> 63, N=28 float32 437 -> 323, float64 590 -> 522, complex128 980 -> 893;
-// J1-J2 N=24 float32 81 -> 54; t-J N=19 float64 177 -> 96, N=20 float64 329 ->
-// 264, complex128 529 -> 424.
+// Heisenberg N=24 float32 46.6 -> 35, N=25 float64 102 -> 69, N=24 complex128
+// 86 -> 64, N=28 float32 437 -> 325, float64 590 -> 513; J1-J2 N=24 float32 81 ->
+// 57; t-J N=19 float64 177 -> 96, N=20 float64 333 -> 222, complex128 529 -> 425.
+// Heisenberg N=28 complex128 depends on where the vectors lie: 980 -> 896 in two
+// buffers of cudaMalloc, 990-1033 -> 951-999 in two of torch's allocator (the
+// cause of the difference is not known).
 #include <algorithm>
 #include <cstring>
 #include <map>
@@ -88,7 +90,7 @@ k_hx_group(const __grid_constant__ GroupPlan p, const void* __restrict__ x, void
     sx[(tid / 8) * stride + p.zero_slot + tid % 8] = z;
   }
   // one coefficient for every high entry (uniform chains): summed, then scaled;
-  // complex128 alone gains (Heisenberg N=28 959 -> 924 us), the others need the
+  // complex128 alone gains (Heisenberg N=28, before the coloured slots, 959 -> 924 us), the others need the
   // registers (float64 531 -> 580)
   const bool uni = DT == QK_C128 && !GEN && p.uniform_high;
   const R high = R(p.high_coef);

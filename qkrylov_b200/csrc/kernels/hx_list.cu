@@ -9,16 +9,18 @@
 // target rank, 8 bits of coefficient class; class 0: no term, target = the
 // row itself).  Slots are groups, not packed per row, so the rows of a warp
 // follow the same bond and their targets are neighbouring addresses.  One
-// launch, three dependent loads: slice start, words, targets.
+// launch.  k_hx_list: three dependent loads (slice start, words, targets);
+// k_hx_list_small, for the smallest sectors: two (their slices have one width).
 //
 // Bound: latency up to ~2^17 rows, above that the L1/L2 traffic of words and
 // targets (4 + sizeof(element) bytes per slot and row).  Four slots of a row
 // share a 16-byte load (against one 4-byte word per slot: Heisenberg N=21
 // c128 14.4 -> 12.9 us, t-J N=16 f64 16.4 -> 13.7 us) and a batch of eight
 // loads the next batch's words before its own targets.  Against the row and
-// pair kernels (us per apply, launches back to back): Heisenberg N=16 c128
-// 10.3 -> 6.2, N=20 18.6 -> 10.3, t-J N=14 f64 16.3 -> 6.2, Hubbard chain 10
-// c128 18.5 -> 6.2, transverse Ising N=18 f64 16.4 -> 10.3.
+// pair kernels (us per apply, launches back to back on a caller's stream):
+// Heisenberg N=16 c128 10.3 -> 4.1, N=20 18.6 -> 10.3, Hubbard chain 8 float64
+// 14.4 -> 3.7, t-J N=17 float64 38 -> 25.  A call without a stream costs
+// another 0.3 us (it waits for the default stream).
 #include <algorithm>
 #include <cstring>
 #include <mutex>
@@ -189,9 +191,10 @@ __global__ void __launch_bounds__(256) k_packed_build(DevPlan p, uint32_t dim, c
 // bytes per lane, three at 32: eight targets in flight at fewer CTAs were
 // 10-20% slower (t-J N=18, 64 float32 vectors: 757 us with 3 CTAs, 721 with 4,
 // four targets and 5 CTAs 624; J1-J2 N=24, 32 float64 vectors: 1774 us with 2
-// CTAs, four targets and 3 CTAs 1514).  Against k_hx_rows_block: those two
-// 1117 -> 624 and 2173 -> 1514 us; t-J N=20, 64 vectors float32 4.97 -> 3.41,
-// float64 9.24 -> 6.60 ms; t-J N=13, 64 float32 56 -> 18 us.  Tiles of
+// CTAs, four targets and 3 CTAs 1514; kernel alone, fastest of several runs).
+// Whole applies against k_hx_rows_block: those two 1120 -> 680-705 and 2180 ->
+// 1570-1655 us; t-J N=20, 64 vectors float32 4.97 -> 3.41, float64 9.24 -> 6.60
+// ms; t-J N=13, 64 float32 56 -> 18 us.  Tiles of
 // kBlockTile rows from a queue per die; column dots per tile (sum_items).
 // Sectors with fewer than kBlockTiles tiles (two per resident CTA) take tiles
 // of 64 or 32 rows, so that a warp's rows, one after the other, are not the
